@@ -1,0 +1,38 @@
+"""The block-scaled e4m3 GEMM (gemm_scaled.cu) at the edges of its tiles, rounds and pieces, against 64-bit PyTorch math."""
+import pytest
+import torch
+
+from torch_dist_ext_b200.ops import gemm, quant
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("m,n,k", [
+    (1, 256, 128),          # one row, one K block
+    (33, 384, 256),         # one and a half tiles of weights
+    (64, 7168, 8192),       # decode: tiles in pieces of K
+    (128, 38144, 512),      # decode: 149 tiles, one more than the multiprocessors
+    (129, 256, 1024),       # the smallest pair: one row in the second CTA
+    (257, 1280, 8192),      # ragged rows, fewer tiles than pairs
+    (300, 640, 384),        # half a tile of weights at the end
+    (2048, 7168, 2048),     # three full rounds and two tiles over
+    (4100, 1280, 1024),     # ragged rows over a full round
+])
+def test_block_scaled_matches_64_bit(m, n, k):
+    g = torch.Generator(device="cuda").manual_seed(m + n + k)
+    a_q, a_s = quant.quant_fp8(torch.randn(m, k, device="cuda", generator=g).to(torch.bfloat16), block_scaled=True)
+    w_q, w_s = gemm.quantize_weight_block128(torch.randn(n, k, device="cuda", generator=g) * 0.05)
+    a = (a_q.double().view(m, k // 128, 128) * a_s.double()[..., None]).view(m, k)
+    w = (w_q.double().view(n // 128, 128, k // 128, 128) * w_s.double()[:, None, :, None]).view(n, k)
+    want = a @ w.t()
+    scale = want.abs().max()
+    for out_dtype in (torch.bfloat16, torch.float32):
+        torch.full((20 << 20,), float("nan"), device="cuda")     # freed at once: the scratch may hold anything
+        outs = [gemm.linear_fp8_blockscaled(a_q, a_s, w_q, w_s, out_dtype=out_dtype) for _ in range(2)]
+        torch.cuda.synchronize()
+        assert gemm.pipeline_status() == 0
+        assert torch.equal(outs[0], outs[1]), "the sum must not depend on which piece arrives last"
+        # half a rounding step of the output type (2^-9 for bf16) of the largest value; fp32: one rounding per K block
+        # and sum, 2^-24 each, with a margin of 8
+        bound = scale * (2.0 ** -8 if out_dtype == torch.bfloat16 else (k // 128 + 8) * 2.0 ** -21)
+        assert (outs[0].double() - want).abs().max() <= bound

@@ -67,6 +67,22 @@ std::string gemm_tn_pair(const GemmProblem& g, cudaStream_t stream);
 // operands, no split-K; block_n, splits and the scratch fields are ignored.
 std::string gemm_tn_persistent(const GemmProblem& g, cudaStream_t stream);
 
+// Block-scaled e4m3 product for any row count (gemm_scaled.cu): X are the activations (x_scale [x_rows, k / 128]), Y the
+// weights (y_scale [ceil(y_rows / 128), k / 128]). The plan says how the tiles are divided and which scratch that needs:
+// `slice_floats` fp32 values with any contents and `counters` zeroed words (left zeroed), through g.ws / g.counters.
+struct ScaledGemmPlan {
+  int ctas;            // CTAs that share a tile: 2 (256 x 256 tiles) or 1 (128 x 256)
+  int workers;         // CTA pairs or CTAs
+  int full_rounds;     // rounds in which every worker takes a whole tile
+  int parts, per;      // pieces per remaining tile, and K blocks per piece
+  size_t slice_floats;
+  size_t counters;
+};
+// `clusters`: how many clusters of 2, 4 and 8 CTAs the device holds at a time
+ScaledGemmPlan gemm_scaled_plan(int x_rows, int y_rows, int kblocks, int sms, const int (&clusters)[3]);
+ScaledGemmPlan gemm_scaled_plan_here(int x_rows, int y_rows, int kblocks);    // for the current device
+std::string gemm_scaled(const GemmProblem& g, const ScaledGemmPlan& plan, cudaStream_t stream);
+
 // Row-parallel linear fused with reduce(-scatter) + residual + RMSNorm (gemm_fused.cu).
 // `ar` carries the communication state (Workspace::fill_params) and describes the tail: tokens,
 // hidden, residual_in, gamma, residual_out, norm_out, scale_out, eps, out_mode (bf16 or e4m3 with

@@ -27,6 +27,16 @@ __device__ __forceinline__ void store_out(const Args& a, int64_t idx, float v) {
   else static_cast<float*>(a.out)[idx] = v;
 }
 
+// Two neighbouring values as one 32-bit word of the 16-bit output type.
+__device__ __forceinline__ uint32_t pack2(int out_dtype, float lo, float hi) {
+  if (out_dtype == kBF16) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&h);
+  }
+  const __half2 h = __floats2half2_rn(lo, hi);
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
+
 // Writes 16 consecutive y columns of row x (values already final): two 16-byte stores when the 16 columns are
 // contiguous 16-bit values at an aligned address, else element by element with bounds checks.
 template <typename Args>

@@ -322,6 +322,43 @@ void gemm_tn_persistent(const Tensor& x, const Tensor& y, Tensor out, int64_t sx
   TORCH_CHECK(err.empty(), "gemm_tn_persistent: ", err);
 }
 
+// Block-scaled e4m3 linear: out[m, n] = sum over 128-wide K blocks of a_scale * w_scale * (a . w).
+// A problem whose last tiles are divided along K brings its own scratch, so that calls on different streams share nothing.
+void gemm_scaled(const Tensor& a, const Tensor& w, Tensor out, const Tensor& a_scale, const Tensor& w_scale,
+                 const c10::optional<Tensor>& status) {
+  tdx::GemmProblem g = gemm_problem(a, w, out, w.size(0), 1, status);
+  TORCH_CHECK(a.scalar_type() == at::kFloat8_e4m3fn, "gemm_scaled: float8_e4m3fn operands");
+  TORCH_CHECK(g.k > 0 && g.k % 128 == 0, "gemm_scaled: K must be a positive multiple of 128");
+  TORCH_CHECK(a_scale.scalar_type() == at::kFloat && w_scale.scalar_type() == at::kFloat && a_scale.is_contiguous() && w_scale.is_contiguous(),
+              "gemm_scaled: scales must be contiguous float32");
+  const int64_t kb = g.k / 128;
+  TORCH_CHECK(a_scale.numel() == (int64_t)g.x_rows * kb, "gemm_scaled: a_scale has the wrong size");
+  TORCH_CHECK(w_scale.numel() == (int64_t)(g.y_rows + 127) / 128 * kb, "gemm_scaled: w_scale has the wrong size");
+  TORCH_CHECK(w.device() == a.device() && out.device() == a.device() && a_scale.device() == a.device() && w_scale.device() == a.device(),
+              "gemm_scaled: every tensor must live on a's device");
+  if (g.x_rows == 0 || g.y_rows == 0) return;
+  const c10::cuda::CUDAGuard guard(a.device());
+  g.x_scale = a_scale.data_ptr<float>();
+  g.y_scale = w_scale.data_ptr<float>();
+  const tdx::ScaledGemmPlan plan = tdx::gemm_scaled_plan_here(g.x_rows, g.y_rows, (int)kb);
+  Tensor slices, counters;
+  if (plan.slice_floats > 0) {
+    slices = at::empty({(int64_t)plan.slice_floats}, a.options().dtype(at::kFloat));
+    counters = at::zeros({(int64_t)plan.counters}, a.options().dtype(at::kInt));
+    gemm_scratch(g, slices, counters, "gemm_scaled");
+  }
+  const std::string err = tdx::gemm_scaled(g, plan, cur_stream());
+  TORCH_CHECK(err.empty(), "gemm_scaled: ", err);
+}
+
+// (ctas, workers, full_rounds, parts, per, slice_floats, counters) of a block-scaled problem on a device of `sms`
+// multiprocessors that holds so many clusters of 2, 4 and 8 CTAs
+std::vector<int64_t> gemm_scaled_plan(int64_t m, int64_t n, int64_t kblocks, int64_t sms, int64_t c2, int64_t c4, int64_t c8) {
+  const int clusters[3] = {(int)c2, (int)c4, (int)c8};
+  const tdx::ScaledGemmPlan p = tdx::gemm_scaled_plan((int)m, (int)n, (int)kblocks, (int)sms, clusters);
+  return {p.ctas, p.workers, p.full_rounds, p.parts, p.per, (int64_t)p.slice_floats, (int64_t)p.counters};
+}
+
 static void attention_decode_impl(const Tensor& q, const Tensor& k_cache, const Tensor& v_cache, const Tensor& seq_lens, Tensor& out,
                                   Tensor& partial, int64_t nsplit, double scale, const c10::optional<Tensor>& status,
                                   bool tensor_cores) {
@@ -504,6 +541,9 @@ void register_extra_ops(torch::Library& m) {
   m.def("gemm_tn(Tensor x, Tensor y, Tensor(a!) out, int sx, int sy, int block_n, int splits, Tensor(b!)? ws, "
         "Tensor(c!)? counters, Tensor(d!)? status, Tensor? x_scale, Tensor? y_scale, bool x_scale_per_row, "
         "bool y_scale_per_row, bool x_static=False) -> ()", &gemm_tn);
+  m.def("gemm_scaled(Tensor a, Tensor w, Tensor(a!) out, Tensor a_scale, Tensor w_scale, Tensor(b!)? status) -> ()",
+        &gemm_scaled);
+  m.def("gemm_scaled_plan(int m, int n, int kblocks, int sms, int c2, int c4, int c8) -> int[]", &gemm_scaled_plan);
   m.def("gemm_tn_rope_kv(Tensor w, Tensor a, Tensor(a!) out, int block_n, int splits, Tensor(b!) ws, Tensor(c!) counters, "
         "Tensor(d!)? status, Tensor? w_scale, Tensor? a_scale, Tensor positions, Tensor cos_sin, Tensor(e!) k_cache, "
         "Tensor(f!) v_cache, int q_heads, int kv_heads) -> ()", &gemm_tn_rope_kv);

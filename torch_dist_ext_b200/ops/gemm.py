@@ -132,11 +132,20 @@ def linear_fp8_blockscaled(a_q: torch.Tensor, a_scale: torch.Tensor, w_q: torch.
     """``(a_q * a_scale) @ (w_q * w_scale)^T`` with ``a_scale [M, K/128]`` and ``w_scale [N/128, K/128]``."""
     m, k = a_q.shape
     n = w_q.shape[0]
-    _, bn, p_splits = plan(m, n, k, 1, scaled=True)
-    splits = p_splits if splits is None else splits
     if out is None:
         out = torch.empty(m, n, dtype=out_dtype, device=a_q.device)
     ws, counters, status = _workspace(a_q.device)
+    # The kernel of gemm_scaled.cu (activations on the 128-row side, 256 weight rows per tile), except for a few tokens of
+    # a weight with so few rows that its tiles, in up to eight pieces each, leave most multiprocessors idle: there the
+    # swapped kernel cuts finer. B200, us per call, swapped / this one: 5120 x 8192 at 16 tokens 15.1 / 16.4, 1280 x 8192 at
+    # 32 tokens 9.2 / 10.5; 7168 x 8192 at 16 tokens 19.4 / 17.8, 1280 x 8192 at 64 tokens 13.1 / 11.6, 8192 x 1024 at 1 token
+    # 6.5 / 6.4, 28672 x 8192 at 64 tokens 81 / 47.
+    few = m <= 32 and n <= 20 * 256 and k > 2048
+    if splits is None and not few and out.is_contiguous():
+        _lib.ops().gemm_scaled(a_q, w_q, out, a_scale.contiguous(), w_scale.contiguous(), status)
+        return out
+    _, bn, p_splits = plan(m, n, k, 1, scaled=True)
+    splits = p_splits if splits is None else splits
     _lib.ops().gemm_tn(w_q, a_q, out, 1, n, bn, splits, ws, counters, status, w_scale.contiguous(),
                        a_scale.contiguous(), False, True, True)
     return out
