@@ -98,7 +98,7 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
   const int b = blockIdx.x, hkv = blockIdx.y, split = blockIdx.z;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   ptx::pdl_wait();                // q, the caches and seq_lens come from earlier kernels of the stream
   ptx::pdl_launch_dependents();
   const int len = a.seq_lens[b];
@@ -155,41 +155,40 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
     o[g] = 0.f;
   }
 
-  // Three single-thread roles, each with its own chain of waits: one thread needs 70-90 cycles per asynchronous
-  // instruction (four copies, eight score MMAs, eight P*V MMAs and three commits per chunk), which done one after the
-  // other took as long as HBM needs to deliver the chunk.
+  // Three issuing warps, each with its own chain of waits; the whole warp walks the loop and one elected lane issues.
   if (warp == 4) {
-    if (lane == 0 && nchunks > 0) {
-      // ---- copies: a stage is refilled when the P*V product that read its V tile has completed ----
-      auto issue_copy = [&](int c) {
-        const int st = c % kStages;
-        uint8_t* base = ring + st * kStageBytes;
+    // ---- copies: a stage is refilled when the P*V product that read its V tile has completed ----
+    auto issue_copy = [&](int c) {
+      const int st = c % kStages;
+      uint8_t* base = ring + st * kStageBytes;
+      const int pos0 = s0 + c * kKeys;
+      if (tc::elect_one()) {
         tc::mbar_arrive_expect_tx(&kv_full[st], kStageBytes);
-        const int pos0 = s0 + c * kKeys;
         tc::tma_load_4d(base, &map_k, &kv_full[st], 0, hkv, pos0, b);
         tc::tma_load_4d(base + kHalfBytes, &map_k, &kv_full[st], 64, hkv, pos0, b);
         tc::tma_load_4d(base + 2 * kHalfBytes, &map_v, &kv_full[st], 0, hkv, pos0, b);
         tc::tma_load_4d(base + 3 * kHalfBytes, &map_v, &kv_full[st], 64, hkv, pos0, b);
-      };
-      bool ok = true;
-      for (int c = 0; c < nchunks && c < kStages; ++c) issue_copy(c);
-      for (int i = 0; i + kStages < nchunks && ok; ++i) {
-        ok = tc::mbar_wait(&kv_free[i % kStages], (i / kStages) & 1, kWaitLimit, abort_flag);
-        if (ok) issue_copy(i + kStages);
       }
-      if (!ok) fail();
+      __syncwarp();
+    };
+    bool ok = true;
+    for (int c = 0; c < nchunks && c < kStages; ++c) issue_copy(c);
+    for (int i = 0; i + kStages < nchunks && ok; ++i) {
+      ok = tc::mbar_wait_warp(&kv_free[i % kStages], (i / kStages) & 1, kWaitLimit, abort_flag);
+      if (ok) issue_copy(i + kStages);
     }
+    if (!ok) fail();
   } else if (warp == 5) {
-    if (lane == 0 && nchunks > 0) {
-      // ---- scores: S^T[buf c & 1] = K chunk * Q^T, as soon as the chunk has landed and the buffer is free ----
-      const uint32_t qbase = tc::smem_u32(q_tile);
-      bool ok = true;
-      for (int c = 0; c < nchunks && ok; ++c) {
-        ok = tc::mbar_wait(&kv_full[c % kStages], (c / kStages) & 1, kWaitLimit, abort_flag) &&
-             (c < 2 || tc::mbar_wait(&s_free[c & 1], ((c >> 1) - 1) & 1, kWaitLimit, abort_flag));
-        if (!ok) break;
-        tc::fence_after_thread_sync();
-        const uint32_t kbase = tc::smem_u32(ring + (c % kStages) * kStageBytes);
+    // ---- scores: S^T[buf c & 1] = K chunk * Q^T, as soon as the chunk has landed and the buffer is free ----
+    const uint32_t qbase = tc::smem_u32(q_tile);
+    bool ok = true;
+    for (int c = 0; c < nchunks && ok; ++c) {
+      ok = tc::mbar_wait_warp(&kv_full[c % kStages], (c / kStages) & 1, kWaitLimit, abort_flag) &&
+           (c < 2 || tc::mbar_wait_warp(&s_free[c & 1], ((c >> 1) - 1) & 1, kWaitLimit, abort_flag));
+      if (!ok) break;
+      tc::fence_after_thread_sync();
+      const uint32_t kbase = tc::smem_u32(ring + (c % kStages) * kStageBytes);
+      if (tc::elect_one()) {
 #pragma unroll
         for (int kb = 0; kb < 2; ++kb)
 #pragma unroll
@@ -198,19 +197,20 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
                             tc::make_smem_desc_sw128(qbase + kb * (kNq * 128)) + (uint64_t)(ks * 2), a.idesc_s, (kb | ks) ? 1u : 0u);
         tc::umma_commit(&s_full[c & 1]);
       }
-      if (!ok) fail();
+      __syncwarp();
     }
+    if (!ok) fail();
   } else if (warp == 6) {
-    if (lane == 0 && nchunks > 0) {
-      // ---- O^T (+)= V chunk^T * P^T, 16 cache positions per instruction, once the probabilities are written ----
-      bool ok = true;
-      for (int c = 0; c < nchunks && ok; ++c) {
-        ok = tc::mbar_wait(&p_full[c & 1], (c >> 1) & 1, kWaitLimit, abort_flag) &&
-             tc::mbar_wait(&kv_full[c % kStages], (c / kStages) & 1, kWaitLimit, abort_flag);
-        if (!ok) break;
-        tc::fence_after_thread_sync();
-        const uint32_t vbase = tc::smem_u32(ring + (c % kStages) * kStageBytes + 2 * kHalfBytes);
-        const uint32_t pbase = tc::smem_u32(p_tile + (c & 1) * kSmallTileBytes);
+    // ---- O^T (+)= V chunk^T * P^T, 16 cache positions per instruction, once the probabilities are written ----
+    bool ok = true;
+    for (int c = 0; c < nchunks && ok; ++c) {
+      ok = tc::mbar_wait_warp(&p_full[c & 1], (c >> 1) & 1, kWaitLimit, abort_flag) &&
+           tc::mbar_wait_warp(&kv_full[c % kStages], (c / kStages) & 1, kWaitLimit, abort_flag);
+      if (!ok) break;
+      tc::fence_after_thread_sync();
+      const uint32_t vbase = tc::smem_u32(ring + (c % kStages) * kStageBytes + 2 * kHalfBytes);
+      const uint32_t pbase = tc::smem_u32(p_tile + (c & 1) * kSmallTileBytes);
+      if (tc::elect_one()) {
 #pragma unroll
         for (int j = 0; j < 8; ++j)
           tc::umma<false>(tmem_base + kColO, tc::make_smem_desc_mn_sw128(vbase + j * 2048, kHalfBytes),
@@ -219,8 +219,9 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
         tc::umma_commit(&o_full[c & 1]);
         tc::umma_commit(&kv_free[c % kStages]);
       }
-      if (!ok) fail();
+      __syncwarp();
     }
+    if (!ok) fail();
   } else {
     // ---- softmax warps: thread t owns cache position t of the chunk and head-dimension index t of the output ----
     // O^T accumulates in tensor memory over all chunks of the split (the P*V MMAs add to it), so a chunk costs the

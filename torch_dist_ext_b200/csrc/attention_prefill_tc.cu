@@ -137,7 +137,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   const int qb = (int)gridDim.y - 1 - (int)blockIdx.y;
   const int h = blockIdx.x;
   const int hkv = h / (a.Hq / a.Hkv);
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int q0 = qb * kRows;
   const int nchunks = (q0 + kRows) / kKeys;  // key positions 0 .. q0 + 127 (causal)
 #ifdef TDX_ATTN_PROBE
@@ -185,9 +185,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     if (a.status) atomicExch(a.status, (uint32_t)kTimeoutGemmPipeline);
   };
 
-  // Three single-thread roles in three warps, each with its own chain of waits, so that none of them queues behind
-  // the others' (one thread doing all three spent about 2300 cycles per chunk issuing copies, MMAs and commits one
-  // after the other, twice what a softmax group needs for the chunk):
+  // Five issuing warps, each with its own chain of waits, so that none of them queues behind the others'. The whole warp
+  // walks the loop and one elected lane issues (tc::elect_one):
   //   loader        TMA copies of Q, K and V; refills a K stage when its scores are complete, a V stage after P*V
   //   score issuers S_(c & 1) = Q K_c^T as soon as K_c has landed and the group has taken chunk c - 2 out of the buffer
 //                 (two of them: one for the even chunks, one for the odd ones)
@@ -195,59 +194,60 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   // MMAs of the two issuers touch different tensor-memory columns and different tiles; what orders them against the
   // softmax groups are the barriers below, and each issuer's commits cover its own MMAs.
   if (warp == kLoadWarp) {
-    if (lane == 0) {
-      auto load_k = [&](int c) {
-        uint8_t* base = k_ring + (c % kStagesK) * kKVBytes;
-        tc::mbar_arrive_expect_tx(&k_full[c % kStagesK], kKVBytes);
-        tc::tma_load_3d(base, &map_k, &k_full[c % kStagesK], 0, hkv, c * kKeys);
-        tc::tma_load_3d(base + kKVHalfBytes, &map_k, &k_full[c % kStagesK], 64, hkv, c * kKeys);
-      };
-      auto load_v = [&](int c) {
-        uint8_t* base = v_ring + (c % kStagesV) * kKVBytes;
-        tc::mbar_arrive_expect_tx(&v_full[c % kStagesV], kKVBytes);
-        tc::tma_load_3d(base, &map_v, &v_full[c % kStagesV], 0, hkv, c * kKeys);
-        tc::tma_load_3d(base + kKVHalfBytes, &map_v, &v_full[c % kStagesV], 64, hkv, c * kKeys);
-      };
+    auto load_k = [&](int c) {
+      uint8_t* base = k_ring + (c % kStagesK) * kKVBytes;
+      tc::mbar_arrive_expect_tx(&k_full[c % kStagesK], kKVBytes);
+      tc::tma_load_3d(base, &map_k, &k_full[c % kStagesK], 0, hkv, c * kKeys);
+      tc::tma_load_3d(base + kKVHalfBytes, &map_k, &k_full[c % kStagesK], 64, hkv, c * kKeys);
+    };
+    auto load_v = [&](int c) {
+      uint8_t* base = v_ring + (c % kStagesV) * kKVBytes;
+      tc::mbar_arrive_expect_tx(&v_full[c % kStagesV], kKVBytes);
+      tc::tma_load_3d(base, &map_v, &v_full[c % kStagesV], 0, hkv, c * kKeys);
+      tc::tma_load_3d(base + kKVHalfBytes, &map_v, &v_full[c % kStagesV], 64, hkv, c * kKeys);
+    };
+    if (tc::elect_one()) {
       tc::mbar_arrive_expect_tx(q_full, kQBytes);
       tc::tma_load_3d(q_tile, &map_q, q_full, 0, h, q0);
       tc::tma_load_3d(q_tile + kQHalfBytes, &map_q, q_full, 64, h, q0);
       for (int c = 0; c < nchunks && c < kStagesK; ++c) load_k(c);
       for (int c = 0; c < nchunks && c < kStagesV; ++c) load_v(c);
-      bool ok = true;
-      // The P*V products trail the score MMAs by about two chunks, so the V stages come free two chunks after the
-      // K stages: the K refill of chunk j shares an iteration with the V refill of chunk j - 2, and neither wait
-      // holds the other's copies back.
-      for (int j = 0; j < nchunks + 2 && ok; ++j) {
-        if (j + kStagesK < nchunks) {
-          // K stage of chunk j is free once its scores are complete (long before P*V of the chunk)
-          ok = tc::mbar_wait(&k_free[j % kStagesK], (j / kStagesK) & 1, kWaitLimit, abort_flag);
-          if (!ok) break;
-          load_k(j + kStagesK);
-        }
-        const int i = j - 2;
-        if (i >= 0 && i + kStagesV < nchunks) {
-          // V stage of chunk i is free once its P*V product is complete
-          ok = tc::mbar_wait(&v_free[i % kStagesV], (i / kStagesV) & 1, kWaitLimit, abort_flag);
-          if (!ok) break;
-          load_v(i + kStagesV);
-        }
-      }
-      if (!ok) fail();
     }
-  } else if (warp == kScoreWarp || warp == kScoreWarp + 1) {
-    if (lane == 0) {
-      // issuing the eight MMAs and two commits of a chunk takes one thread longer than a softmax group needs for
-      // the chunk, so the even and the odd chunks have an issuer each
-      const uint32_t qbase = tc::smem_u32(q_tile);
-      bool ok = tc::mbar_wait(q_full, 0, kWaitLimit, abort_flag);
-      for (int c = warp - kScoreWarp; c < nchunks && ok; c += 2) {
-        TDX_PROBE(0, c, 0);
-        ok = tc::mbar_wait(&k_full[c % kStagesK], (c / kStagesK) & 1, kWaitLimit, abort_flag) &&
-             (c < 2 || tc::mbar_wait(&s_free[c & 1], ((c >> 1) - 1) & 1, kWaitLimit, abort_flag));
+    __syncwarp();
+    bool ok = true;
+    // The P*V products trail the score MMAs by about two chunks, so the V stages come free two chunks after the
+    // K stages: the K refill of chunk j shares an iteration with the V refill of chunk j - 2, and neither wait
+    // holds the other's copies back.
+    for (int j = 0; j < nchunks + 2 && ok; ++j) {
+      if (j + kStagesK < nchunks) {
+        // K stage of chunk j is free once its scores are complete (long before P*V of the chunk)
+        ok = tc::mbar_wait_warp(&k_free[j % kStagesK], (j / kStagesK) & 1, kWaitLimit, abort_flag);
         if (!ok) break;
-        TDX_PROBE(0, c, 1);
-        tc::fence_after_thread_sync();
-        const uint32_t kbase = tc::smem_u32(k_ring + (c % kStagesK) * kKVBytes);
+        if (tc::elect_one()) load_k(j + kStagesK);
+        __syncwarp();
+      }
+      const int i = j - 2;
+      if (i >= 0 && i + kStagesV < nchunks) {
+        // V stage of chunk i is free once its P*V product is complete
+        ok = tc::mbar_wait_warp(&v_free[i % kStagesV], (i / kStagesV) & 1, kWaitLimit, abort_flag);
+        if (!ok) break;
+        if (tc::elect_one()) load_v(i + kStagesV);
+        __syncwarp();
+      }
+    }
+    if (!ok) fail();
+  } else if (warp == kScoreWarp || warp == kScoreWarp + 1) {
+    const uint32_t qbase = tc::smem_u32(q_tile);
+    bool ok = tc::mbar_wait_warp(q_full, 0, kWaitLimit, abort_flag);
+    for (int c = warp - kScoreWarp; c < nchunks && ok; c += 2) {
+      TDX_PROBE(0, c, 0);
+      ok = tc::mbar_wait_warp(&k_full[c % kStagesK], (c / kStagesK) & 1, kWaitLimit, abort_flag) &&
+           (c < 2 || tc::mbar_wait_warp(&s_free[c & 1], ((c >> 1) - 1) & 1, kWaitLimit, abort_flag));
+      if (!ok) break;
+      TDX_PROBE(0, c, 1);
+      tc::fence_after_thread_sync();
+      const uint32_t kbase = tc::smem_u32(k_ring + (c % kStagesK) * kKVBytes);
+      if (tc::elect_one()) {
 #pragma unroll
         for (int kb = 0; kb < 2; ++kb)     // the two 64-column halves of the head dimension
 #pragma unroll
@@ -256,21 +256,22 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                             tc::make_smem_desc_sw128(kbase + kb * kKVHalfBytes) + (uint64_t)(ks * 2), a.idesc_s, (kb | ks) ? 1u : 0u);
         tc::umma_commit(&s_full[c & 1]);
         tc::umma_commit(&k_free[c % kStagesK]);    // the K stage is free once these complete
-        TDX_PROBE(0, c, 2);
       }
-      if (!ok) fail();
+      __syncwarp();
+      TDX_PROBE(0, c, 2);
     }
+    if (!ok) fail();
   } else if (warp == kPvWarp || warp == kPvWarp + 1) {
-    if (lane == 0) {
-      bool ok = true;
-      for (int c = warp - kPvWarp; c < nchunks && ok; c += 2) {
-        ok = tc::mbar_wait(&p_full[c & 3], (c >> 2) & 1, kWaitLimit, abort_flag) &&
-             tc::mbar_wait(&v_full[c % kStagesV], (c / kStagesV) & 1, kWaitLimit, abort_flag);
-        if (!ok) break;
-        TDX_PROBE(0, c, 3);
-        tc::fence_after_thread_sync();
-        const uint32_t vbase = tc::smem_u32(v_ring + (c % kStagesV) * kKVBytes);
-        const uint32_t pbase = tc::smem_u32(p_tile + (c & 3) * kPBytes);
+    bool ok = true;
+    for (int c = warp - kPvWarp; c < nchunks && ok; c += 2) {
+      ok = tc::mbar_wait_warp(&p_full[c & 3], (c >> 2) & 1, kWaitLimit, abort_flag) &&
+           tc::mbar_wait_warp(&v_full[c % kStagesV], (c / kStagesV) & 1, kWaitLimit, abort_flag);
+      if (!ok) break;
+      TDX_PROBE(0, c, 3);
+      tc::fence_after_thread_sync();
+      const uint32_t vbase = tc::smem_u32(v_ring + (c % kStagesV) * kKVBytes);
+      const uint32_t pbase = tc::smem_u32(p_tile + (c & 3) * kPBytes);
+      if (tc::elect_one()) {
 #pragma unroll
         for (int j = 0; j < kKeys / 16; ++j)   // 16 key positions per instruction
           tc::umma<false>(tmem_base + kColO + (uint32_t)(c & 1) * kD, tc::make_smem_desc_sw128(pbase) + (uint64_t)(j * 2),
@@ -278,10 +279,11 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         tc::umma_commit(&pv_done[c & 3]);
         tc::umma_commit(&v_free[c % kStagesV]);
         if (c + 2 >= nchunks) tc::umma_commit(o_final);      // this issuer's last chunk
-        TDX_PROBE(0, c, 4);
       }
-      if (!ok) fail();
+      __syncwarp();
+      TDX_PROBE(0, c, 4);
     }
+    if (!ok) fail();
   } else {
     // ---- softmax warps: group g = warp / 4 takes the chunks g, g + 2, ...; its thread t owns query row q0 + t ----
     // A thread whose wait ran out keeps walking the loop (its waits return at once because the abort flag is up),

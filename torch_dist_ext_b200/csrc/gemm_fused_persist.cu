@@ -83,7 +83,7 @@ gemm_ar_rmsnorm_persist_kernel(const __grid_constant__ CUtensorMap map_w, const 
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
   const ArParams& p = f.ar;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const int cta = blockIdx.x, nctas = gridDim.x;
   const int ntiles = f.tiles_x * f.tiles_y;
   const int nkb = f.kblocks;
@@ -126,61 +126,63 @@ gemm_ar_rmsnorm_persist_kernel(const __grid_constant__ CUtensorMap map_w, const 
   };
 
   if (warp == 0) {
-    if (lane == 0) {
-      // ---- producer: the hidden-column tile index runs fastest, so CTAs working side by side share the token tile ----
-      uint32_t it = 0;
-      for (int t = cta; t < ntiles && !*abort_flag; t += nctas) {
-        const int x_row0 = (t % f.tiles_x) * kBM, y_row0 = (t / f.tiles_x) * kBN;
-        bool ok = true;
-        for (int kb = 0; kb < nkb; ++kb, ++it) {
-          const uint32_t s = it % kStages;
-          if (it >= (uint32_t)kStages && !tc::mbar_wait(&empty[s], ((it / kStages) - 1) & 1, kWaitLimit, abort_flag)) {
-            ok = false;
-            break;
-          }
-          uint8_t* dst = smem + s * kStageBytes;
+    // ---- producer (one elected lane issues): the hidden-column tile index runs fastest, so CTAs working side by side share the token tile ----
+    uint32_t it = 0;
+    for (int t = cta; t < ntiles; t += nctas) {
+      const int x_row0 = (t % f.tiles_x) * kBM, y_row0 = (t / f.tiles_x) * kBN;
+      bool ok = true;
+      for (int kb = 0; kb < nkb; ++kb, ++it) {
+        const uint32_t s = it % kStages;
+        if (it >= (uint32_t)kStages && !tc::mbar_wait_warp(&empty[s], ((it / kStages) - 1) & 1, kWaitLimit, abort_flag)) {
+          ok = false;
+          break;
+        }
+        uint8_t* dst = smem + s * kStageBytes;
+        if (tc::elect_one()) {
           tc::mbar_arrive_expect_tx(&full[s], kStageBytes);
           tc::tma_load_2d(dst, &map_w, &full[s], kb * 64, x_row0);
           tc::tma_load_2d(dst + kXBytes, &map_a, &full[s], kb * 64, y_row0);
         }
-        if (!ok) {
-          fail();
-          break;
-        }
+        __syncwarp();
+      }
+      if (!ok) {
+        fail();
+        break;
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      // ---- MMA issue ----
-      uint32_t it = 0;
-      int n = 0;
-      bool ok = true;
-      for (int t = cta; t < ntiles && ok; t += nctas, ++n) {
-        const uint32_t buf = n & 1;
-        if (n >= 2 && !tc::mbar_wait(&acc_empty[buf], ((n >> 1) - 1) & 1, kWaitLimit, abort_flag)) {
+    // ---- MMA issue (one elected lane issues) ----
+    uint32_t it = 0;
+    int n = 0;
+    bool ok = true;
+    for (int t = cta; t < ntiles && ok; t += nctas, ++n) {
+      const uint32_t buf = n & 1;
+      if (n >= 2 && !tc::mbar_wait_warp(&acc_empty[buf], ((n >> 1) - 1) & 1, kWaitLimit, abort_flag)) {
+        ok = false;
+        break;
+      }
+      tc::fence_after_thread_sync();
+      for (int kb = 0; kb < nkb; ++kb, ++it) {
+        const uint32_t s = it % kStages;
+        if (!tc::mbar_wait_warp(&full[s], (it / kStages) & 1, kWaitLimit, abort_flag)) {
           ok = false;
           break;
         }
         tc::fence_after_thread_sync();
-        for (int kb = 0; kb < nkb; ++kb, ++it) {
-          const uint32_t s = it % kStages;
-          if (!tc::mbar_wait(&full[s], (it / kStages) & 1, kWaitLimit, abort_flag)) {
-            ok = false;
-            break;
-          }
-          tc::fence_after_thread_sync();
-          const uint32_t xa = tc::smem_u32(smem + s * kStageBytes);
-          const uint64_t dx = tc::make_smem_desc_sw128(xa);
-          const uint64_t dy = tc::make_smem_desc_sw128(xa + kXBytes);
+        const uint32_t xa = tc::smem_u32(smem + s * kStageBytes);
+        const uint64_t dx = tc::make_smem_desc_sw128(xa);
+        const uint64_t dy = tc::make_smem_desc_sw128(xa + kXBytes);
+        if (tc::elect_one()) {
 #pragma unroll
           for (int k = 0; k < 4; ++k)
             tc::umma<false>(tmem_base + buf * kBN, dx + (uint64_t)(k * 2), dy + (uint64_t)(k * 2), f.idesc, (kb > 0 || k > 0) ? 1u : 0u);
           tc::umma_commit(&empty[s]);
+          if (kb + 1 == nkb) tc::umma_commit(&acc_full[buf]);
         }
-        if (ok) tc::umma_commit(&acc_full[buf]);
+        __syncwarp();
       }
-      if (!ok) fail();
     }
+    if (!ok) fail();
   } else if (warp < 6) {
     // ---- epilogue (warps 2..5): TMEM lane quarter = warp % 4; the four warps push a tile together ----
     const int q = warp & 3;

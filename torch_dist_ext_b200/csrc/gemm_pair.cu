@@ -120,7 +120,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
   volatile uint32_t* abort_flag = tmem_slot + 1;
   uint32_t* last_flag = tmem_slot + 2;       // tail split: "this CTA arrived last at its half of the tile"
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const uint32_t rank = tc::cluster_ctarank();      // 0: leader, 1: peer
   const uint32_t leader = rank & ~1u, other = rank ^ 1u;
   const int pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
@@ -161,34 +161,36 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     if (a.status) atomicExch(a.status, (uint32_t)kTimeoutGemmPipeline);
   };
 
+  // The loops of the copying and issuing warps are walked by the whole warp, one elected lane issues (tc::elect_one).
   if (warp == 0) {
-    if (lane == 0) {
-      // ---- producer (both CTAs): own halves of X and Y, bytes credited to the leader's barrier ----
-      const uint32_t leader_full = tc::map_to_cta(tc::smem_u32(&full[0]), leader);
-      uint32_t it = 0;                                   // K blocks issued so far by this CTA
-      bool ok = true;
-      WorkItem w;
-      for (int n = 0; work_item(a, pair, npairs, n, &w) && ok && !*abort_flag; ++n) {
-        const int t = w.tile;
-        const int x_row0 = (t % a.tiles_x) * kTileM + (int)(rank & 1u) * kRowsPerCta;
-        const int y_row0 = (t / a.tiles_x) * kTileN + (int)(rank & 1u) * kRowsPerCta;
-        for (int kb = w.kb0; kb < w.kb1; ++kb, ++it) {
-          const uint32_t s = it % kStages;
-          if (it >= (uint32_t)kStages && !tc::mbar_wait(&empty[s], ((it / kStages) - 1) & 1, kWaitLimit, abort_flag)) {
-            ok = false;
-            break;
-          }
+    // ---- producer (both CTAs): own halves of X and Y, bytes credited to the leader's barrier ----
+    const uint32_t leader_full = tc::map_to_cta(tc::smem_u32(&full[0]), leader);
+    uint32_t it = 0;                                   // K blocks issued so far by this CTA
+    bool ok = true;
+    WorkItem w;
+    for (int n = 0; work_item(a, pair, npairs, n, &w) && ok; ++n) {
+      const int t = w.tile;
+      const int x_row0 = (t % a.tiles_x) * kTileM + (int)(rank & 1u) * kRowsPerCta;
+      const int y_row0 = (t / a.tiles_x) * kTileN + (int)(rank & 1u) * kRowsPerCta;
+      for (int kb = w.kb0; kb < w.kb1; ++kb, ++it) {
+        const uint32_t s = it % kStages;
+        if (it >= (uint32_t)kStages && !tc::mbar_wait_warp(&empty[s], ((it / kStages) - 1) & 1, kWaitLimit, abort_flag)) {
+          ok = false;
+          break;
+        }
+        const uint32_t dst = tc::smem_u32(smem + s * kStageBytes);
+        const uint32_t bar = leader_full + s * 8u;
+        if (tc::elect_one()) {
           if (rank == leader) tc::mbar_arrive_expect_tx(&full[s], 2 * kStageBytes);
-          const uint32_t dst = tc::smem_u32(smem + s * kStageBytes);
-          const uint32_t bar = leader_full + s * 8u;
           tc::tma_load_2d_pair(dst, &map_x, bar, kb * kElemsPerBlock, x_row0);
           tc::tma_load_2d_pair(dst + kOperandBytes, &map_y, bar, kb * kElemsPerBlock, y_row0);
         }
+        __syncwarp();
       }
-      if (!ok) fail();
     }
+    if (!ok) fail();
   } else if (warp == 1) {
-    if (lane == 0 && rank == leader) {
+    if (rank == leader) {
       // ---- MMA issue (leader only) ----
       uint32_t it = 0;
       int n = 0;                                         // tiles started so far by this pair
@@ -196,14 +198,14 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
       WorkItem w;
       for (; work_item(a, pair, npairs, n, &w) && ok; ++n) {
         const uint32_t buf = n & 1;
-        if (n >= 2 && !tc::mbar_wait(&acc_empty[buf], ((n >> 1) - 1) & 1, kWaitLimit, abort_flag)) {
+        if (n >= 2 && !tc::mbar_wait_warp(&acc_empty[buf], ((n >> 1) - 1) & 1, kWaitLimit, abort_flag)) {
           ok = false;
           break;
         }
         tc::fence_after_thread_sync();
         for (int kb = w.kb0; kb < w.kb1; ++kb, ++it) {
           const uint32_t s = it % kStages;
-          if (!tc::mbar_wait(&full[s], (it / kStages) & 1, kWaitLimit, abort_flag)) {
+          if (!tc::mbar_wait_warp(&full[s], (it / kStages) & 1, kWaitLimit, abort_flag)) {
             ok = false;
             break;
           }
@@ -211,13 +213,16 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
           const uint32_t xa = tc::smem_u32(smem + s * kStageBytes);
           const uint64_t dx = tc::make_smem_desc_sw128(xa);
           const uint64_t dy = tc::make_smem_desc_sw128(xa + kOperandBytes);
+          if (tc::elect_one()) {
 #pragma unroll
-          for (int k = 0; k < 4; ++k)   // 32 bytes of K per instruction, stepped inside the swizzle span
-            tc::umma_pair<kFp8>(tmem_base + buf * kTileN, dx + (uint64_t)(k * 2), dy + (uint64_t)(k * 2), a.idesc,
-                                (kb > w.kb0 || k > 0) ? 1u : 0u);
-          tc::umma_commit_pair(&empty[s], other);   // the stage is free again in both CTAs
+            for (int k = 0; k < 4; ++k)   // 32 bytes of K per instruction, stepped inside the swizzle span
+              tc::umma_pair<kFp8>(tmem_base + buf * kTileN, dx + (uint64_t)(k * 2), dy + (uint64_t)(k * 2), a.idesc,
+                                  (kb > w.kb0 || k > 0) ? 1u : 0u);
+            tc::umma_commit_both(&empty[s]);   // the stage is free again in both CTAs
+            if (kb + 1 == w.kb1) tc::umma_commit_both(&acc_full[buf]);
+          }
+          __syncwarp();
         }
-        if (ok) tc::umma_commit_pair(&acc_full[buf], other);
       }
       if (!ok) fail();
     }
@@ -248,7 +253,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         }
         tc::fence_before_thread_sync();
         __syncwarp();
-        if (lane == 0) tc::mbar_arrive_cluster(leader_acc_empty + buf * 8u);   // this warp has read its part of the buffer
+        if (lane == 0) tc::mbar_arrive_cluster_relaxed(leader_acc_empty + buf * 8u);   // this warp has read its part of the buffer
       } else {
         // A K range of a tail tile: this CTA's 128 x 256 partial sums go to the piece's own slice of the scratch
         // (column-major, so that a warp's lanes write 32 consecutive floats; plain stores - fp32 atomics on a
@@ -267,7 +272,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         }
         tc::fence_before_thread_sync();
         __syncwarp();
-        if (lane == 0) tc::mbar_arrive_cluster(leader_acc_empty + buf * 8u);
+        if (lane == 0) tc::mbar_arrive_cluster_relaxed(leader_acc_empty + buf * 8u);
         __threadfence();
         tc::named_barrier_sync(1, 128);
         if (threadIdx.x == 64) {

@@ -72,7 +72,7 @@ gemm_persist_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const int ntiles = a.tiles_x * a.tiles_y;
   const int nkb = a.kblocks;
 
@@ -107,61 +107,63 @@ gemm_persist_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
   };
 
   if (warp == 0) {
-    if (lane == 0) {
-      // ---- producer: the x tile index runs fastest, so CTAs that work side by side share the Y (weight) tile in L2 ----
-      uint32_t it = 0;                                   // K blocks issued so far by this CTA
-      for (int t = blockIdx.x; t < ntiles && !*abort_flag; t += gridDim.x) {
-        const int x_row0 = (t % a.tiles_x) * kBM, y_row0 = (t / a.tiles_x) * kBN;
-        bool ok = true;
-        for (int kb = 0; kb < nkb; ++kb, ++it) {
-          const uint32_t s = it % kStages;
-          if (it >= (uint32_t)kStages && !tc::mbar_wait(&empty[s], ((it / kStages) - 1) & 1, kWaitLimit, abort_flag)) {
-            ok = false;
-            break;
-          }
-          uint8_t* dst = smem + s * kStageBytes;
+    // ---- producer (one elected lane issues): the x tile index runs fastest, so CTAs that work side by side share the Y (weight) tile in L2 ----
+    uint32_t it = 0;                                   // K blocks issued so far by this CTA
+    for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
+      const int x_row0 = (t % a.tiles_x) * kBM, y_row0 = (t / a.tiles_x) * kBN;
+      bool ok = true;
+      for (int kb = 0; kb < nkb; ++kb, ++it) {
+        const uint32_t s = it % kStages;
+        if (it >= (uint32_t)kStages && !tc::mbar_wait_warp(&empty[s], ((it / kStages) - 1) & 1, kWaitLimit, abort_flag)) {
+          ok = false;
+          break;
+        }
+        uint8_t* dst = smem + s * kStageBytes;
+        if (tc::elect_one()) {
           tc::mbar_arrive_expect_tx(&full[s], kStageBytes);
           tc::tma_load_2d(dst, &map_x, &full[s], kb * kElemsPerBlock, x_row0);
           tc::tma_load_2d(dst + kXBytes, &map_y, &full[s], kb * kElemsPerBlock, y_row0);
         }
-        if (!ok) {
-          fail();
-          break;
-        }
+        __syncwarp();
+      }
+      if (!ok) {
+        fail();
+        break;
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      // ---- MMA issue ----
-      uint32_t it = 0;
-      int n = 0;                                         // tiles started so far by this CTA
-      bool ok = true;
-      for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x, ++n) {
-        const uint32_t buf = n & 1;
-        if (n >= 2 && !tc::mbar_wait(&acc_empty[buf], ((n >> 1) - 1) & 1, kWaitLimit, abort_flag)) {
+    // ---- MMA issue (one elected lane issues) ----
+    uint32_t it = 0;
+    int n = 0;                                         // tiles started so far by this CTA
+    bool ok = true;
+    for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x, ++n) {
+      const uint32_t buf = n & 1;
+      if (n >= 2 && !tc::mbar_wait_warp(&acc_empty[buf], ((n >> 1) - 1) & 1, kWaitLimit, abort_flag)) {
+        ok = false;
+        break;
+      }
+      tc::fence_after_thread_sync();
+      for (int kb = 0; kb < nkb; ++kb, ++it) {
+        const uint32_t s = it % kStages;
+        if (!tc::mbar_wait_warp(&full[s], (it / kStages) & 1, kWaitLimit, abort_flag)) {
           ok = false;
           break;
         }
         tc::fence_after_thread_sync();
-        for (int kb = 0; kb < nkb; ++kb, ++it) {
-          const uint32_t s = it % kStages;
-          if (!tc::mbar_wait(&full[s], (it / kStages) & 1, kWaitLimit, abort_flag)) {
-            ok = false;
-            break;
-          }
-          tc::fence_after_thread_sync();
-          const uint32_t xa = tc::smem_u32(smem + s * kStageBytes);
-          const uint64_t dx = tc::make_smem_desc_sw128(xa);
-          const uint64_t dy = tc::make_smem_desc_sw128(xa + kXBytes);
+        const uint32_t xa = tc::smem_u32(smem + s * kStageBytes);
+        const uint64_t dx = tc::make_smem_desc_sw128(xa);
+        const uint64_t dy = tc::make_smem_desc_sw128(xa + kXBytes);
+        if (tc::elect_one()) {
 #pragma unroll
           for (int k = 0; k < 4; ++k)   // 32 bytes of K per instruction, stepped inside the swizzle span
             tc::umma<kFp8>(tmem_base + buf * kBN, dx + (uint64_t)(k * 2), dy + (uint64_t)(k * 2), a.idesc, (kb > 0 || k > 0) ? 1u : 0u);
           tc::umma_commit(&empty[s]);   // the stage is reusable once these MMAs have read it
+          if (kb + 1 == nkb) tc::umma_commit(&acc_full[buf]);
         }
-        if (ok) tc::umma_commit(&acc_full[buf]);
+        __syncwarp();
       }
-      if (!ok) fail();
     }
+    if (!ok) fail();
   } else {
     // ---- epilogue (warps 2..5): TMEM lane quarter = warp % 4 ----
     const int q = warp & 3;

@@ -172,27 +172,25 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
   uint32_t* last_flag = pipe.scratch;
   const uint32_t tmem_base = pipe.tmem_base;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const int tile_x = blockIdx.x, tile_y = blockIdx.y;
   const int kb0 = blockIdx.z * a.kblocks_per_split;
   const int kb1 = min(a.kblocks, kb0 + a.kblocks_per_split);
   const int nkb = kb1 - kb0;
 
   if (warp == 0) {
-    if (lane == 0) {
-      // With static X (decode orientation: the weights) the first ring of X tiles is requested before the wait for
-      // the previous kernel of the stream; everything else is read and written after it.
-      if (!a.x_static) ptx::pdl_wait();
-      // silu(gate) * up: 64 gate rows and the 64 up rows of the same features make one 128-row tile
-      const bool halves = a.epi.kind == kEpiSiluMul;
-      pipe.template produce<kElemsPerBlock>(&map_x, &map_y, halves ? tile_x * 64 : tile_x * kBM, tile_y * kBN, kb0, nkb, a.status, [] {
-        ptx::pdl_wait();
-        return true;
-      }, halves ? a.epi.ffn + tile_x * 64 : -1);
-      ptx::pdl_launch_dependents();
-    }
+    // With static X (decode orientation: the weights) the first ring of X tiles is requested before the wait for
+    // the previous kernel of the stream; everything else is read and written after it.
+    if (!a.x_static) ptx::pdl_wait();
+    // silu(gate) * up: 64 gate rows and the 64 up rows of the same features make one 128-row tile
+    const bool halves = a.epi.kind == kEpiSiluMul;
+    pipe.template produce<kElemsPerBlock>(&map_x, &map_y, halves ? tile_x * 64 : tile_x * kBM, tile_y * kBN, kb0, nkb, a.status, [] {
+      ptx::pdl_wait();
+      return true;
+    }, halves ? a.epi.ffn + tile_x * 64 : -1);
+    ptx::pdl_launch_dependents();
   } else if (warp == 1) {
-    if (lane == 0) pipe.template issue<kFp8, kScaled>(nkb, a.idesc, a.status);
+    pipe.template issue<kFp8, kScaled>(nkb, a.idesc, a.status);
   } else {
     ptx::pdl_wait();   // scales, split-K scratch and the output belong to the stream's order
     // ---- epilogue (warps 2..5): TMEM lane quarter = warp % 4 -----------------------------------------

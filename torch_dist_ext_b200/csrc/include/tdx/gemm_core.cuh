@@ -152,9 +152,9 @@ struct Pipeline {
     if (status) atomicExch(status, (uint32_t)kTimeoutGemmPipeline);
   }
 
-  // One thread. Streams `nkb` K blocks starting at block `kb0`. `gate_y` is called once, before the
-  // first Y (narrow-side) tile is requested; X tiles of the first ring pass are requested before it,
-  // so that a wait inside the gate overlaps the fetch of the wide operand.
+  // One warp, converged; the copies are issued by one elected lane (tc::elect_one). Streams `nkb` K blocks starting at
+  // block `kb0`. `gate_y` is called once, by one lane, before the first Y (narrow-side) tile is requested; X tiles of the
+  // first ring pass are requested before it, so that a wait inside the gate overlaps the fetch of the wide operand.
   // `x_row1 >= 0`: the X tile is two runs of 64 rows, starting at x_row0 and x_row1, fetched by two copies through a
   // tensor map whose box is 64 rows (the second run lands 8 KB into the stage, where a 128-row box would have put
   // its rows 64-127: the swizzle pattern repeats every 1 KB, so the MMA sees one 128-row tile).
@@ -165,10 +165,11 @@ struct Pipeline {
   }
 
   // The same with the Y tensor map chosen only after the gate has passed (`*parity` odd: my1, else my0), for a Y
-  // operand whose buffer is selected by state that may be read only behind the gate.
+  // operand whose buffer is selected by state that may be read only behind the gate (`parity` in shared memory, written
+  // by the gate).
   template <int kElemsPerBlock, typename Gate>
   __device__ __forceinline__ void produce_late_y(const CUtensorMap* mx, const CUtensorMap* my0, const CUtensorMap* my1,
-                                                 const uint32_t* parity, int x_row0, int y_row0, int kb0, int nkb,
+                                                 const volatile uint32_t* parity, int x_row0, int y_row0, int kb0, int nkb,
                                                  uint32_t* status, Gate gate_y) {
     produce_pick<kElemsPerBlock>(mx, x_row0, y_row0, kb0, nkb, status, gate_y, [=] { return (*parity & 1u) ? my1 : my0; });
   }
@@ -178,47 +179,58 @@ struct Pipeline {
                                                uint32_t* status, Gate gate_y, PickY pick_y, int x_row1 = -1) {
     using L = SmemLayout<kBN, kStages>;
     const int first = nkb < kStages ? nkb : kStages;
-    for (int i = 0; i < first; ++i) {
-      tc::mbar_arrive_expect_tx(&full[i], L::kStageBytes);
-      tc::tma_load_2d(smem + i * L::kStageBytes, mx, &full[i], (kb0 + i) * kElemsPerBlock, x_row0);
-      if (x_row1 >= 0) tc::tma_load_2d(smem + i * L::kStageBytes + L::kXBytes / 2, mx, &full[i], (kb0 + i) * kElemsPerBlock, x_row1);
+    if (tc::elect_one()) {
+      for (int i = 0; i < first; ++i) {
+        tc::mbar_arrive_expect_tx(&full[i], L::kStageBytes);
+        tc::tma_load_2d(smem + i * L::kStageBytes, mx, &full[i], (kb0 + i) * kElemsPerBlock, x_row0);
+        if (x_row1 >= 0) tc::tma_load_2d(smem + i * L::kStageBytes + L::kXBytes / 2, mx, &full[i], (kb0 + i) * kElemsPerBlock, x_row1);
+      }
     }
-    if (!gate_y()) {
+    __syncwarp();
+    bool passed = false;
+    if (tc::elect_one()) passed = gate_y();
+    if (!__any_sync(0xffffffffu, passed)) {
       fail(status);
       return;
     }
     const CUtensorMap* my = pick_y();
-    for (int i = 0; i < first; ++i)
-      tc::tma_load_2d(smem + i * L::kStageBytes + L::kXBytes, my, &full[i], (kb0 + i) * kElemsPerBlock, y_row0);
+    if (tc::elect_one()) {
+      for (int i = 0; i < first; ++i)
+        tc::tma_load_2d(smem + i * L::kStageBytes + L::kXBytes, my, &full[i], (kb0 + i) * kElemsPerBlock, y_row0);
+    }
+    __syncwarp();
     for (int i = first; i < nkb; ++i) {
       const int s = i % kStages;
-      if (!tc::mbar_wait(&empty[s], ((i / kStages) - 1) & 1, kWaitLimit, abort_flag)) {
+      if (!tc::mbar_wait_warp(&empty[s], ((i / kStages) - 1) & 1, kWaitLimit, abort_flag)) {
         fail(status);
         return;
       }
       uint8_t* sx = smem + s * L::kStageBytes;
-      tc::mbar_arrive_expect_tx(&full[s], L::kStageBytes);
-      tc::tma_load_2d(sx, mx, &full[s], (kb0 + i) * kElemsPerBlock, x_row0);
-      if (x_row1 >= 0) tc::tma_load_2d(sx + L::kXBytes / 2, mx, &full[s], (kb0 + i) * kElemsPerBlock, x_row1);
-      tc::tma_load_2d(sx + L::kXBytes, my, &full[s], (kb0 + i) * kElemsPerBlock, y_row0);
+      if (tc::elect_one()) {
+        tc::mbar_arrive_expect_tx(&full[s], L::kStageBytes);
+        tc::tma_load_2d(sx, mx, &full[s], (kb0 + i) * kElemsPerBlock, x_row0);
+        if (x_row1 >= 0) tc::tma_load_2d(sx + L::kXBytes / 2, mx, &full[s], (kb0 + i) * kElemsPerBlock, x_row1);
+        tc::tma_load_2d(sx + L::kXBytes, my, &full[s], (kb0 + i) * kElemsPerBlock, y_row0);
+      }
+      __syncwarp();
     }
   }
 
-  // One thread. kScaled: every K block goes to its own TMEM buffer (two, alternating) and is handed to
+  // One warp, converged; one elected lane issues. kScaled: every K block goes to its own TMEM buffer (two, alternating) and is handed to
   // the epilogue through acc_full/acc_empty; else all blocks accumulate into one buffer.
   template <bool kFp8, bool kScaled>
   __device__ __forceinline__ void issue(int nkb, uint32_t idesc, uint32_t* status) {
     using L = SmemLayout<kBN, kStages>;
     for (int i = 0; i < nkb; ++i) {
       const int s = i % kStages;
-      if (!tc::mbar_wait(&full[s], (i / kStages) & 1, kWaitLimit, abort_flag)) {
+      if (!tc::mbar_wait_warp(&full[s], (i / kStages) & 1, kWaitLimit, abort_flag)) {
         fail(status);
         return;
       }
       uint32_t acc_col = 0;
       if constexpr (kScaled) {
         const int buf = i & 1;
-        if (i >= 2 && !tc::mbar_wait(&acc_empty[buf], ((i >> 1) - 1) & 1, kWaitLimit, abort_flag)) {
+        if (i >= 2 && !tc::mbar_wait_warp(&acc_empty[buf], ((i >> 1) - 1) & 1, kWaitLimit, abort_flag)) {
           fail(status);
           return;
         }
@@ -228,16 +240,19 @@ struct Pipeline {
       const uint32_t xa = tc::smem_u32(smem + s * L::kStageBytes);
       const uint64_t dx = tc::make_smem_desc_sw128(xa);
       const uint64_t dy = tc::make_smem_desc_sw128(xa + L::kXBytes);
+      if (tc::elect_one()) {
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        // one instruction covers 32 bytes of K; step the start address inside the swizzle span
-        const uint32_t accumulate = kScaled ? (k > 0) : (i > 0 || k > 0);
-        tc::umma<kFp8>(tmem_base + acc_col, dx + (uint64_t)(k * 2), dy + (uint64_t)(k * 2), idesc, accumulate);
+        for (int k = 0; k < 4; ++k) {
+          // one instruction covers 32 bytes of K; step the start address inside the swizzle span
+          const uint32_t accumulate = kScaled ? (k > 0) : (i > 0 || k > 0);
+          tc::umma<kFp8>(tmem_base + acc_col, dx + (uint64_t)(k * 2), dy + (uint64_t)(k * 2), idesc, accumulate);
+        }
+        tc::umma_commit(&empty[s]);  // stage reusable once these MMAs have read it
+        if constexpr (kScaled) tc::umma_commit(&acc_full[i & 1]);
+        else if (i + 1 == nkb) tc::umma_commit(&acc_full[0]);
       }
-      tc::umma_commit(&empty[s]);  // stage reusable once these MMAs have read it
-      if constexpr (kScaled) tc::umma_commit(&acc_full[i & 1]);
+      __syncwarp();
     }
-    if constexpr (!kScaled) tc::umma_commit(&acc_full[0]);
   }
 
   // Called by every thread at the end of the kernel.
