@@ -18,6 +18,10 @@
 // in shared memory, so that the scores of chunk i+1 and the P*V product of chunk i-1 run while the softmax
 // warps work on chunk i.
 //
+// Up to eight splits of a (sequence, KV head) are one cluster and merge through distributed shared memory, where the device
+// holds all clusters at a time; more splits, or more clusters, leave partial results in global memory and the split that
+// arrives last at an atomic counter merges them (about 9 us of a launch, the cluster 3).
+//
 // Every wait is bounded; a wait that runs out records a status word, raises the CTA's abort flag
 // (which ends every other wait early) and all threads still reach the common exit, where copies in
 // flight are given time to land and the tensor memory is freed.
@@ -28,6 +32,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <cfloat>
+#include <map>
 #include <mutex>
 #include <set>
 #include <string>
@@ -56,6 +61,8 @@ constexpr uint32_t kTmemCols = 64;                // S^T buffers at columns 0 an
 constexpr uint32_t kColO = 32;
 constexpr uint32_t kWaitLimit = 1u << 22;
 constexpr float kRescaleThreshold = 5.f;          // natural-log units
+constexpr int kMaxCluster = 8;                    // splits that merge inside a cluster (the portable cluster size)
+constexpr int kMergePitch = kD + 4;               // floats per head of a partial result in shared memory: output, maximum, sum
 constexpr int kCounterWords = 4096;               // head of the scratch buffer reserved by the other kernel
 
 struct TcAttnArgs {
@@ -66,6 +73,8 @@ struct TcAttnArgs {
   __nv_bfloat16* out;          // [B, Hq, D]
   int B, Hq, Hkv, nsplit;
   int64_t q_stride_b;
+  int q_vec;                   // every query row starts on a 16-byte boundary
+  int cluster;                 // the splits of a (sequence, KV head) are one cluster and merge through shared memory
   float scale;
   uint32_t idesc_s, idesc_pv;
   uint32_t* status;
@@ -99,13 +108,8 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
 
   const int b = blockIdx.x, hkv = blockIdx.y, split = blockIdx.z;
   const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
-  ptx::pdl_wait();                // q, the caches and seq_lens come from earlier kernels of the stream
-  ptx::pdl_launch_dependents();
-  const int len = a.seq_lens[b];
-  const int per = (len + a.nsplit - 1) / a.nsplit;
-  const int s0 = split * per, s1 = min(len, s0 + per);
-  const int nchunks = s1 > s0 ? (s1 - s0 + kKeys - 1) / kKeys : 0;
 
+  // what touches no memory of an earlier kernel comes before the wait for it
   if (tid == 0) {
     for (int s = 0; s < kStages; ++s) {
       tc::mbar_init(&kv_full[s], 1);
@@ -124,19 +128,28 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
     tc::tma_prefetch_desc(&map_k);
     tc::tma_prefetch_desc(&map_v);
   }
-  // Q and P tiles: zero everything (rows beyond the G real heads stay zero), then the query rows
+  // Q and P tiles: rows beyond the G real heads stay zero
   for (int i = tid; i < 3 * kSmallTileBytes / 16; i += kThreads) reinterpret_cast<uint4*>(q_tile)[i] = make_uint4(0, 0, 0, 0);
-  __syncthreads();
-  for (int i = tid; i < kG * kD; i += kThreads) {
-    const int g = i / kD, d = i % kD;
-    *reinterpret_cast<__nv_bfloat16*>(q_tile + small_tile_offset(g, d)) =
-        a.q[(int64_t)b * a.q_stride_b + (int64_t)(hkv * kG + g) * kD + d];
-  }
-  tc::fence_proxy_async();   // the tiles were written by threads and are read by the tensor core
   if (warp == 4) {
     tc::tmem_alloc(tmem_slot, kTmemCols);
     tc::tmem_relinquish();
   }
+  __syncthreads();
+  ptx::pdl_wait();                // q, the caches and seq_lens come from earlier kernels of the stream
+  ptx::pdl_launch_dependents();
+  const int len = a.seq_lens[b];
+  const int per = (len + a.nsplit - 1) / a.nsplit;
+  const int s0 = split * per, s1 = min(len, s0 + per);
+  const int nchunks = s1 > s0 ? (s1 - s0 + kKeys - 1) / kKeys : 0;
+  const __nv_bfloat16* q_rows = a.q + (int64_t)b * a.q_stride_b + (int64_t)(hkv * kG) * kD;
+  if (a.q_vec) {
+    for (int i = tid; i < kG * (kD / 8); i += kThreads)
+      *reinterpret_cast<uint4*>(q_tile + small_tile_offset(i / (kD / 8), i % (kD / 8) * 8)) = ptx::ld_v4(q_rows + i * 8);
+  } else {
+    for (int i = tid; i < kG * kD; i += kThreads)
+      *reinterpret_cast<__nv_bfloat16*>(q_tile + small_tile_offset(i / kD, i % kD)) = q_rows[i];
+  }
+  tc::fence_proxy_async();   // the tiles were written by threads and are read by the tensor core
   tc::fence_before_thread_sync();
   __syncthreads();
   tc::fence_after_thread_sync();
@@ -316,7 +329,14 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
 #pragma unroll
     for (int g = 0; g < kG; ++g) {
       const int h = hkv * kG + g;
-      if (a.nsplit == 1) {
+      if (a.cluster) {
+        float* mine = reinterpret_cast<float*>(ring) + g * kMergePitch;     // no copy is in flight any more
+        mine[tid] = o[g];
+        if (tid == 0) {
+          mine[kD] = m_run[g];
+          mine[kD + 1] = l_run[g];
+        }
+      } else if (a.nsplit == 1) {
         a.out[((int64_t)b * a.Hq + h) * kD + tid] = __float2bfloat16(l_run[g] > 0.f ? o[g] / l_run[g] : 0.f);
       } else {
         float* dst = a.partial + (((int64_t)b * a.Hq + h) * a.nsplit + split) * (kD + 2);
@@ -327,7 +347,7 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
         }
       }
     }
-    if (a.nsplit > 1 && a.counters != nullptr) {
+    if (a.nsplit > 1 && !a.cluster && a.counters != nullptr) {
       // the split that arrives last merges all of them (saves a launch per layer)
       __threadfence();
       tc::named_barrier_sync(1, kSoftmaxThreads);
@@ -391,6 +411,41 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
   if (*abort_flag) {
     for (int i = 0; i < 64; ++i) __nanosleep(1000);   // copies already issued land before shared memory goes away
   }
+  if (a.cluster) {
+    // The splits of this (sequence, KV head) are the cluster: split s merges the heads s, s + nsplit, ... out of the
+    // others' shared memory.
+    tc::cluster_arrive();
+    tc::cluster_wait();
+    if (warp < 4) {
+      const uint32_t base = tc::smem_u32(ring);
+      for (int g = split; g < kG; g += a.nsplit) {
+        float ov[kMaxCluster], mv[kMaxCluster], lv[kMaxCluster];
+#pragma unroll
+        for (int u = 0; u < kMaxCluster; ++u) {
+          if (u >= a.nsplit) continue;
+          const uint32_t row = tc::map_to_cta(base + g * (kMergePitch * 4), u);
+          ov[u] = tc::ld_cluster_f1(row + tid * 4);
+          mv[u] = tc::ld_cluster_f1(row + kD * 4);
+          lv[u] = tc::ld_cluster_f1(row + kD * 4 + 4);
+        }
+        float m = -FLT_MAX;
+#pragma unroll
+        for (int u = 0; u < kMaxCluster; ++u)
+          if (u < a.nsplit) m = fmaxf(m, mv[u]);
+        float num = 0.f, den = 0.f;
+#pragma unroll
+        for (int u = 0; u < kMaxCluster; ++u) {
+          if (u >= a.nsplit) continue;
+          const float wgt = __expf(mv[u] - m);
+          num = fmaf(wgt, ov[u], num);
+          den = fmaf(wgt, lv[u], den);
+        }
+        a.out[((int64_t)b * a.Hq + hkv * kG + g) * kD + tid] = __float2bfloat16(den > 0.f ? num / den : 0.f);
+      }
+    }
+    tc::cluster_arrive();
+    tc::cluster_wait();       // no CTA leaves while another may still read its partial result
+  }
   if (warp == 4) {
     tc::fence_after_thread_sync();
     tc::tmem_dealloc(tmem_base, kTmemCols);
@@ -415,15 +470,65 @@ __global__ void __launch_bounds__(kD) attn_tc_combine_kernel(const TcAttnArgs a)
 }
 
 template <int kG>
+cudaLaunchConfig_t config(const TcAttnArgs& a, dim3 grid, cudaStream_t stream, cudaLaunchAttribute (&attr)[2]) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = kSmem;
+  cfg.stream = stream;
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 1;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = a.cluster ? a.nsplit : 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl_enabled() ? 2 : 1;
+  return cfg;
+}
+
+template <int kG>
 std::string launch(const CUtensorMap& mk, const CUtensorMap& mv, const TcAttnArgs& a, dim3 grid, cudaStream_t stream) {
   auto kern = attn_decode_tc_kernel<kG>;
   const std::string smem_err = reserve_dynamic_smem(kern, kSmem);
   if (!smem_err.empty()) return smem_err;
-  const cudaError_t e = launch_chained(kern, grid, dim3(kThreads), kSmem, stream, mk, mv, a);
+  cudaLaunchAttribute attr[2];
+  const cudaLaunchConfig_t cfg = config<kG>(a, grid, stream, attr);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, mk, mv, a);
   return e == cudaSuccess ? "" : std::string("attention launch failed: ") + cudaGetErrorString(e);
 }
 
 }  // namespace
+
+// How many clusters of `nsplit` splits the current device holds at a time (0: such splits merge through global memory).
+int attention_decode_clusters(int nsplit) {
+  if (nsplit < 2 || nsplit > kMaxCluster) return 0;
+  static std::mutex mu;
+  static std::map<std::pair<int, int>, int> known;
+  int dev = 0, n = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  std::lock_guard<std::mutex> lock(mu);
+  const auto it = known.find({dev, nsplit});
+  if (it != known.end()) return it->second;
+  auto kern = attn_decode_tc_kernel<kMaxG>;
+  if (reserve_dynamic_smem(kern, kSmem).empty()) {
+    TcAttnArgs a{};
+    a.cluster = 1;
+    a.nsplit = nsplit;
+    cudaLaunchAttribute attr[2];
+    cudaLaunchConfig_t cfg = config<kMaxG>(a, dim3(1, 1, nsplit), nullptr, attr);
+    cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      n = 0;
+    }
+  }
+  known[{dev, nsplit}] = n;
+  return n;
+}
 
 std::string attention_decode_tc(const void* q, const void* k_cache, const void* v_cache, const int32_t* seq_lens,
                                 float* partial, size_t partial_floats, void* out, int B, int Hq, int Hkv, int D, int S_max,
@@ -450,6 +555,8 @@ std::string attention_decode_tc(const void* q, const void* k_cache, const void* 
   a.out = static_cast<__nv_bfloat16*>(out);
   a.B = B; a.Hq = Hq; a.Hkv = Hkv; a.nsplit = nsplit;
   a.q_stride_b = q_stride_b;
+  a.q_vec = reinterpret_cast<uintptr_t>(q) % 16 == 0 && (q_stride_b * 2) % 16 == 0;
+  a.cluster = nsplit > 1 && B * Hkv <= attention_decode_clusters(nsplit);
   a.scale = scale;
   a.idesc_s = tc::make_idesc(kKeys, kNq, 1, 1);                    // both operands K-major bf16
   a.idesc_pv = tc::make_idesc(kD, kNq, 1, 1) | tc::kIdescAMnMajor;         // A (the V chunk) is read MN-major
@@ -467,7 +574,7 @@ std::string attention_decode_tc(const void* q, const void* k_cache, const void* 
     case 8: err = launch<8>(mk, mv, a, grid, stream); break;
   }
   if (!err.empty()) return err;
-  if (nsplit > 1 && !in_kernel_merge) launch_chained(attn_tc_combine_kernel, dim3(B, Hq), dim3(kD), 0, stream, a);
+  if (nsplit > 1 && !a.cluster && !in_kernel_merge) launch_chained(attn_tc_combine_kernel, dim3(B, Hq), dim3(kD), 0, stream, a);
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? "" : cudaGetErrorString(e);
 }

@@ -104,23 +104,38 @@ __global__ void __launch_bounds__(256) silu_mul_kernel(const T* __restrict__ in,
   const int nvec = inter / kVec;
   const size_t total = (size_t)rows * nvec;
   const size_t stride = (size_t)gridDim.x * blockDim.x;
-  // Warp-uniform trip count: the quantising variant shuffles inside the loop.
-  for (size_t base = (size_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < total; base += stride) {
-    const size_t idx = base + (threadIdx.x & 31u);
-    const bool live = idx < total;
-    const size_t row = live ? idx / nvec : 0;
-    const int i = live ? int(idx % nvec) : 0;
+  // Row and column of this thread's vector are carried along (one division per thread, not one per vector), and the next
+  // vectors are requested before the current ones are used. Warp-uniform trip count: the quantising variant shuffles
+  // inside the loop.
+  const size_t first = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  size_t row = first / nvec;
+  int i = int(first % nvec);
+  const size_t row_step = stride / nvec;
+  const int col_step = int(stride % nvec);
+  const size_t row_bytes = (size_t)inter * sizeof(T);
+  uint4 gate = make_uint4(0u, 0u, 0u, 0u), up = gate;
+  auto request = [&](size_t r, int col) {
+    const char* src = reinterpret_cast<const char*>(in) + r * 2 * row_bytes + (size_t)col * 16;
+    gate = ptx::ld_stream_v4(src);
+    up = ptx::ld_stream_v4(src + row_bytes);
+  };
+  if (first < total) request(row, i);
+  for (size_t base = first & ~(size_t)31; base < total; base += stride) {
+    const bool live = base + (threadIdx.x & 31u) < total;
     float g[kVec], u[kVec], y[kVec];
-    if (live) {
-      const char* base = reinterpret_cast<const char*>(in + row * 2 * (size_t)inter);
-      unpack<T>(ptx::ld_stream_v4(base + (size_t)i * 16), g);
-      unpack<T>(ptx::ld_stream_v4(base + (size_t)inter * sizeof(T) + (size_t)i * 16), u);
-#pragma unroll
-      for (int k = 0; k < kVec; ++k) y[k] = g[k] / (1.f + __expf(-g[k])) * u[k];
-    } else {
-#pragma unroll
-      for (int k = 0; k < kVec; ++k) y[k] = 0.f;
+    unpack<T>(gate, g);
+    unpack<T>(up, u);
+    const size_t at_row = row;
+    const int at = i;
+    row += row_step;
+    i += col_step;
+    if (i >= nvec) {
+      i -= nvec;
+      ++row;
     }
+    if (base + stride + (threadIdx.x & 31u) < total) request(row, i);
+#pragma unroll
+    for (int k = 0; k < kVec; ++k) y[k] = live ? g[k] / (1.f + __expf(-g[k])) * u[k] : 0.f;
     if constexpr (kQuant) {
       constexpr int kLanes = 128 / kVec;
       round_through<T>(y);  // quantise what a separate kernel would have stored in T
@@ -134,11 +149,11 @@ __global__ void __launch_bounds__(256) silu_mul_kernel(const T* __restrict__ in,
       if (live) {
 #pragma unroll
         for (int k = 0; k < kVec; ++k) y[k] *= inv;
-        store_fp8_vec<kVec>(static_cast<uint8_t*>(out) + row * inter + (size_t)i * kVec, y);
-        if ((i & (kLanes - 1)) == 0) scales[row * (inter / 128) + (size_t)i * kVec / 128] = scale;
+        store_fp8_vec<kVec>(static_cast<uint8_t*>(out) + at_row * inter + (size_t)at * kVec, y);
+        if ((at & (kLanes - 1)) == 0) scales[at_row * (inter / 128) + (size_t)at * kVec / 128] = scale;
       }
     } else {
-      if (live) ptx::st_stream_v4(static_cast<char*>(out) + (row * inter + (size_t)i * kVec) * sizeof(T), pack<T>(y));
+      if (live) ptx::st_stream_v4(static_cast<char*>(out) + (at_row * inter + (size_t)at * kVec) * sizeof(T), pack<T>(y));
     }
   }
 }

@@ -245,12 +245,23 @@ __device__ __forceinline__ uint4 poll_vec(const char* addr, Waiter& w, const ArP
 
 // ---- local (single rank): residual add + RMSNorm (+ quant) --------------------------------
 
+// Bound by memory. A block walks several rows of a large message, and the vectors of its next row are requested before
+// the block-wide reduction of the current one, so that loads are in flight while the block meets at the barriers.
 template <typename T, int kVpt, int kOut>
 __device__ __forceinline__ void local_body(const ArParams& p) {
   constexpr int kVec = VecTraits<T>::kVec;
   __shared__ float red[4][32];
   const RowView<T, kVpt> rv(p.hidden);
-  uint4 gamma[kVpt];
+  uint4 gamma[kVpt], in[kVpt], res[kVpt];
+  auto request = [&](int row) {
+#pragma unroll
+    for (int v = 0; v < kVpt; ++v) {
+      if (rv.active(v))
+        in[v] = ptx::ld_stream_v4(static_cast<const char*>(p.in) + (size_t)row * rv.row_bytes + (size_t)rv.vec_index(v) * 16);
+    }
+    request_residual<T, kVpt>(p, rv, row, res);
+  };
+  if ((int)blockIdx.x < p.tokens) request(blockIdx.x);
   load_gamma<T, kVpt>(p, rv, gamma);
   int parity = 0;
   for (int row = blockIdx.x; row < p.tokens; row += gridDim.x, parity ^= 1) {
@@ -258,15 +269,16 @@ __device__ __forceinline__ void local_body(const ArParams& p) {
 #pragma unroll
     for (int v = 0; v < kVpt; ++v) {
       if (rv.active(v)) {
-        const size_t off = (size_t)row * rv.row_bytes + (size_t)rv.vec_index(v) * 16;
-        unpack<T>(ptx::ld_stream_v4(static_cast<const char*>(p.in) + off), x[v]);
-        add_residual<T>(x[v], p.residual_in ? static_cast<const char*>(p.residual_in) + off : nullptr);
-        if (p.residual_out) ptx::st_stream_v4(static_cast<char*>(p.residual_out) + off, pack<T>(x[v]));
+        unpack<T>(in[v], x[v]);
+        add_residual_loaded<T>(x[v], p.residual_in != nullptr, res[v]);
+        if (p.residual_out)
+          ptx::st_stream_v4(static_cast<char*>(p.residual_out) + (size_t)row * rv.row_bytes + (size_t)rv.vec_index(v) * 16, pack<T>(x[v]));
       } else {
 #pragma unroll
         for (int i = 0; i < kVec; ++i) x[v][i] = 0.f;
       }
     }
+    if (row + (int)gridDim.x < p.tokens) request(row + gridDim.x);
     float rstd, sc;
     finish_row<T, kVpt, kOut>(p, rv, row, x, gamma, red, parity, rstd, sc);
   }

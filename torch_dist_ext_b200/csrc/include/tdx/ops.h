@@ -49,6 +49,9 @@ std::string attention_decode_tc(const void* q, const void* k_cache, const void* 
                                 float* partial, size_t partial_floats, void* out, int B, int Hq, int Hkv, int D, int S_max,
                                 int64_t q_stride_b, int64_t kv_stride_b, int64_t kv_stride_s, int nsplit, float scale,
                                 cudaStream_t stream, uint32_t* status = nullptr);
+// How many clusters of `nsplit` of its CTAs the current device holds at a time: with at most that many (sequence, KV head)
+// pairs the splits merge inside clusters. 0 where they never do (one split, more than eight, no device).
+int attention_decode_clusters(int nsplit);
 
 // Causal self-attention over one prompt on the tensor cores (attention_prefill_tc.cu): q [S, Hq, 128],
 // k / v [S, Hkv, 128] bf16 with unit stride inside a head, heads 128 elements apart and rows `*_stride_s`

@@ -535,6 +535,7 @@ void register_extra_ops(torch::Library& m) {
         "int nsplit, float scale, Tensor(c!)? status) -> ()", &attention_decode);
   m.def("attention_decode_tc(Tensor q, Tensor k_cache, Tensor v_cache, Tensor seq_lens, Tensor(a!) out, Tensor(b!) partial, "
         "int nsplit, float scale, Tensor(c!)? status) -> ()", &attention_decode_tc);
+  m.def("attention_decode_clusters(int nsplit) -> int", [](int64_t nsplit) -> int64_t { return tdx::attention_decode_clusters((int)nsplit); });
   m.def("attention_prefill_tc(Tensor q, Tensor k, Tensor v, Tensor(a!) out, float scale, Tensor(b!)? status) -> ()",
         &attention_prefill_tc);
   m.def("ag_gemm(Tensor x_shard, Tensor w, Tensor(a!) out, int tokens, Tensor workspace, Tensor(b!)? status) -> ()", &ag_gemm);

@@ -31,13 +31,32 @@ def _partial(device, floats: int) -> torch.Tensor:
 _CHUNK_US, _CHUNK_US_PER_CTA, _UNSPLIT_US, _SPLIT_US, _PER_SPLIT_US = 1.0, 0.0131, 2.6, 9.0, 0.4
 
 
-def _split_cost_us(pairs: int, chunks: int, nsplit: int) -> float:
+# Splits that merge inside a cluster pay about 4.7 us, however many they are (1 x 2000 positions, 8 heads on one KV head:
+# 19.8 us unsplit, 9.1 in 4, 7.0 in 8 splits; 19.2 in 8 splits that merge through global memory).
+_CLUSTER_US = 4.7
+
+
+def _split_cost_us(pairs: int, chunks: int, nsplit: int, in_cluster: bool = False) -> float:
     ctas = pairs * nsplit
     per_chunk = max(_CHUNK_US, _CHUNK_US_PER_CTA * ctas)
-    return -(-chunks // nsplit) * per_chunk + (_UNSPLIT_US if nsplit == 1 else _SPLIT_US + _PER_SPLIT_US * nsplit)
+    fixed = _UNSPLIT_US if nsplit == 1 else _CLUSTER_US if in_cluster else _SPLIT_US + _PER_SPLIT_US * nsplit
+    return -(-chunks // nsplit) * per_chunk + fixed
 
 
-def pick_splits(batch: int, kv_heads: int, max_len: int, sms: int = 148, ctas_per_sm: int = 2) -> int:
+_clusters = {}
+
+
+def _resident_clusters(device: torch.device) -> dict:
+    """{splits: clusters of so many CTAs of the tensor-core kernel that the device holds at a time}."""
+    key = device.index if device.index is not None else torch.cuda.current_device()
+    if key not in _clusters:
+        with torch.cuda.device(key):
+            _clusters[key] = {n: int(_lib.ops().attention_decode_clusters(n)) for n in range(2, 9)}
+    return _clusters[key]
+
+
+def pick_splits(batch: int, kv_heads: int, max_len: int, sms: int = 148, ctas_per_sm: int = 2,
+                clusters: Optional[dict] = None) -> int:
     """KV splits of at least 128 positions each, such that the grid fits ONE wave of the CTAs that the SMs hold at a
     time (two per SM for the SIMT kernel, one for the tensor-core kernel; a second, partly filled wave costs more than
     shorter splits save).
@@ -45,13 +64,15 @@ def pick_splits(batch: int, kv_heads: int, max_len: int, sms: int = 148, ctas_pe
     The SIMT kernel takes the most splits that fit. The tensor-core kernel (``ctas_per_sm=1``) takes the split count
     with the least estimated time: a split that leaves some CTAs one chunk more than others (16 chunks over 9 splits)
     is no faster than the next count that divides evenly (8), and once the unsplit grid already covers a third of
-    the SMs (64 sequences on one KV head) the merge costs more than the shorter loops save."""
+    the SMs (64 sequences on one KV head) the merge costs more than the shorter loops save. ``clusters`` ({splits:
+    clusters the device holds}) says which split counts merge inside clusters, which is cheaper."""
     pairs = batch * kv_heads
     chunks = max(1, (max_len + 127) // 128)
     most = max(1, min((ctas_per_sm * sms) // pairs, chunks))
     if ctas_per_sm != 1:
         return most
-    return min(range(1, most + 1), key=lambda n: (_split_cost_us(pairs, chunks, n), n))
+    fits = clusters or {}
+    return min(range(1, most + 1), key=lambda n: (_split_cost_us(pairs, chunks, n, pairs <= fits.get(n, 0)), n))
 
 
 @traced("tdx.decode_attention")
@@ -66,7 +87,7 @@ def decode_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tens
     hkv = k_cache.shape[2]
     use_tc = _TC_DEFAULT if tensor_cores is None else tensor_cores
     if nsplit is None:
-        nsplit = pick_splits(b, hkv, max_len, ctas_per_sm=1 if use_tc else 2)
+        nsplit = pick_splits(b, hkv, max_len, ctas_per_sm=1 if use_tc else 2, clusters=_resident_clusters(q.device) if use_tc else None)
     out = torch.empty(b, hq, d, dtype=q.dtype, device=q.device) if out is None else out
     part = _partial(q.device, 4096 + b * hq * nsplit * (d + 2))
     from . import gemm as _gemm
