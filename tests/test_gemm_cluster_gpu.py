@@ -1,0 +1,34 @@
+"""Decode GEMMs whose K splits meet inside a cluster: uneven splits, ragged rows and columns, every output type and the
+pair epilogues, against 64-bit PyTorch math; and the same call with its splits meeting in global memory."""
+import pytest
+import torch
+
+from torch_dist_ext_b200.ops import gemm
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("m,n,k", [
+    (1, 128, 128),       # two K blocks, two splits
+    (3, 130, 576),       # nine K blocks over eight splits; two rows in the second tile
+    (17, 768, 4096),     # six tiles of eight splits
+    (64, 4096, 1792),    # 28 K blocks over four splits
+    (100, 3584, 4096),   # ragged columns of a 128-wide tile
+    (128, 9472, 128),    # 74 tiles, as many as there are clusters of two
+    (33, 9600, 256),     # 75 tiles: no room for clusters, one split
+])
+@pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32])
+def test_cluster_splits_match_64_bit(m, n, k, out_dtype):
+    g = torch.Generator(device="cuda").manual_seed(m + n + k)
+    a = torch.randn(m, k, device="cuda", generator=g).to(torch.bfloat16)
+    w = (torch.randn(n, k, device="cuda", generator=g) * 0.05).to(torch.bfloat16)
+    want = a.double() @ w.double().t()
+    outs = [gemm.linear(a, w, out_dtype=out_dtype) for _ in range(2)]
+    torch.cuda.synchronize()
+    assert gemm.pipeline_status() == 0
+    assert torch.equal(outs[0], outs[1]), "the splits are added in a fixed order"
+    # bf16: half a rounding step (2^-9) of the largest value, doubled; fp32: 2^-24 per addition along K, with a margin of 4
+    bound = want.abs().max() * (2.0 ** -8 if out_dtype == torch.bfloat16 else k * 2.0 ** -22)
+    assert (outs[0].double() - want).abs().max() <= bound
+    ws, counters, _ = gemm._workspace(a.device)
+    assert float(ws.abs().max()) == 0.0 and int(counters.abs().sum()) == 0

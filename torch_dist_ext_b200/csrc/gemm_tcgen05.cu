@@ -29,7 +29,10 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <cstdlib>
+#include <map>
 #include <mutex>
+#include <string>
+#include <tuple>
 #include "tdx/comm.h"
 #include "tdx/gemm.h"
 #include "tdx/gemm_core.cuh"
@@ -66,6 +69,7 @@ struct GemmArgs {
   const float* y_scale;
   int x_scale_per_row, y_scale_per_row;
   int scale_kb;            // K blocks per scale row (= total K / 128)
+  int cluster;             // the K splits of a tile are one cluster and meet in shared memory (ws and counters unused)
   int x_static;            // X is never written by a kernel (weights): its first tiles may be requested before the
                            // previous kernel of the stream has finished
   PairEpilogue epi;        // what the split-K finalizer does with rows r and r + 64 of a tile (kEpiNone: plain store)
@@ -155,10 +159,87 @@ __device__ __forceinline__ void pair_finalize(const GemmArgs& a, int tile_x, flo
   }
 }
 
+// ---- K splits that are one cluster -------------------------------------------------------------------------
+// Every CTA has left its 128 x kBN sums in its shared memory ([column][128 rows]) and passed the cluster barrier. CTA
+// `rank` finishes the columns rank * kBN / splits ..: its 128 epilogue threads (`t`) add up the splits' values in the
+// order of the splits and store, rotate or activate them.
+constexpr int kMaxCluster = 8;
+
+template <int kCols>
+__device__ __forceinline__ void cluster_sums(uint32_t base, int splits, int column, int row, float (&sum)[kCols]) {
+  float v[kCols][kMaxCluster];
+#pragma unroll
+  for (int p = 0; p < kMaxCluster; ++p) {
+    if (p >= splits) continue;
+    const uint32_t src = tc::map_to_cta(base + (uint32_t)((column * kBM + row) * 4), p);
+#pragma unroll
+    for (int j = 0; j < kCols; ++j) v[j][p] = tc::ld_cluster_f1(src + j * (kBM * 4));
+  }
+#pragma unroll
+  for (int j = 0; j < kCols; ++j) {
+    sum[j] = 0.f;
+#pragma unroll
+    for (int p = 0; p < kMaxCluster; ++p)
+      if (p < splits) sum[j] += v[j][p];
+  }
+}
+
+template <int kBN>
+__device__ __forceinline__ void cluster_finalize(const GemmArgs& a, uint32_t base, int tile_x, int y_base, int rank, int splits, int t) {
+  const int share = (kBN + splits - 1) / splits;
+  const int c0 = rank * share, c1 = min(min(kBN, c0 + share), a.y_rows - y_base);
+  const PairEpilogue& e = a.epi;
+  if (e.kind == kEpiNone) {
+    const int x = tile_x * kBM + t;
+    for (int c = c0; c < c1; c += 2) {
+      float s[2];
+      cluster_sums<2>(base, splits, c, t, s);      // an odd share's last column is followed by one that is in bounds too
+      if (x >= a.x_rows) continue;
+      gemm_core::store_out(a, (int64_t)x * a.sx + (int64_t)(y_base + c) * a.sy, s[0]);
+      if (c + 1 < c1) gemm_core::store_out(a, (int64_t)x * a.sx + (int64_t)(y_base + c + 1) * a.sy, s[1]);
+    }
+    return;
+  }
+  // rows r and r + 64 belong together; the two halves of the threads take alternate columns
+  const int r = t & 63;
+  const bool rope = e.kind == kEpiRopeKv;
+  const bool is_q = tile_x < e.q_heads, is_v = tile_x >= e.q_heads + e.kv_heads;
+  __nv_bfloat16* cache = (!rope || is_q) ? nullptr : static_cast<__nv_bfloat16*>(is_v ? e.v_cache : e.k_cache);
+  const int kv_head = tile_x - e.q_heads - (is_v ? e.kv_heads : 0);
+  const int64_t x_lo = rope ? (int64_t)tile_x * kBM + r : (int64_t)tile_x * 64 + r;
+  for (int c = c0 + (t >> 6); c < c1; c += 2) {
+    const int y = y_base + c;
+    const int pos = rope ? (int)__ldg(e.positions + y) : 0;
+    float lo[1], hi[1];
+    cluster_sums<1>(base, splits, c, r, lo);
+    cluster_sums<1>(base, splits, c, r + 64, hi);
+    const int64_t at = x_lo * a.sx + (int64_t)y * a.sy;
+    if (!rope) {   // silu(gate) * up
+      gemm_core::store_out(a, at, lo[0] / (1.f + __expf(-lo[0])) * hi[0]);
+      continue;
+    }
+    float o_lo = lo[0], o_hi = hi[0];
+    if (!is_v) {
+      const int p = pos < 0 ? 0 : (pos >= e.max_pos ? e.max_pos - 1 : pos);
+      const float cs = __ldg(e.cos_sin + (int64_t)p * 128 + r), sn = __ldg(e.cos_sin + (int64_t)p * 128 + 64 + r);
+      o_lo = lo[0] * cs - hi[0] * sn;
+      o_hi = hi[0] * cs + lo[0] * sn;
+    }
+    gemm_core::store_out(a, at, o_lo);
+    gemm_core::store_out(a, at + 64 * a.sx, o_hi);
+    if (cache != nullptr && pos >= 0 && pos < e.cache_seq) {
+      __nv_bfloat16* dst = cache + (int64_t)y * e.cache_batch_stride + (int64_t)pos * e.cache_pos_stride + kv_head * 128 + r;
+      dst[0] = __float2bfloat16(o_lo);
+      dst[64] = __float2bfloat16(o_hi);
+    }
+  }
+}
+
 template <int kBN, int kStages, bool kFp8, bool kScaled>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_tn_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_y, const GemmArgs a) {
   using L = SmemLayout<kBN, kStages>;
+  static_assert(kBN * kBM * 4 <= L::kBarrierOffset, "the sums of a cluster's CTA take the ring's place");
   constexpr int kElemsPerBlock = kFp8 ? 128 : 64;   // K elements per 128-byte block
   constexpr uint32_t kTmemCols = kScaled ? (2 * kBN < 32 ? 32 : 2 * kBN) : (kBN < 32 ? 32 : kBN);
   static_assert((kTmemCols & (kTmemCols - 1)) == 0 && kTmemCols <= 512, "TMEM columns must be a power of two");
@@ -251,6 +332,11 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
         }
         if (!split) {
           store_chunk(a, x, y_base + c, v);
+        } else if (a.cluster) {
+          // every MMA has read its operands: the sums take the ring's place
+          float* sums = reinterpret_cast<float*>(pipe.smem) + c * kBM + q * 32 + lane;
+#pragma unroll
+          for (int j = 0; j < 16; ++j) sums[j * kBM] = v[j];
         } else {
           // scratch tile is column-major ([column][128 rows]): the lanes of a warp add to 32
           // consecutive floats, one 128-byte line per instruction
@@ -261,8 +347,8 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
       }
     }
     int pair_pos[PairShape<kBN>::kW] = {};
-    if (split && a.epi.kind == kEpiRopeKv) pair_positions<PairShape<kBN>::kW>(a, y_base + (q >> 1) * PairShape<kBN>::kHalf, pair_pos);
-    if (split) {
+    if (split && !a.cluster && a.epi.kind == kEpiRopeKv) pair_positions<PairShape<kBN>::kW>(a, y_base + (q >> 1) * PairShape<kBN>::kHalf, pair_pos);
+    if (split && !a.cluster) {
       // the CTA that arrives last at this tile turns the fp32 sums into the output and re-zeroes them
       __threadfence();
       tc::named_barrier_sync(1, 128);
@@ -294,18 +380,84 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
     }
   }
 
+  if (a.cluster) {
+    __syncwarp();
+    tc::cluster_arrive();
+    tc::cluster_wait();
+    if (warp >= 2 && !*abort_flag)
+      cluster_finalize<kBN>(a, tc::smem_u32(pipe.smem), tile_x, tile_y * kBN, blockIdx.z, gridDim.z, threadIdx.x - 64);
+    __syncwarp();
+    tc::cluster_arrive();
+    tc::cluster_wait();        // no CTA leaves while another may still read its sums
+  }
   pipe.finish(kTmemCols);
 }
 
 // ---- host side -------------------------------------------------------------------------------------
 
+// How many clusters of `splits` CTAs of a kernel the current device holds at a time.
+template <typename Kernel>
+int resident_clusters(Kernel kern, int smem, int splits) {
+  static std::mutex mu;
+  static std::map<std::tuple<const void*, int, int>, int> known;
+  int dev = 0, n = 0;
+  cudaGetDevice(&dev);
+  const auto key = std::make_tuple(reinterpret_cast<const void*>(kern), dev, splits);
+  std::lock_guard<std::mutex> lock(mu);
+  const auto it = known.find(key);
+  if (it != known.end()) return it->second;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(1, 1, splits);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = smem;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 1;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = splits;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    n = 0;
+  }
+  known[key] = n;
+  return n;
+}
+
 template <int kBN, int kStages, bool kFp8, bool kScaled>
-std::string launch(const CUtensorMap& mx, const CUtensorMap& my, const GemmArgs& a, dim3 grid, cudaStream_t stream) {
+std::string launch(const CUtensorMap& mx, const CUtensorMap& my, GemmArgs a, dim3 grid, cudaStream_t stream) {
   using L = SmemLayout<kBN, kStages>;
   auto kern = gemm_tn_kernel<kBN, kStages, kFp8, kScaled>;
   const std::string err = reserve_dynamic_smem(kern, L::kTotal);
   if (!err.empty()) return err;
-  const cudaError_t e = launch_chained(kern, grid, dim3(kThreads), L::kTotal, stream, mx, my, a);
+  // K splits meet inside a cluster where the device holds one cluster per tile at a time: as many splits as were asked
+  // for, at most eight.
+  const int tiles = grid.x * grid.y;
+  for (int want = (int)grid.z < kMaxCluster ? grid.z : kMaxCluster; want >= 2; --want) {
+    const int per = (a.kblocks + want - 1) / want, splits = (a.kblocks + per - 1) / per;
+    if (splits < 2) break;
+    if (tiles > resident_clusters(kern, L::kTotal, splits)) continue;
+    a.cluster = 1;
+    a.kblocks_per_split = per;
+    grid.z = splits;
+    break;
+  }
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = L::kTotal;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 1;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = a.cluster ? grid.z : 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl_enabled() ? 2 : 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, mx, my, a);
   return e == cudaSuccess ? "" : std::string("GEMM launch failed: ") + cudaGetErrorString(e);
 }
 
