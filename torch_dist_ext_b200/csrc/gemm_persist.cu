@@ -1,8 +1,9 @@
-// Persistent tcgen05 GEMM for prefill-sized problems:  D[x, y] = sum_k X[x, k] * Y[y, k], both K-major.
+// Persistent tcgen05 GEMM:  D[x, y] = sum_k X[x, k] * Y[y, k], both K-major; prompts (128 < M < 256: 128 x 256 tiles), and
+// decode-sized products with more 128-row weight tiles than SMs (128 x 16 .. 128 x 128, the weights as X).
 //
-// One CTA per SM walks the 128 x 256 output tiles t = blockIdx.x, blockIdx.x + gridDim.x, ... The
+// One CTA per SM walks the output tiles t = blockIdx.x, blockIdx.x + gridDim.x, ... The
 // operand ring (TMA -> 128-byte-swizzled shared memory) keeps streaming across tile boundaries, and
-// the accumulator is double-buffered in tensor memory (2 x 256 columns): while the epilogue warps read
+// the accumulator is double-buffered in tensor memory: while the epilogue warps read
 // tile n back with tcgen05.ld and store it, the MMA thread is already accumulating tile n + 1. The
 // one-tile-per-CTA kernel (gemm_tcgen05.cu) pays a pipeline fill, a drain and a serial epilogue per
 // tile; here they are paid once per CTA.
@@ -38,15 +39,17 @@ using gemm_core::store_chunk;
 
 constexpr int kThreads = 192;
 constexpr int kBM = 128;
-constexpr int kBN = 256;
-constexpr int kStages = 4;
 constexpr int kXBytes = kBM * 128;
-constexpr int kYBytes = kBN * 128;
-constexpr int kStageBytes = kXBytes + kYBytes;          // 48 KB
-constexpr int kBarrierOffset = kStages * kStageBytes;
-constexpr int kSmemTotal = kBarrierOffset + 1024 /* barriers */ + 1024 /* alignment slack */;
-constexpr uint32_t kTmemCols = 2 * kBN;                 // two accumulator buffers
 constexpr uint32_t kWaitLimit = 1u << 22;
+
+template <int kBN>
+struct Shape {
+  static constexpr int kStageBytes = kXBytes + kBN * 128;        // 48 KB at 256 columns
+  static constexpr int kStages = kBN == 256 ? 4 : kBN == 128 ? 6 : kBN == 64 ? 8 : 10;
+  static constexpr int kBarrierOffset = kStages * kStageBytes;
+  static constexpr int kSmemTotal = kBarrierOffset + 1024 /* barriers */ + 1024 /* alignment slack */;
+  static constexpr uint32_t kTmemCols = 2 * kBN;                 // two accumulator buffers
+};
 
 struct PersistArgs {
   int x_rows, y_rows, kblocks;
@@ -55,12 +58,16 @@ struct PersistArgs {
   int64_t sx, sy;
   int out_dtype;
   uint32_t idesc;
+  int x_static;            // no kernel writes X: its first tiles are requested before the previous kernel has finished
   uint32_t* status;
 };
 
-template <bool kFp8>
+template <int kBN, bool kFp8>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_persist_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_y, const PersistArgs a) {
+  using S = Shape<kBN>;
+  constexpr int kStages = S::kStages, kStageBytes = S::kStageBytes, kBarrierOffset = S::kBarrierOffset;
+  constexpr uint32_t kTmemCols = S::kTmemCols;
   constexpr int kElemsPerBlock = kFp8 ? 128 : 64;   // K elements in one 128-byte span
 
   extern __shared__ uint8_t smem_raw[];
@@ -98,8 +105,10 @@ gemm_persist_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
   __syncthreads();
   tc::fence_after_thread_sync();
   const uint32_t tmem_base = *tmem_slot;
-  ptx::pdl_wait();                // prefill shapes: both operands may come from earlier kernels of the stream
-  ptx::pdl_launch_dependents();
+  if (warp != 0 || !a.x_static) {
+    ptx::pdl_wait();              // operands may come from earlier kernels of the stream; static X: see the producer
+    ptx::pdl_launch_dependents();
+  }
 
   auto fail = [&]() {
     *abort_flag = 1;
@@ -109,9 +118,22 @@ gemm_persist_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
   if (warp == 0) {
     // ---- producer (one elected lane issues): the x tile index runs fastest, so CTAs that work side by side share the Y (weight) tile in L2 ----
     uint32_t it = 0;                                   // K blocks issued so far by this CTA
-    for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
+    uint32_t ahead = 0;                                // X tiles of the first ring pass requested ahead of the stream
+    if (a.x_static) {
+      ahead = min(kStages, nkb);
+      if (tc::elect_one()) {
+        for (uint32_t i = 0; i < ahead; ++i) {
+          tc::mbar_arrive_expect_tx(&full[i], kStageBytes);
+          tc::tma_load_2d(smem + i * kStageBytes, &map_x, &full[i], i * kElemsPerBlock, (int)(blockIdx.x % a.tiles_x) * kBM);
+        }
+      }
+      __syncwarp();
+      ptx::pdl_wait();
+      ptx::pdl_launch_dependents();
+    }
+    bool ok = true;
+    for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
       const int x_row0 = (t % a.tiles_x) * kBM, y_row0 = (t / a.tiles_x) * kBN;
-      bool ok = true;
       for (int kb = 0; kb < nkb; ++kb, ++it) {
         const uint32_t s = it % kStages;
         if (it >= (uint32_t)kStages && !tc::mbar_wait_warp(&empty[s], ((it / kStages) - 1) & 1, kWaitLimit, abort_flag)) {
@@ -120,17 +142,16 @@ gemm_persist_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
         }
         uint8_t* dst = smem + s * kStageBytes;
         if (tc::elect_one()) {
-          tc::mbar_arrive_expect_tx(&full[s], kStageBytes);
-          tc::tma_load_2d(dst, &map_x, &full[s], kb * kElemsPerBlock, x_row0);
+          if (it >= ahead) {
+            tc::mbar_arrive_expect_tx(&full[s], kStageBytes);
+            tc::tma_load_2d(dst, &map_x, &full[s], kb * kElemsPerBlock, x_row0);
+          }
           tc::tma_load_2d(dst + kXBytes, &map_y, &full[s], kb * kElemsPerBlock, y_row0);
         }
         __syncwarp();
       }
-      if (!ok) {
-        fail();
-        break;
-      }
     }
+    if (!ok) fail();
   } else if (warp == 1) {
     // ---- MMA issue (one elected lane issues) ----
     uint32_t it = 0;
@@ -173,7 +194,7 @@ gemm_persist_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
       const uint32_t buf = n & 1;
       const int x = (t % a.tiles_x) * kBM + q * 32 + lane;
       const int y_base = (t / a.tiles_x) * kBN;
-      if (nkb <= 0 || !tc::mbar_wait(&acc_full[buf], (n >> 1) & 1, kWaitLimit, abort_flag)) {
+      if (nkb <= 0 || !tc::mbar_wait_warp(&acc_full[buf], (n >> 1) & 1, kWaitLimit, abort_flag)) {
         if (nkb > 0 && lane == 0 && q == 0) fail();
         break;
       }
@@ -201,13 +222,24 @@ gemm_persist_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
   }
 }
 
-template <bool kFp8>
+template <int kBN, bool kFp8>
 std::string launch(const CUtensorMap& mx, const CUtensorMap& my, const PersistArgs& a, int grid, cudaStream_t stream) {
-  auto kern = gemm_persist_kernel<kFp8>;
-  const std::string err = reserve_dynamic_smem(kern, kSmemTotal);
+  auto kern = gemm_persist_kernel<kBN, kFp8>;
+  const std::string err = reserve_dynamic_smem(kern, Shape<kBN>::kSmemTotal);
   if (!err.empty()) return err;
-  const cudaError_t e = launch_chained(kern, dim3(grid), dim3(kThreads), kSmemTotal, stream, mx, my, a);
+  const cudaError_t e = launch_chained(kern, dim3(grid), dim3(kThreads), Shape<kBN>::kSmemTotal, stream, mx, my, a);
   return e == cudaSuccess ? "" : std::string("GEMM launch failed: ") + cudaGetErrorString(e);
+}
+
+template <bool kFp8>
+std::string launch_bn(int bn, const CUtensorMap& mx, const CUtensorMap& my, const PersistArgs& a, int grid, cudaStream_t stream) {
+  switch (bn) {
+    case 16: return launch<16, kFp8>(mx, my, a, grid, stream);
+    case 32: return launch<32, kFp8>(mx, my, a, grid, stream);
+    case 64: return launch<64, kFp8>(mx, my, a, grid, stream);
+    case 128: return launch<128, kFp8>(mx, my, a, grid, stream);
+    default: return launch<256, kFp8>(mx, my, a, grid, stream);
+  }
 }
 
 }  // namespace
@@ -223,24 +255,30 @@ std::string gemm_tn_persistent(const GemmProblem& g, cudaStream_t stream) {
   a.y_rows = g.y_rows;
   a.kblocks = g.k / epb;
   a.tiles_x = (g.x_rows + kBM - 1) / kBM;
-  a.tiles_y = (g.y_rows + kBN - 1) / kBN;
+  const int bn = gemm_pick_block_n(g.y_rows, false);
+  a.tiles_y = (g.y_rows + bn - 1) / bn;
   a.out = g.out;
   a.sx = g.sx;
   a.sy = g.sy;
   a.out_dtype = g.out_dtype;
-  a.idesc = fp8 ? tc::make_idesc(kBM, kBN, 0, 0) : tc::make_idesc(kBM, kBN, g.elem_kind == kBF16 ? 1 : 0, g.elem_kind == kBF16 ? 1 : 0);
+  a.idesc = fp8 ? tc::make_idesc(kBM, bn, 0, 0) : tc::make_idesc(kBM, bn, g.elem_kind == kBF16 ? 1 : 0, g.elem_kind == kBF16 ? 1 : 0);
   a.status = g.status;
+  a.x_static = g.x_static;
   CUtensorMap mx, my;
   std::string err = tma::kmajor_2d(&mx, g.x, g.x_rows, g.k, g.ldx, g.elem_size, g.elem_kind, kBM);
   if (!err.empty()) return err;
-  err = tma::kmajor_2d(&my, g.y, g.y_rows, g.k, g.ldy, g.elem_size, g.elem_kind, kBN);
+  err = tma::kmajor_2d(&my, g.y, g.y_rows, g.k, g.ldy, g.elem_size, g.elem_kind, bn);
   if (!err.empty()) return err;
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const long long ntiles = (long long)a.tiles_x * a.tiles_y;
-  const int grid = (int)(ntiles < sms ? ntiles : sms);
-  return fp8 ? launch<true>(mx, my, a, grid, stream) : launch<false>(mx, my, a, grid, stream);
+  // As many CTAs as give every one the same number of tiles: a last round of a few CTAs streams its weights at what a few
+  // multiprocessors can pull (about 58 GB/s each), while 112 of them already take all of HBM (224 tiles of 128 x 4096
+  // weights, 64 tokens: 148 CTAs 48.2 us, 112 CTAs 45.8).
+  const long long rounds = (ntiles + sms - 1) / sms;
+  const int grid = (int)((ntiles + rounds - 1) / rounds);
+  return fp8 ? launch_bn<true>(bn, mx, my, a, grid, stream) : launch_bn<false>(bn, mx, my, a, grid, stream);
 }
 
 }  // namespace tdx

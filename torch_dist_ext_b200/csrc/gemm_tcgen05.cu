@@ -312,7 +312,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
         tc::mbar_arrive(&acc_empty[buf]);
       }
     } else {
-      ok = nkb <= 0 || tc::mbar_wait(&acc_full[0], 0, kWaitLimit, abort_flag);
+      ok = nkb <= 0 || tc::mbar_wait_warp(&acc_full[0], 0, kWaitLimit, abort_flag);
       tc::fence_after_thread_sync();
     }
     if (!ok) {

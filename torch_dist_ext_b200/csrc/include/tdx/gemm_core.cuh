@@ -37,31 +37,41 @@ __device__ __forceinline__ uint32_t pack2(int out_dtype, float lo, float hi) {
   return *reinterpret_cast<const uint32_t*>(&h);
 }
 
-// Writes 16 consecutive y columns of row x (values already final): two 16-byte stores when the 16 columns are
-// contiguous 16-bit values at an aligned address, else element by element with bounds checks.
+// Writes 16 consecutive y columns of row x (values already final). Warp-wide: lane l holds row x = (row of lane 0) + l.
+//  * columns contiguous in memory (sy == 1), 16-bit, aligned: two 16-byte stores per lane;
+//  * rows contiguous in memory (sx == 1, the decode orientation), 16-bit, even sizes: neighbouring lanes exchange every
+//    other column, so that each stores two rows of a column with one 4-byte store (half the stores: the epilogue of a
+//    128 x 128 tile is bound by issuing them);
+//  * else element by element with bounds checks.
 template <typename Args>
 __device__ __forceinline__ void store_chunk(const Args& a, int x, int y0, const float (&v)[16]) {
-  if (x >= a.x_rows) return;
-  if (a.sy == 1 && a.out_dtype != kF32 && y0 + 16 <= a.y_rows && ((a.sx * 2) % 16 == 0) && (y0 % 8 == 0) &&
+  const bool narrow = a.out_dtype != kF32;
+  if (a.sy == 1 && narrow && y0 + 16 <= a.y_rows && ((a.sx * 2) % 16 == 0) && (y0 % 8 == 0) &&
       (reinterpret_cast<uintptr_t>(a.out) % 16 == 0)) {
+    if (x >= a.x_rows) return;
     uint32_t w[8];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      if (a.out_dtype == kBF16) {
-        __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
-        w[i] = *reinterpret_cast<uint32_t*>(&h);
-      } else {
-        __half2 h = __floats2half2_rn(v[2 * i], v[2 * i + 1]);
-        w[i] = *reinterpret_cast<uint32_t*>(&h);
-      }
-    }
+    for (int i = 0; i < 8; ++i) w[i] = pack2(a.out_dtype, v[2 * i], v[2 * i + 1]);
     uint4* dst = reinterpret_cast<uint4*>(static_cast<char*>(a.out) + ((int64_t)x * a.sx + y0) * 2);
     dst[0] = make_uint4(w[0], w[1], w[2], w[3]);
     dst[1] = make_uint4(w[4], w[5], w[6], w[7]);
-  } else {
+  } else if (a.sx == 1 && narrow && (a.sy & 1) == 0 && (a.x_rows & 1) == 0 && (reinterpret_cast<uintptr_t>(a.out) & 3u) == 0) {
+    const bool odd = x & 1;
+    char* dst = static_cast<char*>(a.out) + ((int64_t)(x & ~1) + (int64_t)(y0 + (odd ? 1 : 0)) * a.sy) * 2;
 #pragma unroll
-    for (int i = 0; i < 16; ++i)
-      if (y0 + i < a.y_rows) store_out(a, (int64_t)x * a.sx + (int64_t)(y0 + i) * a.sy, v[i]);
+    for (int i = 0; i < 16; i += 2) {
+      // the even lane takes column i, the odd lane column i + 1, each of both rows
+      const float other = __shfl_xor_sync(0xffffffffu, odd ? v[i] : v[i + 1], 1);
+      const uint32_t w = odd ? pack2(a.out_dtype, other, v[i + 1]) : pack2(a.out_dtype, v[i], other);
+      if (x < a.x_rows && y0 + i + (odd ? 1 : 0) < a.y_rows) *reinterpret_cast<uint32_t*>(dst) = w;
+      dst += a.sy * 4;
+    }
+  } else {
+    if (x >= a.x_rows) return;
+    int64_t at = (int64_t)x * a.sx + (int64_t)y0 * a.sy;
+#pragma unroll
+    for (int i = 0; i < 16; ++i, at += a.sy)
+      if (y0 + i < a.y_rows) store_out(a, at, v[i]);
   }
 }
 

@@ -315,8 +315,10 @@ void gemm_tn_pair(const Tensor& x, const Tensor& y, Tensor out, int64_t sx, int6
 }
 
 // The same product by a persistent grid with the accumulator double-buffered in tensor memory.
-void gemm_tn_persistent(const Tensor& x, const Tensor& y, Tensor out, int64_t sx, int64_t sy, const c10::optional<Tensor>& status) {
+void gemm_tn_persistent(const Tensor& x, const Tensor& y, Tensor out, int64_t sx, int64_t sy, const c10::optional<Tensor>& status,
+                        bool x_static) {
   tdx::GemmProblem g = gemm_problem(x, y, out, sx, sy, status);
+  g.x_static = x_static;
   const c10::cuda::CUDAGuard guard(x.device());
   const std::string err = tdx::gemm_tn_persistent(g, cur_stream());
   TORCH_CHECK(err.empty(), "gemm_tn_persistent: ", err);
@@ -552,7 +554,8 @@ void register_extra_ops(torch::Library& m) {
         "Tensor(d!)? status) -> ()", &gemm_tn_silu_mul);
   m.def("gemm_tn_pair(Tensor x, Tensor y, Tensor(a!) out, int sx, int sy, Tensor(b!)? status, Tensor(c!)? ws=None, "
         "Tensor(d!)? counters=None) -> ()", &gemm_tn_pair);
-  m.def("gemm_tn_persistent(Tensor x, Tensor y, Tensor(a!) out, int sx, int sy, Tensor(b!)? status) -> ()", &gemm_tn_persistent);
+  m.def("gemm_tn_persistent(Tensor x, Tensor y, Tensor(a!) out, int sx, int sy, Tensor(b!)? status, bool x_static=False) -> ()",
+        &gemm_tn_persistent);
   m.def("fused_add_rmsnorm(Tensor x, Tensor? residual_in, Tensor gamma, Tensor(a!)? residual_out, Tensor(b!) norm_out, "
         "Tensor(c!)? scale_out, float eps, int out_mode) -> int", &fused_add_rmsnorm);
   m.def("quant_fp8(Tensor x, Tensor(a!) q, Tensor(b!) scales, bool block128) -> ()", &quant_fp8);
