@@ -214,6 +214,16 @@ void gemm_tn(const Tensor& x, const Tensor& y, Tensor out, int64_t sx, int64_t s
   TORCH_CHECK(err.empty(), "gemm_tn: ", err);
 }
 
+// Decode-sized linear layer, out[m, n] = a[m, k] * w[n, k]^T with the weights on the 128-row side, output allocated here.
+Tensor linear_decode(const Tensor& a, const Tensor& w, c10::optional<at::ScalarType> out_dtype, int64_t block_n, int64_t splits,
+                     const Tensor& ws, const Tensor& counters, const c10::optional<Tensor>& status) {
+  TORCH_CHECK(a.is_cuda() && a.dim() == 2 && w.dim() == 2, "linear: a [M, K], w [N, K] on a CUDA device");
+  const at::ScalarType dt = out_dtype.has_value() ? *out_dtype : a.element_size() == 1 ? at::kBFloat16 : a.scalar_type();
+  Tensor out = at::empty({a.size(0), w.size(0)}, a.options().dtype(dt));
+  gemm_tn(w, a, out, 1, w.size(0), block_n, splits, ws, counters, status, c10::nullopt, c10::nullopt, false, false, true);
+  return out;
+}
+
 static void gemm_scratch(tdx::GemmProblem& g, const Tensor& ws, const Tensor& counters, const char* who) {
   TORCH_CHECK(ws.is_cuda() && counters.is_cuda() && ws.scalar_type() == at::kFloat && counters.scalar_type() == at::kInt, who,
               ": the split-K scratch must be float32 / int32 CUDA tensors");
@@ -353,6 +363,15 @@ void gemm_scaled(const Tensor& a, const Tensor& w, Tensor out, const Tensor& a_s
   TORCH_CHECK(err.empty(), "gemm_scaled: ", err);
 }
 
+// The same with the output allocated here.
+Tensor gemm_scaled_call(const Tensor& a, const Tensor& w, at::ScalarType out_dtype, const Tensor& a_scale, const Tensor& w_scale,
+                        const c10::optional<Tensor>& status) {
+  TORCH_CHECK(a.is_cuda() && a.dim() == 2 && w.dim() == 2, "gemm_scaled: a [M, K], w [N, K] on a CUDA device");
+  Tensor out = at::empty({a.size(0), w.size(0)}, a.options().dtype(out_dtype));
+  gemm_scaled(a, w, out, a_scale, w_scale, status);
+  return out;
+}
+
 // (ctas, workers, full_rounds, parts, per, slice_floats, counters) of a block-scaled problem on a device of `sms`
 // multiprocessors that holds so many clusters of 2, 4 and 8 CTAs
 std::vector<int64_t> gemm_scaled_plan(int64_t m, int64_t n, int64_t kblocks, int64_t sms, int64_t c2, int64_t c4, int64_t c8) {
@@ -398,6 +417,15 @@ void attention_decode_tc(const Tensor& q, const Tensor& k_cache, const Tensor& v
   attention_decode_impl(q, k_cache, v_cache, seq_lens, out, partial, nsplit, scale, status, true);
 }
 
+// The same with the output allocated here.
+Tensor attention_decode_call(const Tensor& q, const Tensor& k_cache, const Tensor& v_cache, const Tensor& seq_lens, Tensor partial,
+                             int64_t nsplit, double scale, const c10::optional<Tensor>& status, bool tensor_cores) {
+  TORCH_CHECK(q.is_cuda() && q.dim() == 3, "attention_decode: q [B, Hq, D]");
+  Tensor out = at::empty(q.sizes(), q.options());
+  attention_decode_impl(q, k_cache, v_cache, seq_lens, out, partial, nsplit, scale, status, tensor_cores);
+  return out;
+}
+
 // Causal attention over one prompt, both products on the tensor cores (tcgen05).
 void attention_prefill_tc(const Tensor& q, const Tensor& k, const Tensor& v, Tensor out, double scale,
                           const c10::optional<Tensor>& status) {
@@ -415,6 +443,13 @@ void attention_prefill_tc(const Tensor& q, const Tensor& k, const Tensor& v, Ten
       q.stride(0), k.stride(0), v.stride(0), (float)scale, cur_stream(),
       status.has_value() && status->defined() ? reinterpret_cast<uint32_t*>(status->data_ptr<int>()) : nullptr);
   TORCH_CHECK(err.empty(), "attention_prefill_tc: ", err);
+}
+
+Tensor attention_prefill_call(const Tensor& q, const Tensor& k, const Tensor& v, double scale, const c10::optional<Tensor>& status) {
+  TORCH_CHECK(q.is_cuda() && q.dim() == 3, "attention_prefill_tc: q [S, Hq, D]");
+  Tensor out = at::empty(q.sizes(), q.options());
+  attention_prefill_tc(q, k, v, out, scale, status);
+  return out;
 }
 
 static tdx::Workspace* workspace_of(const Tensor& table) {
@@ -537,6 +572,9 @@ void register_extra_ops(torch::Library& m) {
         "int nsplit, float scale, Tensor(c!)? status) -> ()", &attention_decode);
   m.def("attention_decode_tc(Tensor q, Tensor k_cache, Tensor v_cache, Tensor seq_lens, Tensor(a!) out, Tensor(b!) partial, "
         "int nsplit, float scale, Tensor(c!)? status) -> ()", &attention_decode_tc);
+  m.def("attention_decode_call(Tensor q, Tensor k_cache, Tensor v_cache, Tensor seq_lens, Tensor(a!) partial, int nsplit, float scale, "
+        "Tensor(b!)? status, bool tensor_cores) -> Tensor", &attention_decode_call);
+  m.def("attention_prefill_call(Tensor q, Tensor k, Tensor v, float scale, Tensor(a!)? status) -> Tensor", &attention_prefill_call);
   m.def("attention_decode_clusters(int nsplit) -> int", [](int64_t nsplit) -> int64_t { return tdx::attention_decode_clusters((int)nsplit); });
   m.def("attention_prefill_tc(Tensor q, Tensor k, Tensor v, Tensor(a!) out, float scale, Tensor(b!)? status) -> ()",
         &attention_prefill_tc);
@@ -546,6 +584,10 @@ void register_extra_ops(torch::Library& m) {
         "bool y_scale_per_row, bool x_static=False) -> ()", &gemm_tn);
   m.def("gemm_scaled(Tensor a, Tensor w, Tensor(a!) out, Tensor a_scale, Tensor w_scale, Tensor(b!)? status) -> ()",
         &gemm_scaled);
+  m.def("gemm_scaled_call(Tensor a, Tensor w, ScalarType out_dtype, Tensor a_scale, Tensor w_scale, Tensor(a!)? status) -> Tensor",
+        &gemm_scaled_call);
+  m.def("linear_decode(Tensor a, Tensor w, ScalarType? out_dtype, int block_n, int splits, Tensor(a!) ws, Tensor(b!) counters, "
+        "Tensor(c!)? status) -> Tensor", &linear_decode);
   m.def("gemm_scaled_plan(int m, int n, int kblocks, int sms, int c2, int c4, int c8) -> int[]", &gemm_scaled_plan);
   m.def("gemm_tn_rope_kv(Tensor w, Tensor a, Tensor(a!) out, int block_n, int splits, Tensor(b!) ws, Tensor(c!) counters, "
         "Tensor(d!)? status, Tensor? w_scale, Tensor? a_scale, Tensor positions, Tensor cos_sin, Tensor(e!) k_cache, "

@@ -225,6 +225,30 @@ int64_t allreduce_rms_fusion_ex(const Tensor& in, const c10::optional<Tensor>& r
                       scatter_only, /*allow_pinned=*/false);
 }
 
+// The same, with the outputs allocated here (one call from Python instead of four): (norm_out, residual_out, scales, algorithm).
+std::tuple<Tensor, c10::optional<Tensor>, c10::optional<Tensor>, int64_t> allreduce_rms_call(
+    const Tensor& in, const c10::optional<Tensor>& residual_in, const Tensor& gamma, double eps, const Tensor& workspace,
+    int64_t out_mode, int64_t algo, bool scatter_only, bool want_residual, int64_t nranks) {
+  TORCH_CHECK(in.is_cuda() && in.dim() >= 1, "allreduce_in must be a CUDA tensor with at least one dimension");
+  TORCH_CHECK(nranks >= 1 && nranks <= tdx::kMaxRanks, "nranks out of range");
+  const int64_t hidden = in.size(-1), tokens = in.numel() / std::max<int64_t>(1, hidden);
+  const int64_t rows = scatter_only ? (tokens + nranks - 1) / nranks : tokens;
+  std::vector<int64_t> sizes = in.sizes().vec();
+  if (scatter_only) sizes = {rows, hidden};
+  Tensor norm, res, scales;
+  if (want_residual) res = at::empty(sizes, in.options());
+  if (out_mode == tdx::kOutSame) {
+    norm = at::empty(sizes, in.options());
+  } else {
+    norm = at::empty(sizes, in.options().dtype(at::kFloat8_e4m3fn));
+    scales = at::empty({rows, out_mode == tdx::kOutFp8Token ? 1 : hidden / 128}, in.options().dtype(at::kFloat));
+  }
+  auto opt = [](const Tensor& t) { return t.defined() ? c10::optional<Tensor>(t) : c10::optional<Tensor>(); };
+  const int64_t used = launch_fused(in, residual_in, gamma, opt(res), norm, opt(scales), eps, workspace, out_mode, algo,
+                                    scatter_only, /*allow_pinned=*/false);
+  return {norm, opt(res), opt(scales), used};
+}
+
 // Same op for callers whose data starts and ends in page-locked host memory: any of the data tensors (not
 // gamma) may be a pinned CPU tensor. The reference has no counterpart; its op takes device tensors only
 // (src/ops/all_reduce_fusion.cpp:14-61).
@@ -367,6 +391,10 @@ TORCH_LIBRARY(torch_dist_ext, m) {
       "Tensor(b!) norm_out, Tensor(c!)? scale_out, float eps, Tensor workspace, int out_mode, int algo, "
       "bool scatter_only) -> int",
       &tdx_torch::allreduce_rms_fusion_hostio);
+  m.def(
+      "allreduce_rms_call(Tensor allreduce_in, Tensor? residual_in, Tensor rms_gamma, float eps, Tensor workspace, int out_mode, "
+      "int algo, bool scatter_only, bool want_residual, int nranks) -> (Tensor, Tensor?, Tensor?, int)",
+      &tdx_torch::allreduce_rms_call);
   m.def("set_policy(int nranks, int oneshot_max_bytes, int lamport_max_bytes, int mc_oneshot=-1, int mc_twoshot=-1, int nvls_min_bytes=-1) -> ()", &tdx_torch::set_policy);
   m.def("get_policy(int nranks) -> int[]", &tdx_torch::get_policy);
   m.def(

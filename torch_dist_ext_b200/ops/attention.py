@@ -3,6 +3,7 @@ contiguous bf16 KV cache; tcgen05 kernel, or the SIMT kernel with ``TDX_ATTN_TC=
 prompt (tcgen05 kernel)."""
 from __future__ import annotations
 
+import functools
 import math
 import os
 from typing import Optional
@@ -11,6 +12,7 @@ import torch
 
 from .. import _lib
 from ..utils.tracing import traced
+from . import gemm as _gemm
 
 _scratch = {}
 _TC_DEFAULT = os.environ.get("TDX_ATTN_TC", "1") not in ("0", "", "false", "off")
@@ -75,6 +77,14 @@ def pick_splits(batch: int, kv_heads: int, max_len: int, sms: int = 148, ctas_pe
     return min(range(1, most + 1), key=lambda n: (_split_cost_us(pairs, chunks, n, pairs <= fits.get(n, 0)), n))
 
 
+@functools.lru_cache(maxsize=4096)
+def _planned_splits(batch: int, kv_heads: int, max_len: int, tensor_cores: bool, device: torch.device) -> int:
+    """``pick_splits`` for the kernel and device of a call, remembered by its sizes (the search over split counts takes
+    2 to 20 us of Python, the whole call about 8)."""
+    return pick_splits(batch, kv_heads, max_len, ctas_per_sm=1 if tensor_cores else 2,
+                       clusters=_resident_clusters(device) if tensor_cores else None)
+
+
 @traced("tdx.decode_attention")
 def decode_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, seq_lens: torch.Tensor,
                      max_len: int, out: Optional[torch.Tensor] = None, nsplit: Optional[int] = None,
@@ -84,14 +94,14 @@ def decode_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tens
     ``max_len`` (a host integer >= every sequence length) only sizes the KV split. ``tensor_cores=True``
     runs both products of every 128-position chunk as tcgen05 MMAs (default: ``TDX_ATTN_TC``, on)."""
     b, hq, d = q.shape
-    hkv = k_cache.shape[2]
+    device = q.device
     use_tc = _TC_DEFAULT if tensor_cores is None else tensor_cores
     if nsplit is None:
-        nsplit = pick_splits(b, hkv, max_len, ctas_per_sm=1 if use_tc else 2, clusters=_resident_clusters(q.device) if use_tc else None)
-    out = torch.empty(b, hq, d, dtype=q.dtype, device=q.device) if out is None else out
-    part = _partial(q.device, 4096 + b * hq * nsplit * (d + 2))
-    from . import gemm as _gemm
-
+        nsplit = _planned_splits(b, k_cache.shape[2], max_len, use_tc, device)
+    part = _partial(device, 4096 + b * hq * nsplit * (d + 2))
+    if out is None:
+        return _lib.ops().attention_decode_call.default(q, k_cache, v_cache, seq_lens, part, nsplit, 1.0 / math.sqrt(d),
+                                                        _gemm._workspace(device)[2], use_tc)
     op = _lib.ops().attention_decode_tc if use_tc else _lib.ops().attention_decode
     op(q, k_cache, v_cache, seq_lens, out, part, nsplit, 1.0 / math.sqrt(d), _gemm._workspace(q.device)[2])
     return out
@@ -101,11 +111,10 @@ def decode_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tens
 def prefill_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Causal self-attention over one prompt on the tensor cores: ``q [S, Hq, 128]``, ``k``/``v`` ``[S, Hkv, 128]``
     (views into a fused qkv projection are fine) -> ``[S, Hq, 128]``; query i attends to keys 0..i."""
-    s, hq, d = q.shape
-    out = torch.empty(s, hq, d, dtype=q.dtype, device=q.device) if out is None else out
-    from . import gemm as _gemm
-
-    _lib.ops().attention_prefill_tc(q, k, v, out, 1.0 / math.sqrt(d), _gemm._workspace(q.device)[2])
+    scale, status = 1.0 / math.sqrt(q.shape[2]), _gemm._workspace(q.device)[2]
+    if out is None:
+        return _lib.ops().attention_prefill_call.default(q, k, v, scale, status)
+    _lib.ops().attention_prefill_tc(q, k, v, out, scale, status)
     return out
 
 

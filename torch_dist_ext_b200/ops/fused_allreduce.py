@@ -26,6 +26,10 @@ def _algo_code(algo) -> int:
     return ALGO_CODES[algo]
 
 
+def _call():
+    return _lib.ops().allreduce_rms_call.default
+
+
 def _cpu_path(allreduce_in, residual_in, rms_gamma, eps, out_mode, scatter_only):
     c = _comm.get_comm()
     if c.world_size > 1:
@@ -65,21 +69,9 @@ def fused_allreduce_rms(allreduce_in: torch.Tensor, residual_in: Optional[torch.
     c = _comm.get_comm()
     if workspace is None:
         workspace = c.get_workspace(allreduce_in)
-    hidden = allreduce_in.shape[-1]
-    tokens = allreduce_in.numel() // hidden
-    n = c.world_size
-    rows = (tokens + n - 1) // n if scatter_only else tokens
-    lead = allreduce_in.shape[:-1] if not scatter_only else (rows,)
-    residual_out = allreduce_in.new_empty(*lead, hidden) if want_residual else None
-    if out_mode == OUT_SAME:
-        norm_out = allreduce_in.new_empty(*lead, hidden)
-        scales = None
-    else:
-        norm_out = torch.empty(*lead, hidden, dtype=torch.float8_e4m3fn, device=allreduce_in.device)
-        ncol = 1 if out_mode == OUT_FP8_TOKEN else hidden // 128
-        scales = torch.empty(rows, ncol, dtype=torch.float32, device=allreduce_in.device)
-    used = _lib.ops().allreduce_rms_fusion_ex(allreduce_in, residual_in, rms_gamma, residual_out, norm_out, scales,
-                                              eps, workspace, out_mode, _algo_code(algo), scatter_only)
+    norm_out, residual_out, scales, used = _call()(allreduce_in, residual_in, rms_gamma, eps, workspace, out_mode,
+                                                   config.algo_code if algo is None else _algo_code(algo), scatter_only,
+                                                   want_residual, c.world_size)
     c.algo_counts[used] = c.algo_counts.get(used, 0) + 1
     return norm_out, residual_out, scales
 

@@ -113,11 +113,14 @@ def linear(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None,
     if block_n == 0:
         block_n = p_bn if swap == p_swap else _pick_bn(m if swap else n, 256)
     splits = p_splits if splits is None else splits
+    ws, counters, status = _workspace(a.device)
+    walk = persistent is not False and swap and splits == 1 and m <= 128 and block_n == _pick_bn(m, 256) and (n + 127) // 128 > _SM_COUNT
+    if out is None and swap and not walk:
+        return _lib.ops().linear_decode.default(a, w, out_dtype, block_n, splits, ws, counters, status)
     if out is None:
         dt = out_dtype or (torch.bfloat16 if a.element_size() == 1 else a.dtype)
         out = torch.empty(m, n, dtype=dt, device=a.device)
-    ws, counters, status = _workspace(a.device)
-    if swap and splits == 1 and m <= 128 and block_n == _pick_bn(m, 256) and (n + 127) // 128 > _SM_COUNT:
+    if walk:
         # more weight tiles than multiprocessors: one CTA each walks them with the ring streaming on from tile to tile, where
         # a second, partly filled wave of CTAs fills its pipeline again (28672 x 4096 at 64 tokens: 43.7 against 50.8 us)
         _lib.ops().gemm_tn_persistent(w, a, out, 1, n, status, True)
@@ -137,8 +140,6 @@ def linear_fp8_blockscaled(a_q: torch.Tensor, a_scale: torch.Tensor, w_q: torch.
     """``(a_q * a_scale) @ (w_q * w_scale)^T`` with ``a_scale [M, K/128]`` and ``w_scale [N/128, K/128]``."""
     m, k = a_q.shape
     n = w_q.shape[0]
-    if out is None:
-        out = torch.empty(m, n, dtype=out_dtype, device=a_q.device)
     ws, counters, status = _workspace(a_q.device)
     # The kernel of gemm_scaled.cu (activations on the 128-row side, 256 weight rows per tile), except for a few tokens of
     # a weight with so few rows that its tiles, in up to eight pieces each, leave most multiprocessors idle: there the
@@ -146,6 +147,10 @@ def linear_fp8_blockscaled(a_q: torch.Tensor, a_scale: torch.Tensor, w_q: torch.
     # 32 tokens 9.2 / 10.5; 7168 x 8192 at 16 tokens 19.4 / 17.8, 1280 x 8192 at 64 tokens 13.1 / 11.6, 8192 x 1024 at 1 token
     # 6.5 / 6.4, 28672 x 8192 at 64 tokens 81 / 47.
     few = m <= 32 and n <= 20 * 256 and k > 2048
+    if splits is None and not few and out is None:
+        return _lib.ops().gemm_scaled_call.default(a_q, w_q, out_dtype, a_scale.contiguous(), w_scale.contiguous(), status)
+    if out is None:
+        out = torch.empty(m, n, dtype=out_dtype, device=a_q.device)
     if splits is None and not few and out.is_contiguous():
         _lib.ops().gemm_scaled(a_q, w_q, out, a_scale.contiguous(), w_scale.contiguous(), status)
         return out
