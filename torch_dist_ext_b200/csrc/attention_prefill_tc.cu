@@ -58,14 +58,15 @@ constexpr int kQHalfBytes = kRows * 128;          // 64 head-dimension columns o
 constexpr int kQBytes = 2 * kQHalfBytes;
 constexpr int kKVHalfBytes = kKeys * 128;         // 64 head-dimension columns of the 64 positions of a chunk
 constexpr int kKVBytes = 2 * kKVHalfBytes;        // one K chunk or one V chunk
-constexpr int kPBytes = kRows * kKeys * 2;        // probabilities of a chunk: one 64-key K block of 128 rows
+constexpr int kMlBytes = 2 * kSoftmaxThreads * 8;      // maximum and sum of every row, from either group
 constexpr int kNumBarriers = 2 * kStagesK + 2 * kStagesV + 4 + 2 + 2 * kPTiles;   // k/v full+free, s full+free [2], q_full, o_final, p_full [4], pv_done [4]
 constexpr int kBarrierBytes = 256;                // the mbarriers, the TMEM address and the abort flag
 static_assert(kNumBarriers * 8 + 8 <= kBarrierBytes, "barrier area too small");
-constexpr int kSmem = kQBytes + kPTiles * kPBytes + (kStagesK + kStagesV) * kKVBytes + kBarrierBytes;
+constexpr int kSmem = kQBytes + kMlBytes + (kStagesK + kStagesV) * kKVBytes + kBarrierBytes;
 static_assert(kSmem <= 227 * 1024, "shared memory of one CTA");
-constexpr uint32_t kTmemCols = 512;               // S buffers at columns 0 and 64, O_0 at 128, O_1 at 256
+constexpr uint32_t kTmemCols = 512;               // S buffers at columns 0 and 64, O_0 at 128, O_1 at 256, P tiles from 384
 constexpr uint32_t kColO = 128;
+constexpr uint32_t kColP = 384;                   // four tiles of 32 columns: 64 bf16 probabilities of a row, two per column
 constexpr uint32_t kWaitLimit = 1u << 22;
 constexpr float kRescaleThreshold = 8.f;          // log2 units
 
@@ -115,10 +116,10 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     return;
   }
   uint8_t* q_tile = smem_raw;
-  uint8_t* p_tile = q_tile + kQBytes;
-  uint8_t* k_ring = p_tile + kPTiles * kPBytes;
+  uint8_t* k_ring = q_tile + kQBytes;
   uint8_t* v_ring = k_ring + kStagesK * kKVBytes;
-  uint64_t* k_full = reinterpret_cast<uint64_t*>(v_ring + kStagesV * kKVBytes);
+  float2* ml = reinterpret_cast<float2*>(v_ring + kStagesV * kKVBytes);
+  uint64_t* k_full = reinterpret_cast<uint64_t*>(reinterpret_cast<uint8_t*>(ml) + kMlBytes);
   uint64_t* k_free = k_full + kStagesK;
   uint64_t* v_full = k_free + kStagesK;
   uint64_t* v_free = v_full + kStagesV;
@@ -270,11 +271,11 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       TDX_PROBE(0, c, 3);
       tc::fence_after_thread_sync();
       const uint32_t vbase = tc::smem_u32(v_ring + (c % kStagesV) * kKVBytes);
-      const uint32_t pbase = tc::smem_u32(p_tile + (c & 3) * kPBytes);
+      const uint32_t pbase = tmem_base + kColP + (uint32_t)(c & 3) * (kKeys / 2);
       if (tc::elect_one()) {
 #pragma unroll
         for (int j = 0; j < kKeys / 16; ++j)   // 16 key positions per instruction
-          tc::umma<false>(tmem_base + kColO + (uint32_t)(c & 1) * kD, tc::make_smem_desc_sw128(pbase) + (uint64_t)(j * 2),
+          tc::umma_a_tmem(tmem_base + kColO + (uint32_t)(c & 1) * kD, pbase + (uint32_t)(j * 8),
                           tc::make_smem_desc_mn_sw128(vbase + j * 2048, kKVHalfBytes), a.idesc_pv, (c >= 2 || j > 0) ? 1u : 0u);
         tc::umma_commit(&pv_done[c & 3]);
         tc::umma_commit(&v_free[c % kStagesV]);
@@ -366,29 +367,24 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         fail();
       }
       tc::named_barrier_sync(2 + g, 2 * kSoftmaxThreads);      // this group's turn at the exponentials
-      // probabilities against m_run, row sum, this row of the P tile (bf16, K-major over the 64 key positions,
-      // 128-byte swizzle). A masked score is -FLT_MAX and comes out as zero.
+      // probabilities against m_run, row sum, this row of the P tile (bf16, two keys per 32-bit column of tensor memory).
+      // A masked score is -FLT_MAX and comes out as zero.
       float ps[4] = {0.f, 0.f, 0.f, 0.f};
-      uint8_t* row = p_tile + (i & 3) * kPBytes + t * 128;
       const float neg_m = -m_run;
+      uint32_t w[kKeys / 2];
 #pragma unroll
-      for (int cc = 0; cc < kKeys / 8; ++cc) {
-        uint32_t w[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float p0 = ex2(fmaf(__uint_as_float(sv[cc * 8 + 2 * j]), a.scale_log2, neg_m));
-          const float p1 = ex2(fmaf(__uint_as_float(sv[cc * 8 + 2 * j + 1]), a.scale_log2, neg_m));
-          ps[j] += p0 + p1;
-          __nv_bfloat162 hh = __floats2bfloat162_rn(p0, p1);
-          w[j] = *reinterpret_cast<uint32_t*>(&hh);
-        }
-        *reinterpret_cast<uint4*>(row + ((cc ^ (t & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+      for (int j = 0; j < kKeys / 2; ++j) {
+        const float p0 = ex2(fmaf(__uint_as_float(sv[2 * j]), a.scale_log2, neg_m));
+        const float p1 = ex2(fmaf(__uint_as_float(sv[2 * j + 1]), a.scale_log2, neg_m));
+        ps[j & 3] += p0 + p1;
+        __nv_bfloat162 hh = __floats2bfloat162_rn(p0, p1);
+        w[j] = *reinterpret_cast<uint32_t*>(&hh);
       }
+      tc::tmem_st_x32(lane_addr + kColP + (uint32_t)(i & 3) * (kKeys / 2), w);
       l_run += (ps[0] + ps[1]) + (ps[2] + ps[3]);
       if (g == 0 || i + 2 < nchunks) tc::named_barrier_arrive(2 + (g ^ 1), 2 * kSoftmaxThreads);   // the other group's turn
       TDX_PROBE(1 + g, i, 4);
-      tc::fence_proxy_async();          // P was written by threads and is read by the tensor core
-      tc::fence_before_thread_sync();   // orders the rescaled O (tcgen05.st) before the MMA that the arrival releases
+      tc::fence_before_thread_sync();   // orders P and the rescaled O (tcgen05.st) before the MMA that the arrival releases
       tc::mbar_arrive(&p_full[i & 3]);
       TDX_PROBE(1 + g, i, 5);
     }
@@ -398,8 +394,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       fail();
     }
     tc::fence_after_thread_sync();
-    // the two groups tell each other maximum and sum of their rows (through the first probability tile)
-    float2* ml = reinterpret_cast<float2*>(p_tile);
+    // the two groups tell each other maximum and sum of their rows
     ml[g * kSoftmaxThreads + t] = make_float2(m_run, l_run);
     tc::named_barrier_sync(1, 2 * kSoftmaxThreads);
     const float2 other = ml[(g ^ 1) * kSoftmaxThreads + t];
