@@ -105,6 +105,24 @@ __device__ __forceinline__ float ex2(float x) {
   return y;
 }
 
+// Two neighbouring fp32 values in one register pair, multiplied and added by one instruction (each rounded like its scalar form).
+__device__ __forceinline__ uint64_t pair2(float x, float y) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ void unpair2(uint64_t p, float& x, float& y) { asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(p)); }
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+
 __global__ void __launch_bounds__(kThreads, 1)
 attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                        const __grid_constant__ CUtensorMap map_v, const PrefillArgs a) {
@@ -369,19 +387,22 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       tc::named_barrier_sync(2 + g, 2 * kSoftmaxThreads);      // this group's turn at the exponentials
       // probabilities against m_run, row sum, this row of the P tile (bf16, two keys per 32-bit column of tensor memory).
       // A masked score is -FLT_MAX and comes out as zero.
-      float ps[4] = {0.f, 0.f, 0.f, 0.f};
-      const float neg_m = -m_run;
+      uint64_t ps[4] = {0ull, 0ull, 0ull, 0ull};
+      const uint64_t scale2 = pair2(a.scale_log2, a.scale_log2), neg_m2 = pair2(-m_run, -m_run);
       uint32_t w[kKeys / 2];
 #pragma unroll
       for (int j = 0; j < kKeys / 2; ++j) {
-        const float p0 = ex2(fmaf(__uint_as_float(sv[2 * j]), a.scale_log2, neg_m));
-        const float p1 = ex2(fmaf(__uint_as_float(sv[2 * j + 1]), a.scale_log2, neg_m));
-        ps[j & 3] += p0 + p1;
+        float x0, x1;
+        unpair2(fma2(pair2(__uint_as_float(sv[2 * j]), __uint_as_float(sv[2 * j + 1])), scale2, neg_m2), x0, x1);
+        const float p0 = ex2(x0), p1 = ex2(x1);
+        ps[j & 3] = add2(ps[j & 3], pair2(p0, p1));
         __nv_bfloat162 hh = __floats2bfloat162_rn(p0, p1);
         w[j] = *reinterpret_cast<uint32_t*>(&hh);
       }
       tc::tmem_st_x32(lane_addr + kColP + (uint32_t)(i & 3) * (kKeys / 2), w);
-      l_run += (ps[0] + ps[1]) + (ps[2] + ps[3]);
+      float sum_even, sum_odd;
+      unpair2(add2(add2(ps[0], ps[1]), add2(ps[2], ps[3])), sum_even, sum_odd);
+      l_run += sum_even + sum_odd;
       if (g == 0 || i + 2 < nchunks) tc::named_barrier_arrive(2 + (g ^ 1), 2 * kSoftmaxThreads);   // the other group's turn
       TDX_PROBE(1 + g, i, 4);
       tc::fence_before_thread_sync();   // orders P and the rescaled O (tcgen05.st) before the MMA that the arrival releases
