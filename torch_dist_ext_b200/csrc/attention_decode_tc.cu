@@ -13,7 +13,7 @@
 // do the online-softmax bookkeeping and write the probabilities as a bf16 [heads, keys] tile (128-byte
 // swizzle, the B operand of the second product). O^T accumulates in tensor memory over all chunks of a
 // split; a head's column of it is rescaled there only when its running maximum has to be raised.
-// Three more warps hold one single-thread role each - the TMA copies (3-stage ring), the score MMAs, the P*V MMAs -
+// Three more warps hold one single-thread role each - the TMA copies (rings of K and of V chunks), the score MMAs, the P*V MMAs -
 // so that none of them queues behind the others' asynchronous instructions; S^T is double-buffered in TMEM and P
 // in shared memory, so that the scores of chunk i+1 and the P*V product of chunk i-1 run while the softmax
 // warps work on chunk i.
@@ -49,14 +49,25 @@ namespace {
 constexpr int kD = 128;
 constexpr int kKeys = 128;                        // cache positions per chunk = MMA M of the score product
 constexpr int kNq = 16;                           // MMA N: query heads of one KV head, padded
-constexpr int kStages = 3;
 constexpr int kSoftmaxThreads = 128;
 constexpr int kThreads = kSoftmaxThreads + 3 * 32;   // + three single-thread roles: copies (warp 4), score MMAs (5), P*V MMAs (6)
 constexpr int kMaxG = 8;
 constexpr int kHalfBytes = kKeys * 128;           // one 64-column half of a K or V chunk
-constexpr int kStageBytes = 4 * kHalfBytes;       // K lo, K hi, V lo, V hi
+constexpr int kTileBytes = 2 * kHalfBytes;        // a K chunk or a V chunk
 constexpr int kSmallTileBytes = 2 * kNq * 128;    // Q or P: two 64-wide K blocks of 16 rows x 128 bytes
-constexpr int kSmem = kStages * kStageBytes + 3 * kSmallTileBytes /*Q, two P tiles*/ + 256 /*barriers*/ + 1024 /*alignment*/;
+// Rings of K and V chunks. One CTA per SM with three of each where the grid has no more CTAs than SMs: the few chunks of a
+// short split are all requested at once. More CTAs than SMs run two to an SM, with two K chunks and one V chunk each (the
+// same bytes in flight): one CTA's start (barriers, tensor memory, the first chunk's latency) and end overlap the other's
+// stream. 64 ragged sequences of up to 2048 positions, 32/8 heads: 73.2 us one to an SM, 70.4 two.
+struct Deep {
+  static constexpr int kStagesK = 3, kStagesV = 3, kCtasPerSm = 1;
+};
+struct Shared {
+  static constexpr int kStagesK = 2, kStagesV = 1, kCtasPerSm = 2;
+};
+template <typename R>
+constexpr int kSmemOf = (R::kStagesK + R::kStagesV) * kTileBytes + 3 * kSmallTileBytes /*Q, two P tiles*/ + 256 /*barriers*/ + 1024 /*alignment*/;
+static_assert(kSmemOf<Deep> <= 227 * 1024 && 2 * (kSmemOf<Shared> + 1024) <= 228 * 1024, "shared memory of an SM");
 constexpr uint32_t kTmemCols = 64;                // S^T buffers at columns 0 and 16, O^T chunk at 32
 constexpr uint32_t kColO = 32;
 constexpr uint32_t kWaitLimit = 1u << 22;
@@ -87,19 +98,23 @@ __device__ __forceinline__ int small_tile_offset(int row, int col) {
   return kb * (kNq * 128) + row * 128 + ((c ^ (row & 7)) << 4) + (col & 7) * 2;
 }
 
-template <int kG>
-__global__ void __launch_bounds__(kThreads, 1)
+template <int kG, typename R>
+__global__ void __launch_bounds__(kThreads, R::kCtasPerSm)
 attn_decode_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const TcAttnArgs a) {
+  constexpr int kStagesK = R::kStagesK, kStagesV = R::kStagesV;
   extern __shared__ uint8_t smem_raw[];
   __shared__ float wred[2][kG][4];
   __shared__ uint32_t s_last, s_stop;
   uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* q_tile = ring + kStages * kStageBytes;
+  uint8_t* v_ring = ring + kStagesK * kTileBytes;
+  uint8_t* q_tile = v_ring + kStagesV * kTileBytes;
   uint8_t* p_tile = q_tile + kSmallTileBytes;
   // two P tiles, alternating by chunk: the probabilities of chunk i are written while P*V of chunk i - 1 may still run
-  uint64_t* kv_full = reinterpret_cast<uint64_t*>(p_tile + 2 * kSmallTileBytes);
-  uint64_t* kv_free = kv_full + kStages;
-  uint64_t* s_full = kv_free + kStages;     // [2]
+  uint64_t* k_full = reinterpret_cast<uint64_t*>(p_tile + 2 * kSmallTileBytes);
+  uint64_t* k_free = k_full + kStagesK;
+  uint64_t* v_full = k_free + kStagesK;
+  uint64_t* v_free = v_full + kStagesV;
+  uint64_t* s_full = v_free + kStagesV;     // [2]
   uint64_t* s_free = s_full + 2;            // [2]
   uint64_t* p_full = s_free + 2;            // [2]: the probabilities of chunk c are in P tile c & 1
   uint64_t* o_full = p_full + 2;            // [2]: P*V of chunk c completes o_full[c & 1]
@@ -111,9 +126,13 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
 
   // what touches no memory of an earlier kernel comes before the wait for it
   if (tid == 0) {
-    for (int s = 0; s < kStages; ++s) {
-      tc::mbar_init(&kv_full[s], 1);
-      tc::mbar_init(&kv_free[s], 1);
+    for (int s = 0; s < kStagesK; ++s) {
+      tc::mbar_init(&k_full[s], 1);
+      tc::mbar_init(&k_free[s], 1);
+    }
+    for (int s = 0; s < kStagesV; ++s) {
+      tc::mbar_init(&v_full[s], 1);
+      tc::mbar_init(&v_free[s], 1);
     }
     for (int i = 0; i < 2; ++i) {
       tc::mbar_init(&s_full[i], 1);
@@ -170,25 +189,30 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
 
   // Three issuing warps, each with its own chain of waits; the whole warp walks the loop and one elected lane issues.
   if (warp == 4) {
-    // ---- copies: a stage is refilled when the P*V product that read its V tile has completed ----
-    auto issue_copy = [&](int c) {
-      const int st = c % kStages;
-      uint8_t* base = ring + st * kStageBytes;
+    // ---- copies: a K stage is refilled when its scores are complete, a V stage after P*V ----
+    auto load = [&](const CUtensorMap* map, uint8_t* base, uint64_t* bar, int c) {
       const int pos0 = s0 + c * kKeys;
       if (tc::elect_one()) {
-        tc::mbar_arrive_expect_tx(&kv_full[st], kStageBytes);
-        tc::tma_load_4d(base, &map_k, &kv_full[st], 0, hkv, pos0, b);
-        tc::tma_load_4d(base + kHalfBytes, &map_k, &kv_full[st], 64, hkv, pos0, b);
-        tc::tma_load_4d(base + 2 * kHalfBytes, &map_v, &kv_full[st], 0, hkv, pos0, b);
-        tc::tma_load_4d(base + 3 * kHalfBytes, &map_v, &kv_full[st], 64, hkv, pos0, b);
+        tc::mbar_arrive_expect_tx(bar, kTileBytes);
+        tc::tma_load_4d(base, map, bar, 0, hkv, pos0, b);
+        tc::tma_load_4d(base + kHalfBytes, map, bar, 64, hkv, pos0, b);
       }
       __syncwarp();
     };
+    constexpr int kLag = kStagesK - kStagesV;      // K runs so many chunks ahead of V
     bool ok = true;
-    for (int c = 0; c < nchunks && c < kStages; ++c) issue_copy(c);
-    for (int i = 0; i + kStages < nchunks && ok; ++i) {
-      ok = tc::mbar_wait_warp(&kv_free[i % kStages], (i / kStages) & 1, kWaitLimit, abort_flag);
-      if (ok) issue_copy(i + kStages);
+    for (int j = 0; j < nchunks + kLag && ok; ++j) {
+      if (j < nchunks) {
+        const int st = j % kStagesK;
+        ok = j < kStagesK || tc::mbar_wait_warp(&k_free[st], (j / kStagesK - 1) & 1, kWaitLimit, abort_flag);
+        if (ok) load(&map_k, ring + st * kTileBytes, &k_full[st], j);
+      }
+      const int c = j - kLag;
+      if (ok && c >= 0) {
+        const int st = c % kStagesV;
+        ok = c < kStagesV || tc::mbar_wait_warp(&v_free[st], (c / kStagesV - 1) & 1, kWaitLimit, abort_flag);
+        if (ok) load(&map_v, v_ring + st * kTileBytes, &v_full[st], c);
+      }
     }
     if (!ok) fail();
   } else if (warp == 5) {
@@ -196,11 +220,11 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
     const uint32_t qbase = tc::smem_u32(q_tile);
     bool ok = true;
     for (int c = 0; c < nchunks && ok; ++c) {
-      ok = tc::mbar_wait_warp(&kv_full[c % kStages], (c / kStages) & 1, kWaitLimit, abort_flag) &&
+      ok = tc::mbar_wait_warp(&k_full[c % kStagesK], (c / kStagesK) & 1, kWaitLimit, abort_flag) &&
            (c < 2 || tc::mbar_wait_warp(&s_free[c & 1], ((c >> 1) - 1) & 1, kWaitLimit, abort_flag));
       if (!ok) break;
       tc::fence_after_thread_sync();
-      const uint32_t kbase = tc::smem_u32(ring + (c % kStages) * kStageBytes);
+      const uint32_t kbase = tc::smem_u32(ring + (c % kStagesK) * kTileBytes);
       if (tc::elect_one()) {
 #pragma unroll
         for (int kb = 0; kb < 2; ++kb)
@@ -209,6 +233,7 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
             tc::umma<false>(tmem_base + (uint32_t)(c & 1) * kNq, tc::make_smem_desc_sw128(kbase + kb * kHalfBytes) + (uint64_t)(ks * 2),
                             tc::make_smem_desc_sw128(qbase + kb * (kNq * 128)) + (uint64_t)(ks * 2), a.idesc_s, (kb | ks) ? 1u : 0u);
         tc::umma_commit(&s_full[c & 1]);
+        tc::umma_commit(&k_free[c % kStagesK]);
       }
       __syncwarp();
     }
@@ -218,10 +243,10 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
     bool ok = true;
     for (int c = 0; c < nchunks && ok; ++c) {
       ok = tc::mbar_wait_warp(&p_full[c & 1], (c >> 1) & 1, kWaitLimit, abort_flag) &&
-           tc::mbar_wait_warp(&kv_full[c % kStages], (c / kStages) & 1, kWaitLimit, abort_flag);
+           tc::mbar_wait_warp(&v_full[c % kStagesV], (c / kStagesV) & 1, kWaitLimit, abort_flag);
       if (!ok) break;
       tc::fence_after_thread_sync();
-      const uint32_t vbase = tc::smem_u32(ring + (c % kStages) * kStageBytes + 2 * kHalfBytes);
+      const uint32_t vbase = tc::smem_u32(v_ring + (c % kStagesV) * kTileBytes);
       const uint32_t pbase = tc::smem_u32(p_tile + (c & 1) * kSmallTileBytes);
       if (tc::elect_one()) {
 #pragma unroll
@@ -230,7 +255,7 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
                           tc::make_smem_desc_sw128(pbase + (j >> 2) * (kNq * 128)) + (uint64_t)((j & 3) * 2), a.idesc_pv,
                           (c | j) ? 1u : 0u);
         tc::umma_commit(&o_full[c & 1]);
-        tc::umma_commit(&kv_free[c % kStages]);
+        tc::umma_commit(&v_free[c % kStagesV]);
       }
       __syncwarp();
     }
@@ -469,12 +494,12 @@ __global__ void __launch_bounds__(kD) attn_tc_combine_kernel(const TcAttnArgs a)
   a.out[((int64_t)b * a.Hq + h) * kD + d] = __float2bfloat16(den > 0.f ? num / den : 0.f);
 }
 
-template <int kG>
+template <typename R>
 cudaLaunchConfig_t config(const TcAttnArgs& a, dim3 grid, cudaStream_t stream, cudaLaunchAttribute (&attr)[2]) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
   cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = kSmem;
+  cfg.dynamicSmemBytes = kSmemOf<R>;
   cfg.stream = stream;
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 1;
@@ -487,15 +512,28 @@ cudaLaunchConfig_t config(const TcAttnArgs& a, dim3 grid, cudaStream_t stream, c
   return cfg;
 }
 
-template <int kG>
-std::string launch(const CUtensorMap& mk, const CUtensorMap& mv, const TcAttnArgs& a, dim3 grid, cudaStream_t stream) {
-  auto kern = attn_decode_tc_kernel<kG>;
-  const std::string smem_err = reserve_dynamic_smem(kern, kSmem);
+template <int kG, typename R>
+std::string launch_as(const CUtensorMap& mk, const CUtensorMap& mv, const TcAttnArgs& a, dim3 grid, cudaStream_t stream) {
+  auto kern = attn_decode_tc_kernel<kG, R>;
+  const std::string smem_err = reserve_dynamic_smem(kern, kSmemOf<R>);
   if (!smem_err.empty()) return smem_err;
   cudaLaunchAttribute attr[2];
-  const cudaLaunchConfig_t cfg = config<kG>(a, grid, stream, attr);
+  const cudaLaunchConfig_t cfg = config<R>(a, grid, stream, attr);
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, mk, mv, a);
   return e == cudaSuccess ? "" : std::string("attention launch failed: ") + cudaGetErrorString(e);
+}
+
+int sm_count() {
+  int dev = 0, n = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+  return n;
+}
+
+template <int kG>
+std::string launch(const CUtensorMap& mk, const CUtensorMap& mv, const TcAttnArgs& a, dim3 grid, cudaStream_t stream) {
+  const long long ctas = (long long)grid.x * grid.y * grid.z;
+  return ctas > sm_count() ? launch_as<kG, Shared>(mk, mv, a, grid, stream) : launch_as<kG, Deep>(mk, mv, a, grid, stream);
 }
 
 }  // namespace
@@ -513,13 +551,13 @@ int attention_decode_clusters(int nsplit) {
   std::lock_guard<std::mutex> lock(mu);
   const auto it = known.find({dev, nsplit});
   if (it != known.end()) return it->second;
-  auto kern = attn_decode_tc_kernel<kMaxG>;
-  if (reserve_dynamic_smem(kern, kSmem).empty()) {
+  auto kern = attn_decode_tc_kernel<kMaxG, Deep>;
+  if (reserve_dynamic_smem(kern, kSmemOf<Deep>).empty()) {
     TcAttnArgs a{};
     a.cluster = 1;
     a.nsplit = nsplit;
     cudaLaunchAttribute attr[2];
-    cudaLaunchConfig_t cfg = config<kMaxG>(a, dim3(1, 1, nsplit), nullptr, attr);
+    cudaLaunchConfig_t cfg = config<Deep>(a, dim3(1, 1, nsplit), nullptr, attr);
     cfg.numAttrs = 1;
     if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
       cudaGetLastError();
