@@ -911,8 +911,13 @@ __device__ __forceinline__ void ar_dispatch_body(const ArParams& p) {
 template <int kVpt>
 constexpr int kMaxThreadsFor = (kVpt == 1) ? 1024 : 512;
 
+// The single-rank kernel of two vectors per thread is held to 64 registers, so that an SM has two blocks: with 79 it had one,
+// and the block's loads of one row (28 KB at 7168 x bf16) were all that was in flight (8192 x 7168 to e4m3: 82 us with one, 70 with two, 6.0 TB/s).
+template <int kAlgo, int kVpt>
+constexpr int kMinBlocksFor = (kAlgo == kAlgoLocal && kVpt == 2) ? 2 : 1;
+
 template <typename T, int kAlgo, int kN, int kVpt, int kOut>
-__global__ void __launch_bounds__(kMaxThreadsFor<kVpt>, 1) ar_fused_kernel(const __grid_constant__ ArParams p) {
+__global__ void __launch_bounds__(kMaxThreadsFor<kVpt>, kMinBlocksFor<kAlgo, kVpt>) ar_fused_kernel(const __grid_constant__ ArParams p) {
   // Launched with programmatic stream serialisation (ar_fusion_inst.cu), the blocks of this kernel are scheduled
   // while the previous kernel of the stream still runs, and wait here until it has completed and its memory
   // is visible; the next kernel may then be scheduled in the same way. A plain launch passes straight through.
