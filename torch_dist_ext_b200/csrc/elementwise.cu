@@ -12,6 +12,7 @@
 #include "tdx/ops.h"
 #include "tdx/ptx.cuh"
 #include "tdx/sync.cuh"
+#include "tdx/tc.cuh"
 #include "tdx/vec.cuh"
 
 namespace tdx {
@@ -227,72 +228,92 @@ int grid_for(size_t work_items, int threads, int max_blocks = 148 * 8) {
     default: return "unsupported dtype";                                  \
   }
 
-// Greedy sampling over a vocabulary that is sharded across ranks. One block per token: the largest logit of this
-// rank's slice and its index in the whole vocabulary go into slot `rank` of the token's row of `pack`
-// [tokens, 4 * nranks] fp32 as {value, index, 0, 0}; the other ranks' slots of the row are set to zero, so that the
+// Greedy sampling over a vocabulary that is sharded across ranks. A cluster of CTAs per token (one CTA for a small
+// vocabulary): every CTA scans a slice of this rank's logits, the first one collects the cluster's candidates out of the
+// others' shared memory. The largest logit and its index in the whole vocabulary go into slot `rank` of the token's row of
+// `pack` [tokens, 4 * nranks] fp32 as {value, index, 0, 0}; the other ranks' slots of the row are set to zero, so that the
 // SUM of `pack` over the ranks (one call of the fused all-reduce) is the gather of every rank's candidate. Indices
-// stay exact in fp32 up to 2^24. Of equal logits the lowest index wins; a NaN never wins.
-__global__ void __launch_bounds__(1024) argmax_pack_kernel(const float* __restrict__ logits, int64_t ld, int vocab,
-                                                           int index_base, int rank, int nranks, float* __restrict__ pack) {
+// stay exact in fp32 up to 2^24. With one rank the index goes straight to `tokens_out` (pack unused). Of equal logits the
+// lowest index wins; a NaN never wins. Bound by latency: one CTA per token had 16 CTAs read 1 MB (16 x 16032: 5.9 us).
+__global__ void __launch_bounds__(256) argmax_kernel(const float* __restrict__ logits, int64_t ld, int vocab, int index_base,
+                                                     int rank, int nranks, int cluster, float* __restrict__ pack,
+                                                     int64_t* __restrict__ tokens_out) {
+  __shared__ float s_val[8];
+  __shared__ int s_idx[8];
+  __shared__ float2 s_best;                 // this CTA's candidate: value, index (as bits)
   ptx::pdl_wait();
   ptx::pdl_launch_dependents();
-  __shared__ float s_val[32];
-  __shared__ int s_idx[32];
-  const int t = blockIdx.x;
+  const int t = blockIdx.x / cluster, part = blockIdx.x % cluster;
   const float* row = logits + (int64_t)t * ld;
   float best = -INFINITY;
   int at = 0x7fffffff;
   auto take = [&](float v, int i) {
     if (v > best) { best = v; at = i; }      // a thread walks its indices upwards, so the first of equal values stays
   };
+  auto merge = [&](float v, int i) {
+    if (v > best || (v == best && i < at)) { best = v; at = i; }
+  };
   // 16-byte loads, four of them in flight per thread, when the row allows it; single elements otherwise and at the end
   const bool vec = ((reinterpret_cast<uintptr_t>(row) & 15u) == 0);
   const int nvec = vec ? vocab / 4 : 0;
   const float4* row4 = reinterpret_cast<const float4*>(row);
-  int i = threadIdx.x;
-  for (; i + 3 * (int)blockDim.x < nvec; i += 4 * blockDim.x) {
+  const int step = cluster * blockDim.x;
+  int i = part * blockDim.x + threadIdx.x;
+  for (; i + 3 * step < nvec; i += 4 * step) {
     float4 v[4];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) v[u] = __ldcs(row4 + i + u * blockDim.x);
+    for (int u = 0; u < 4; ++u) v[u] = __ldcs(row4 + i + u * step);
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      const int e = 4 * (i + u * (int)blockDim.x);
+      const int e = 4 * (i + u * step);
       take(v[u].x, e);
       take(v[u].y, e + 1);
       take(v[u].z, e + 2);
       take(v[u].w, e + 3);
     }
   }
-  for (; i < nvec; i += blockDim.x) {
+  for (; i < nvec; i += step) {
     const float4 v = __ldcs(row4 + i);
     take(v.x, 4 * i);
     take(v.y, 4 * i + 1);
     take(v.z, 4 * i + 2);
     take(v.w, 4 * i + 3);
   }
-  for (int e = 4 * nvec + threadIdx.x; e < vocab; e += blockDim.x) take(row[e], e);
+  for (int e = 4 * nvec + part * blockDim.x + threadIdx.x; e < vocab; e += step) take(row[e], e);
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) {
     const float ov = __shfl_xor_sync(0xffffffffu, best, off);
     const int oi = __shfl_xor_sync(0xffffffffu, at, off);
-    if (ov > best || (ov == best && oi < at)) { best = ov; at = oi; }
+    merge(ov, oi);
   }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (lane == 0) { s_val[warp] = best; s_idx[warp] = at; }
   __syncthreads();
-  if (threadIdx.x < 4 * nranks) {
-    float out = 0.f;
-    const int slot = threadIdx.x >> 2, word = threadIdx.x & 3;
-    if (slot == rank && word < 2) {
-      best = s_val[0];
-      at = s_idx[0];
-      for (int w = 1; w < (int)(blockDim.x >> 5); ++w)
-        if (s_val[w] > best || (s_val[w] == best && s_idx[w] < at)) { best = s_val[w]; at = s_idx[w]; }
-      if (at == 0x7fffffff) at = 0;   // a row of NaN or -inf: a valid index all the same
-      out = word == 0 ? best : float(index_base + at);
-    }
-    pack[(int64_t)t * 4 * nranks + threadIdx.x] = out;
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 8; ++w) merge(s_val[w], s_idx[w]);
+    s_best = make_float2(best, __int_as_float(at));
   }
+  if (cluster > 1) {
+    tc::cluster_arrive();
+    tc::cluster_wait();
+    if (part == 0 && threadIdx.x == 0) {
+      const uint32_t mine = tc::smem_u32(&s_best);
+      for (int c = 1; c < cluster; ++c) {
+        const uint32_t src = tc::map_to_cta(mine, c);
+        merge(tc::ld_cluster_f1(src), __float_as_int(tc::ld_cluster_f1(src + 4)));
+      }
+    }
+    tc::cluster_arrive();
+    tc::cluster_wait();       // no CTA leaves while its candidate may still be read
+  }
+  if (part != 0 || threadIdx.x != 0) return;
+  if (at == 0x7fffffff) at = 0;   // a row of NaN or -inf: a valid index all the same
+  if (tokens_out != nullptr) {
+    tokens_out[t] = (int64_t)index_base + at;
+    return;
+  }
+  float* out = pack + (int64_t)t * 4 * nranks;
+  for (int w = 0; w < 4 * nranks; ++w) out[w] = w == 4 * rank ? best : w == 4 * rank + 1 ? float(index_base + at) : 0.f;
 }
 
 // The winner among the ranks' candidates: gathered [tokens, 4 * nranks] fp32 -> token ids int64 [tokens].
@@ -313,12 +334,26 @@ __global__ void __launch_bounds__(128) select_token_kernel(const float* __restri
 }
 
 std::string argmax_pack(const float* logits, int64_t ld, int tokens, int vocab, int index_base, int rank, int nranks,
-                        float* pack, cudaStream_t stream) {
+                        float* pack, int64_t* tokens_out, cudaStream_t stream) {
   if (nranks < 1 || nranks > kMaxRanks || rank < 0 || rank >= nranks) return "rank / nranks out of range";
   if (vocab < 1 || (int64_t)index_base + vocab > (1 << 24)) return "vocabulary indices must stay below 2^24";
   if (tokens == 0) return "";
-  launch_chained(argmax_pack_kernel, dim3(tokens), dim3(vocab >= 8192 ? 1024 : 256), 0, stream, logits, ld, vocab, index_base, rank, nranks, pack);
-  cudaError_t e = cudaGetLastError();
+  // eight CTAs per token from 8192 logits (each then has at least one 16-byte load per thread); one below
+  const int cluster = vocab >= 8192 ? 8 : 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)tokens * cluster);
+  cfg.blockDim = dim3(256);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = cluster;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl_enabled() ? 2 : 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, argmax_kernel, logits, ld, vocab, index_base, rank, nranks, cluster, pack, tokens_out);
   return e == cudaSuccess ? "" : cudaGetErrorString(e);
 }
 

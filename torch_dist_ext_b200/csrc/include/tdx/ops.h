@@ -30,9 +30,10 @@ std::string rope_inplace(void* q, void* k, const int64_t* positions, const float
 // argmax_pack writes {largest logit, its index + index_base, 0, 0} of every row of logits [tokens, vocab] fp32 (rows
 // `ld` elements apart) into slot `rank` of pack [tokens, 4 * nranks] fp32 and zeroes the other slots, so that the
 // sum of `pack` over the ranks holds every rank's candidate; select_token picks the winner per row (the lowest
-// index among equal logits) into out [tokens] int64.
+// index among equal logits) into out [tokens] int64. With `tokens_out` [tokens] int64 (one rank) the index goes there and
+// `pack` is not used.
 std::string argmax_pack(const float* logits, int64_t ld, int tokens, int vocab, int index_base, int rank, int nranks,
-                        float* pack, cudaStream_t stream);
+                        float* pack, int64_t* tokens_out, cudaStream_t stream);
 std::string select_token(const float* gathered, int tokens, int nranks, int64_t* out, cudaStream_t stream);
 
 // Decode attention over a contiguous bf16 KV cache [B, S_max, Hkv, 128] for one new token per

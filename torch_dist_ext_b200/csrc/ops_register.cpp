@@ -93,8 +93,20 @@ void argmax_pack(const Tensor& logits, int64_t index_base, int64_t rank, int64_t
               pack.numel() == logits.size(0) * 4 * nranks, "pack must be a contiguous fp32 [tokens, 4 * nranks] tensor");
   const c10::cuda::CUDAGuard guard(logits.device());
   const std::string err = tdx::argmax_pack(logits.data_ptr<float>(), logits.stride(0), (int)logits.size(0), (int)logits.size(1),
-                                           (int)index_base, (int)rank, (int)nranks, pack.data_ptr<float>(), cur_stream());
+                                           (int)index_base, (int)rank, (int)nranks, pack.data_ptr<float>(), nullptr, cur_stream());
   TORCH_CHECK(err.empty(), "argmax_pack: ", err);
+}
+
+// One rank: the arg-max of every row as int64 [tokens].
+Tensor argmax_tokens(const Tensor& logits, int64_t index_base) {
+  TORCH_CHECK(logits.is_cuda() && logits.dim() == 2 && logits.scalar_type() == at::kFloat && logits.stride(1) == 1,
+              "logits must be a CUDA fp32 [tokens, vocab] tensor with unit stride along the vocabulary");
+  const c10::cuda::CUDAGuard guard(logits.device());
+  Tensor out = at::empty({logits.size(0)}, logits.options().dtype(at::kLong));
+  const std::string err = tdx::argmax_pack(logits.data_ptr<float>(), logits.stride(0), (int)logits.size(0), (int)logits.size(1),
+                                           (int)index_base, 0, 1, nullptr, out.data_ptr<int64_t>(), cur_stream());
+  TORCH_CHECK(err.empty(), "argmax_pack: ", err);
+  return out;
 }
 
 void select_token(const Tensor& gathered, int64_t nranks, Tensor out) {
@@ -604,6 +616,7 @@ void register_extra_ops(torch::Library& m) {
   m.def("silu_mul(Tensor gate_up, Tensor(a!) out, Tensor(b!)? scales) -> ()", &silu_mul);
   m.def("attention_prefill_probe() -> Tensor", &attention_prefill_probe);
   m.def("argmax_pack(Tensor logits, int index_base, int rank, int nranks, Tensor(a!) pack) -> ()", &argmax_pack);
+  m.def("argmax_tokens(Tensor logits, int index_base) -> Tensor", &argmax_tokens);
   m.def("select_token(Tensor gathered, int nranks, Tensor(a!) out) -> ()", &select_token);
   m.def("rope_(Tensor(a!) q, Tensor(b!) k, Tensor positions, Tensor cos_sin_cache) -> ()", &rope_);
   m.def("rope_append_kv_(Tensor(a!) q, Tensor(b!) k, Tensor v, Tensor positions, Tensor cos_sin_cache, Tensor(c!) k_cache, "

@@ -259,7 +259,7 @@ class TPLlama:
         """One token per sequence: ``tokens``/``positions`` int64 [B] on the device. Returns next tokens [B]."""
         b = tokens.shape[0]
         cfg = self.cfg
-        self.seq_lens[:b] = (positions + 1).to(torch.int32)
+        torch.add(positions, 1, out=self.seq_lens[:b])      # one kernel: sum and conversion to int32
         res = self.embed[tokens]                                                  # [B, hidden]
         mode0 = self._norm_out_mode()
         if self.mode == "sp":

@@ -27,12 +27,12 @@ def greedy_sample_sharded(logits: torch.Tensor, rank: int, world: int, index_bas
     if not logits.is_cuda:
         return _ref.greedy_sample_sharded(logits, rank, world, index_base)
     ops = _lib.ops()
+    if world == 1:
+        return ops.argmax_tokens.default(logits, index_base)
     pack = torch.empty(tokens, 4 * world, dtype=torch.float32, device=logits.device)
     ops.argmax_pack(logits, index_base, rank, world, pack)
-    if world > 1:
-        from .fused_allreduce import fused_allreduce_rms
-        ones = _ones(4 * world, logits.device)
-        _, pack, _ = fused_allreduce_rms(pack, None, ones, 1e-6)
+    from .fused_allreduce import fused_allreduce_rms
+    _, pack, _ = fused_allreduce_rms(pack, None, _ones(4 * world, logits.device), 1e-6)
     out = torch.empty(tokens, dtype=torch.int64, device=logits.device)
     ops.select_token(pack, world, out)
     return out
