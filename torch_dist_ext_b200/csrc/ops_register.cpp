@@ -351,7 +351,7 @@ void gemm_tn_persistent(const Tensor& x, const Tensor& y, Tensor out, int64_t sx
 void gemm_scaled(const Tensor& a, const Tensor& w, Tensor out, const Tensor& a_scale, const Tensor& w_scale,
                  const c10::optional<Tensor>& status) {
   tdx::GemmProblem g = gemm_problem(a, w, out, w.size(0), 1, status);
-  TORCH_CHECK(a.scalar_type() == at::kFloat8_e4m3fn, "gemm_scaled: float8_e4m3fn operands");
+  TORCH_CHECK(a.element_size() == 1, "gemm_scaled: one-byte (e4m3) operands");
   TORCH_CHECK(g.k > 0 && g.k % 128 == 0, "gemm_scaled: K must be a positive multiple of 128");
   TORCH_CHECK(a_scale.scalar_type() == at::kFloat && w_scale.scalar_type() == at::kFloat && a_scale.is_contiguous() && w_scale.is_contiguous(),
               "gemm_scaled: scales must be contiguous float32");
