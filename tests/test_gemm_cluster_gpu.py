@@ -32,3 +32,24 @@ def test_cluster_splits_match_64_bit(m, n, k, out_dtype):
     assert (outs[0].double() - want).abs().max() <= bound
     ws, counters, _ = gemm._workspace(a.device)
     assert float(ws.abs().max()) == 0.0 and int(counters.abs().sum()) == 0
+
+
+@pytest.mark.parametrize("m,n,k", [
+    (256, 256, 1024),     # one tile in pieces
+    (300, 1280, 4096),    # ragged rows: ten tiles of four pieces
+    (257, 4352, 2048),    # 34 tiles: too many for clusters of eight CTAs
+    (700, 3584, 1792),    # 42 tiles, whole
+    (260, 263, 4160),     # ragged both ways, uneven pieces, unaligned output rows
+])
+@pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32])
+def test_pieces_of_a_pair_tile_match_64_bit(m, n, k, out_dtype):
+    g = torch.Generator(device="cuda").manual_seed(m + n + k)
+    a = torch.randn(m, k, device="cuda", generator=g).to(torch.bfloat16)
+    w = (torch.randn(n, k, device="cuda", generator=g) * 0.05).to(torch.bfloat16)
+    want = a.double() @ w.double().t()
+    outs = [gemm.linear(a, w, out_dtype=out_dtype) for _ in range(2)]
+    torch.cuda.synchronize()
+    assert gemm.pipeline_status() == 0 and torch.equal(outs[0], outs[1])
+    # as above
+    bound = want.abs().max() * (2.0 ** -8 if out_dtype == torch.bfloat16 else k * 2.0 ** -22)
+    assert (outs[0].double() - want).abs().max() <= bound

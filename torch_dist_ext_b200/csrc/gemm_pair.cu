@@ -12,7 +12,8 @@
 // work side by side share the Y tile in L2). When the last round would be partly filled, its tiles are cut along K
 // into 2-4 pieces, one piece per pair; every piece stores its fp32 partial tile in a scratch slice of its own and the
 // CTA that arrives last at its half of the tile adds the slices up - the idle pairs of the last round then share its
-// work. The operand ring keeps streaming across tile boundaries and the
+// work. With fewer tiles than pairs (a short prompt, a narrow weight) two or four pairs share every tile: they are one
+// cluster, leave their sums in shared memory and each adds up and stores its part of the columns out of the others'. The operand ring keeps streaming across tile boundaries and the
 // accumulator is double-buffered in tensor memory (2 x 256 columns in each CTA): while the epilogue warps of both
 // CTAs read tile n back with tcgen05.ld and store it, the leader is already accumulating tile n + 1.
 //
@@ -36,8 +37,10 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
+#include <map>
 #include <mutex>
 #include <string>
+#include <utility>
 #include "tdx/comm.h"
 #include "tdx/gemm.h"
 #include "tdx/gemm_core.cuh"
@@ -60,6 +63,7 @@ constexpr int kOperandBytes = kRowsPerCta * 128; // 128 rows x one 128-byte swiz
 constexpr int kStageBytes = 2 * kOperandBytes;   // X half + Y half
 constexpr int kBarrierOffset = kStages * kStageBytes;
 constexpr int kSmemTotal = kBarrierOffset + 1024 /* barriers */ + 1024 /* alignment slack */;
+static_assert(kRowsPerCta * gemm_core::kSumPitch<kTileN> * 16 <= kBarrierOffset, "a piece's sums take the ring's place");
 constexpr uint32_t kTmemCols = 2 * kTileN;       // two fp32 accumulator buffers
 constexpr uint32_t kWaitLimit = 1u << 22;
 
@@ -72,6 +76,9 @@ struct PairArgs {
   int tail_first, tail_parts, tail_kb;
   float* ws;               // [tail tiles][parts][256 columns][256 rows] fp32; contents undefined before and after
   uint32_t* counters;      // [tail tiles][2 CTAs of the pair], zero on entry and on exit
+  // Fewer tiles than pairs: `pieces` pairs per tile, piece_kb K blocks each, the CTAs of one cluster; they meet in shared
+  // memory (1: whole tiles).
+  int pieces, piece_kb;
   void* out;
   int64_t sx, sy;
   int out_dtype;
@@ -88,6 +95,11 @@ struct WorkItem {
 };
 __device__ __forceinline__ bool work_item(const PairArgs& a, int pair, int npairs, int n, WorkItem* w) {
   const int ntiles = a.tiles_x * a.tiles_y;
+  if (a.pieces > 1) {
+    const int kb0 = pair % a.pieces * a.piece_kb;
+    *w = WorkItem{pair / a.pieces, kb0, min(a.kblocks, kb0 + a.piece_kb), false, 0};
+    return n == 0;
+  }
   const int full_rounds = a.tail_parts > 1 ? a.tail_first / npairs : 0x7fffffff;   // tail_first is a multiple of npairs
   if (n < full_rounds) {
     const int t = pair + n * npairs;
@@ -105,7 +117,7 @@ __device__ __forceinline__ bool work_item(const PairArgs& a, int pair, int npair
 }
 
 template <bool kFp8>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(kThreads, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_y, const PairArgs a) {
   constexpr int kElemsPerBlock = kFp8 ? 128 : 64;   // K elements in one 128-byte span
 
@@ -121,8 +133,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
   uint32_t* last_flag = tmem_slot + 2;       // tail split: "this CTA arrived last at its half of the tile"
 
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
-  const uint32_t rank = tc::cluster_ctarank();      // 0: leader, 1: peer
-  const uint32_t leader = rank & ~1u, other = rank ^ 1u;
+  const uint32_t rank = tc::cluster_ctarank();      // even: leader, odd: its peer
+  const uint32_t leader = rank & ~1u, other = rank ^ 1u, both = 3u << leader;
   const int pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
   const int nkb = a.kblocks;
 
@@ -218,8 +230,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             for (int k = 0; k < 4; ++k)   // 32 bytes of K per instruction, stepped inside the swizzle span
               tc::umma_pair<kFp8>(tmem_base + buf * kTileN, dx + (uint64_t)(k * 2), dy + (uint64_t)(k * 2), a.idesc,
                                   (kb > w.kb0 || k > 0) ? 1u : 0u);
-            tc::umma_commit_both(&empty[s]);   // the stage is free again in both CTAs
-            if (kb + 1 == w.kb1) tc::umma_commit_both(&acc_full[buf]);
+            tc::umma_commit_both(&empty[s], both);   // the stage is free again in both CTAs
+            if (kb + 1 == w.kb1) tc::umma_commit_both(&acc_full[buf], both);
           }
           __syncwarp();
         }
@@ -244,7 +256,18 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         break;
       }
       tc::fence_after_thread_sync();
-      if (!w.partial) {
+      if (a.pieces > 1) {
+        // a piece: every MMA of the pair has read its operands, the sums take the ring's place (one row per lane)
+        float4* sums = reinterpret_cast<float4*>(smem) + (q * 32 + lane) * gemm_core::kSumPitch<kTileN>;
+#pragma unroll 2
+        for (int c = 0; c < kTileN; c += 32) {
+          uint32_t v[32];
+          tc::tmem_ld_x32(lane_addr + buf * kTileN + c, v);
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            sums[c / 4 + j] = make_float4(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]), __uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3]));
+        }
+      } else if (!w.partial) {
 #pragma unroll 4
         for (int c = 0; c < kTileN; c += 16) {
           float v[16];
@@ -320,18 +343,87 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
   }
   tc::cluster_arrive();
   tc::cluster_wait();
+  if (a.pieces > 1) {
+    if (warp >= 2 && !*abort_flag) {
+      const int tile = pair / a.pieces, x0 = (tile % a.tiles_x) * kTileM + (int)(rank & 1u) * kRowsPerCta;
+      gemm_core::add_up_cluster<kTileN, 128>(a, tc::smem_u32(smem), threadIdx.x - 64, pair % a.pieces, a.pieces, rank & 1u, 2,
+                                             min(kRowsPerCta, a.x_rows - x0), x0, (tile / a.tiles_x) * kTileN);
+    }
+    __syncwarp();
+    tc::cluster_arrive();
+    tc::cluster_wait();        // no CTA leaves while another may still read its sums
+  }
   if (warp == 1) {
     tc::fence_after_thread_sync();
     tc::tmem_dealloc_pair(tmem_base, kTmemCols);
   }
 }
 
+cudaLaunchConfig_t config(dim3 grid, int cluster, cudaStream_t stream, cudaLaunchAttribute (&attr)[2]) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = kSmemTotal;
+  cfg.stream = stream;
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = cluster;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl_enabled() ? 2 : 1;
+  return cfg;
+}
+
+// How many clusters of `cluster` CTAs the current device holds at a time.
 template <bool kFp8>
-std::string launch(const CUtensorMap& mx, const CUtensorMap& my, const PairArgs& a, dim3 grid, cudaStream_t stream) {
+int resident_clusters(int cluster) {
+  static std::mutex mu;
+  static std::map<std::pair<int, int>, int> known;
+  int dev = 0, n = 0;
+  cudaGetDevice(&dev);
+  std::lock_guard<std::mutex> lock(mu);
+  const auto it = known.find({dev, cluster});
+  if (it != known.end()) return it->second;
+  auto kern = gemm_pair_kernel<kFp8>;
+  if (reserve_dynamic_smem(kern, kSmemTotal).empty()) {
+    cudaLaunchAttribute attr[2];
+    cudaLaunchConfig_t cfg = config(dim3(cluster), cluster, nullptr, attr);
+    cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      n = 0;
+    }
+  }
+  known[{dev, cluster}] = n;
+  return n;
+}
+
+template <bool kFp8>
+std::string launch(const CUtensorMap& mx, const CUtensorMap& my, PairArgs a, dim3 grid, cudaStream_t stream) {
   auto kern = gemm_pair_kernel<kFp8>;
   const std::string err = reserve_dynamic_smem(kern, kSmemTotal);
   if (!err.empty()) return err;
-  const cudaError_t e = launch_chained(kern, grid, dim3(kThreads), kSmemTotal, stream, mx, my, a);
+  // Fewer tiles than pairs: two or four pairs per tile where the device holds the clusters and K is long enough to pay for
+  // the meeting. Measured: a K block takes 0.375 us, the meeting of two pairs 8.5 us (each adds up half the columns), of
+  // four 6.5. B200, us, whole / in pieces: 300 x 768 x 4096 27.1 / 14.3, 512 x 4096 x 14336 81.5 / 53.3, 300 x 4096 x 4096
+  // 27.3 / 24.1; 300 x 4096 x 1792 would be 15.0 / 17.8 in two pieces and stays whole.
+  const int tiles = a.tiles_x * a.tiles_y;
+  double best = 0.375 * a.kblocks;
+  a.pieces = 1;
+  for (int pieces = 2; pieces <= 4 && a.tail_parts == 0; pieces *= 2) {
+    const int per = (a.kblocks + pieces - 1) / pieces;
+    const double us = 0.375 * per + (pieces == 2 ? 8.5 : 6.5);
+    if ((pieces - 1) * per >= a.kblocks || us >= best || tiles > resident_clusters<kFp8>(2 * pieces)) continue;
+    best = us;
+    a.pieces = pieces;
+    a.piece_kb = per;
+  }
+  if (a.pieces > 1) grid = dim3(2 * tiles * a.pieces);
+  cudaLaunchAttribute attr[2];
+  const cudaLaunchConfig_t cfg = config(grid, 2 * a.pieces, stream, attr);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, mx, my, a);
   return e == cudaSuccess ? "" : std::string("GEMM launch failed: ") + cudaGetErrorString(e);
 }
 

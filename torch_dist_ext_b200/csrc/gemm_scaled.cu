@@ -69,7 +69,7 @@ constexpr int kXBytes = kRows * 128;
 constexpr uint32_t kTmemCols = 2 * kCols;
 constexpr uint32_t kWaitLimit = 1u << 22;
 constexpr size_t kSliceFloats = (size_t)kRows * kCols;   // partial sums of one CTA
-constexpr int kSumPitch = kCols / 4 + 1;                 // decode: row pitch of the sums in shared memory, in 16-byte quads
+constexpr int kSumPitch = gemm_core::kSumPitch<kCols>;                 // decode: row pitch of the sums in shared memory, in 16-byte quads
 // Scale products: a ring of 16 K blocks, handed over in groups of four, [K block][half][row]; a block's pitch is padded by
 // eight floats so that the writing lanes (eight rows x four blocks) hit distinct banks.
 constexpr int kGroup = 4;
@@ -149,46 +149,6 @@ __device__ __forceinline__ void store_sector(void* dst, const uint32_t (&w)[8]) 
   asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]),
                "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
                : "memory");
-}
-
-// Decode sizes, after the cluster barrier: this CTA's part of the tile's columns, summed over the cluster's CTAs in
-// their order. Lanes run along the columns, so that a row's part is read and written in one piece.
-__device__ __forceinline__ void add_up(const ScaledArgs& a, uint8_t* smem, int worker) {
-  const int tile = worker / a.parts, quads = kCols / 4 / a.parts;
-  const int t = threadIdx.x - kFirstPromoteWarp * 32;
-  const int quad = worker % a.parts * quads + t % quads, row_step = kPromoteWarps * 32 / quads;
-  const int rows = min(kRows, a.x_rows - (tile % a.tiles_x) * kRows);
-  const int y = (tile / a.tiles_x) * kCols + quad * 4;
-  if (y >= a.y_rows) return;
-  const uint32_t base = tc::smem_u32(smem) + quad * 16;
-  const bool quad_store = a.sy == 1 && y + 4 <= a.y_rows && (a.sx * (a.out_dtype == kF32 ? 4 : 2)) % 16 == 0 && reinterpret_cast<uintptr_t>(a.out) % 16 == 0;
-  for (int row = t / quads; row < rows; row += row_step) {
-    float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
-    float4 in[8];
-#pragma unroll
-    for (int p = 0; p < 8; ++p)
-      if (p < a.parts) in[p] = tc::ld_cluster_f4(tc::map_to_cta(base + row * (kSumPitch * 16), p));
-#pragma unroll
-    for (int p = 0; p < 8; ++p) {
-      if (p >= a.parts) continue;
-      sum.x += in[p].x;
-      sum.y += in[p].y;
-      sum.z += in[p].z;
-      sum.w += in[p].w;
-    }
-    const int64_t at = (int64_t)((tile % a.tiles_x) * kRows + row) * a.sx + (int64_t)y * a.sy;
-    if (quad_store && a.out_dtype == kF32) {
-      *reinterpret_cast<float4*>(static_cast<float*>(a.out) + at) = sum;
-    } else if (quad_store) {
-      *reinterpret_cast<uint2*>(static_cast<char*>(a.out) + at * 2) =
-          make_uint2(gemm_core::pack2(a.out_dtype, sum.x, sum.y), gemm_core::pack2(a.out_dtype, sum.z, sum.w));
-    } else {
-      const float v[4] = {sum.x, sum.y, sum.z, sum.w};
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-        if (y + j < a.y_rows) gemm_core::store_out(a, at + j * a.sy, v[j]);
-    }
-  }
 }
 
 template <int kCtas>
@@ -338,8 +298,8 @@ gemm_scaled_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
             else tc::umma<true>(dst, dx + (uint64_t)(k * 2), dy + (uint64_t)(k * 2), a.idesc, k > 0 ? 1u : 0u);
           }
           if constexpr (kCtas == 2) {
-            tc::umma_commit_both(&part_full[half * 2 + buf]);
-            tc::umma_commit_both(&empty[s]);
+            tc::umma_commit_both(&part_full[half * 2 + buf], 3);
+            tc::umma_commit_both(&empty[s], 3);
           } else {
             tc::umma_commit(&part_full[half * 2 + buf]);
             tc::umma_commit(&empty[s]);
@@ -537,7 +497,11 @@ gemm_scaled_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
     tc::cluster_wait();        // pairs: no CTA leaves while its peer may still read its shared memory or write its barriers
   }
   if (kCtas == 1 && a.parts > 1) {
-    if (warp >= kFirstPromoteWarp && !*abort_flag) add_up(a, smem, worker);
+    if (warp >= kFirstPromoteWarp && !*abort_flag) {
+      const int tile = worker / a.parts, x0 = (tile % a.tiles_x) * kRows;
+      gemm_core::add_up_cluster<kCols, kPromoteWarps * 32>(a, tc::smem_u32(smem), threadIdx.x - kFirstPromoteWarp * 32, worker % a.parts, a.parts,
+                                                           0, 1, min(kRows, a.x_rows - x0), x0, (tile / a.tiles_x) * kCols);
+    }
     tc::cluster_arrive();
     tc::cluster_wait();        // no CTA leaves while another may still read its sums
   }

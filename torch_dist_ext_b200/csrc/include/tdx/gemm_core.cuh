@@ -75,6 +75,52 @@ __device__ __forceinline__ void store_chunk(const Args& a, int x, int y0, const 
   }
 }
 
+// ---- pieces of a tile that are the CTAs of one cluster -------------------------------------------------------
+// Row pitch, in 16-byte quads, of a tile's fp32 sums in shared memory: one more than the columns fill, so that lanes along
+// the rows write, and lanes along the columns read, without bank conflicts.
+template <int kCols>
+constexpr int kSumPitch = kCols / 4 + 1;
+
+// After the cluster barrier: `kThreads` threads (`t`) of piece `part` add up part `part` of the columns over the pieces, in
+// their order, and store it. Piece p's sums are at `base` in the CTA of cluster rank rank0 + p * rank_step. Lanes run along
+// the columns, so that a row's part is read and written in one piece.
+template <int kCols, int kThreads, typename Args>
+__device__ __forceinline__ void add_up_cluster(const Args& a, uint32_t base, int t, int part, int parts, int rank0, int rank_step, int rows,
+                                               int x0, int y_tile) {
+  const int quads = kCols / 4 / parts, row_step = kThreads / quads;
+  const int quad = part * quads + t % quads;
+  const int y = y_tile + quad * 4;
+  if (y >= a.y_rows) return;
+  const bool quad_store = a.sy == 1 && y + 4 <= a.y_rows && (a.sx * (a.out_dtype == kF32 ? 4 : 2)) % 16 == 0 &&
+                          reinterpret_cast<uintptr_t>(a.out) % 16 == 0;
+  for (int row = t / quads; row < rows; row += row_step) {
+    float4 in[8];
+#pragma unroll
+    for (int p = 0; p < 8; ++p)
+      if (p < parts) in[p] = tc::ld_cluster_f4(tc::map_to_cta(base + (row * kSumPitch<kCols> + quad) * 16, rank0 + p * rank_step));
+    float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int p = 0; p < 8; ++p) {
+      if (p >= parts) continue;
+      sum.x += in[p].x;
+      sum.y += in[p].y;
+      sum.z += in[p].z;
+      sum.w += in[p].w;
+    }
+    const int64_t at = (int64_t)(x0 + row) * a.sx + (int64_t)y * a.sy;
+    if (quad_store && a.out_dtype == kF32) {
+      *reinterpret_cast<float4*>(static_cast<float*>(a.out) + at) = sum;
+    } else if (quad_store) {
+      *reinterpret_cast<uint2*>(static_cast<char*>(a.out) + at * 2) = make_uint2(pack2(a.out_dtype, sum.x, sum.y), pack2(a.out_dtype, sum.z, sum.w));
+    } else {
+      const float v[4] = {sum.x, sum.y, sum.z, sum.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (y + j < a.y_rows) store_out(a, at + j * a.sy, v[j]);
+    }
+  }
+}
+
 // Block-scale promotion of one K block: acc[j] += partial[j] * xs * ys[j] for the kBN (<= 64) columns of this
 // thread's row. The partial products are fetched from tensor memory with ONE load (one round trip per K block);
 // the column scales sit two per lane (`ys_lo`: columns 0-31, `ys_hi`: 32-63) and are handed round by shuffles.

@@ -378,10 +378,11 @@ __device__ __forceinline__ void umma_pair(uint32_t tmem_d, uint64_t desc_a, uint
 }
 // Arrive on the mbarrier `bar` of BOTH CTAs of the pair (same offset in each CTA's shared memory) once all MMAs issued so
 // far by this thread have completed. Called by the leader's MMA thread.
-__device__ __forceinline__ void umma_commit_both(uint64_t* bar) {
+// `ctas`: the two CTAs' bits of the cluster (3 when the pair is the cluster).
+__device__ __forceinline__ void umma_commit_both(uint64_t* bar, uint32_t ctas) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
                    smem_u32(bar)),
-               "h"((uint16_t)3)
+               "h"((uint16_t)ctas)
                : "memory");
 }
 

@@ -48,14 +48,20 @@ _PREFILL_ATTN_TC = os.environ.get("TDX_PREFILL_ATTN", "tc").lower() != "sdpa"
 _FUSED_FP8 = os.environ.get("TDX_FUSED_FP8", "0") != "0"
 _FUSED_BF16 = os.environ.get("TDX_FUSED_BF16", "0") != "0"
 # Decode steps in "ar" mode run the rotary embedding + KV append inside the qkv GEMM and (bf16 weights) silu(gate) * up
-# inside the gate_up GEMM: both live in the GEMM's split-K finalizer and each saves a launch of the layer's latency
-# chain. Measured on one B200 at the per-rank shapes of TP=8 (CUDA-graph replay of 8 layers, same box, fused against
-# separate kernels): Llama-3-8B 51.3 / 55.2 against 54.3 / 59.7 us per layer at batch 1 / 16, Llama-3-70B (e4m3, rotary
-# part only) 84.7 / 88.3 against 85.8 / 90.1; at batch 64 the finalizer - one CTA per 128 output features, after the
-# last K split has arrived - is the longer path (100.0 against 94.5 and 137.1 against 130.9), so the fused form is used
-# up to TDX_FUSED_EPILOGUE_TOKENS (16) tokens. TDX_FUSED_EPILOGUES=0 keeps the separate kernels everywhere.
+# inside the gate_up GEMM: both are done by the CTAs of the cluster in which the GEMM's K splits meet, and each saves a launch
+# of the layer's latency chain. Measured on one B200 at the per-rank shapes of TP=8 (CUDA-graph replay of four Llama-3-8B
+# layers and the lm-head, 2048 positions, fused against separate kernels): 186 against 197 us per step at batch 1, 200 / 212
+# at 16, 217 / 228 at 17, 257 / 263 at 33, 280 / 284 at 64, so bf16 weights use them up to 64 tokens where the GEMM has at
+# most 74 tiles, as many as a B200 holds clusters of two; with more tiles one CTA finishes each alone, and 16 tokens is the
+# limit. The block-scaled e4m3 kernel that has the rotary epilogue is the faster one for a few tokens only, hence 16 there too.
+# TDX_FUSED_EPILOGUE_TOKENS sets one limit for all, TDX_FUSED_EPILOGUES=0 keeps the separate kernels everywhere.
 _FUSED_EPILOGUES = os.environ.get("TDX_FUSED_EPILOGUES", "1") != "0"
-_FUSED_EPILOGUE_TOKENS = int(os.environ.get("TDX_FUSED_EPILOGUE_TOKENS", "16"))
+_FUSED_EPILOGUE_TOKENS = os.environ.get("TDX_FUSED_EPILOGUE_TOKENS")
+
+
+def _epilogue_fits(tokens: int, tiles: int, fp8: bool) -> bool:
+    limit = int(_FUSED_EPILOGUE_TOKENS) if _FUSED_EPILOGUE_TOKENS else 64 if tiles <= 74 and not fp8 else 16
+    return _FUSED_EPILOGUES and tokens <= limit
 
 
 @dataclass
@@ -205,7 +211,7 @@ class TPLlama:
         down projection is a plain GEMM followed by the all-reduce whose epilogue writes bf16,
         because the final norm feeds the bf16 lm_head."""
         cfg, L, d = self.cfg, self.layers[i], self.cfg.head_dim
-        fuse = (_FUSED_EPILOGUES and self.mode == "ar" and d == 128 and tokens <= _FUSED_EPILOGUE_TOKENS
+        fuse = (self.mode == "ar" and d == 128 and _epilogue_fits(tokens, self.hq + 2 * self.hkv, cfg.fp8)
                 and gemm.fused_epilogue_fits(tokens, cfg.hidden, 1 if cfg.fp8 else 2, cfg.fp8))
         if fuse:
             if cfg.fp8 and x_scale is None:
@@ -221,7 +227,7 @@ class TPLlama:
             rope.rope_append_kv_(q, k, v, positions, self.cos_sin, self.k_cache[i], self.v_cache[i])
         attn = attention.decode_attention(q, self.k_cache[i][:tokens], self.v_cache[i][:tokens], self.seq_lens[:tokens], max_len)
         x, x_scale, res = self._row_parallel(attn.view(tokens, self.hq * d), L["wo"], res, L["ln2"])
-        if fuse and not cfg.fp8 and self.ffn_r % 64 == 0:
+        if fuse and not cfg.fp8 and self.ffn_r % 64 == 0 and _epilogue_fits(tokens, self.ffn_r // 64, False):
             act, act_scale = gemm.linear_silu_mul(x, L["wgu"].w), None
         else:
             gu = self._col_parallel(x, L["wgu"], tokens, x_scale)

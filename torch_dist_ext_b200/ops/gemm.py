@@ -83,7 +83,7 @@ def linear(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None,
            cta_pair: Optional[bool] = None, persistent: Optional[bool] = None) -> torch.Tensor:
     """``a [M, K] @ w [N, K]^T -> [M, N]`` (bf16 / fp16 / e4m3 operands, fp32 accumulation).
 
-    ``cta_pair=True`` runs prefill-sized problems (M, N >= 256) on 256 x 256 tiles computed by pairs of
+    ``cta_pair=True`` runs prefill-sized problems (M > 128, N >= 256) on 256 x 256 tiles computed by pairs of
     CTAs (``tcgen05.mma.cta_group::2``) that walk the tiles persistently with the accumulator double-buffered in
     tensor memory; the default follows ``TDX_GEMM_PAIR`` (on: it is the fastest kernel for these shapes). ``persistent=True`` runs
     them on a persistent grid (one CTA per SM, accumulator double-buffered in tensor memory so that the epilogue
@@ -94,7 +94,10 @@ def linear(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None,
     # an explicit choice of one kernel is not overridden by the default of the other
     use_pair = cta_pair if cta_pair is not None else (_PAIR_DEFAULT and persistent is None)
     use_persistent = persistent if persistent is not None else (_PERSIST_DEFAULT and not use_pair)
-    if use_pair and m >= 256 and n >= 256 and not swap and splits in (None, 1):
+    # From 129 rows: tiles of 256 rows that are half padding still beat 128-row tiles on single CTAs, because few tiles are cut
+    # into pieces (B200, us, single CTAs / pairs: 200 x 4096 x 4096 28.1 / 23.0, 200 x 768 x 4096 28.2 / 14.1, 200 x 28672 x 4096
+    # 63.7 / 57.2, 129 x 4096 x 512 7.6 / 7.6).
+    if use_pair and m > 128 and n >= 256 and not swap and splits in (None, 1):
         if out is None:
             dt = out_dtype or (torch.bfloat16 if a.element_size() == 1 else a.dtype)
             out = torch.empty(m, n, dtype=dt, device=a.device)
