@@ -1,0 +1,56 @@
+"""Rules of the tcgen05 kernels that no run shows while all goes well, checked on their sources."""
+import re
+from pathlib import Path
+
+import pytest
+
+CSRC = Path(__file__).resolve().parent.parent / "torch_dist_ext_b200" / "csrc"
+KERNELS = sorted(p.name for p in CSRC.glob("*.cu"))
+
+
+def _code(name):
+    text = (CSRC / name).read_text()
+    return re.sub(r"//[^\n]*|/\*.*?\*/", lambda m: re.sub(r"[^\n]", " ", m.group()), text, flags=re.S)
+
+
+def _exits_before_barrier(code):
+    """(line of the loop, line of the exit) of every work loop that a thread may leave before the loop's first named barrier."""
+    found = []
+    for barrier in re.finditer(r"tc::named_barrier_sync\(", code):
+        stack = []                                   # (position, text in front) of the blocks that are open here
+        start = 0
+        for m in re.finditer(r"[{}]|;", code[:barrier.start()]):
+            if m.group() == "{":
+                stack.append((m.end(), code[start:m.start()]))
+            elif m.group() == "}" and stack:
+                stack.pop()
+            if m.group() != ";" or code[start:m.start()].count("(") == code[start:m.start()].count(")"):
+                start = m.end()                      # a `;` inside the parentheses of a `for` ends nothing
+        loops = [s for s in stack if re.search(r"\bfor \(", s[1])]
+        if not loops:
+            continue
+        begin = loops[-1][0]
+        body = code[begin:barrier.start()]
+        if "tc::named_barrier_sync(" in body:
+            continue                                 # not the first one
+        kinds, start = [], 0
+        for m in re.finditer(r"[{}]|;|\bbreak;|\breturn;", body):
+            if m.group() == "{":
+                kinds.append(bool(re.search(r"\b(for|while) \(", body[start:m.start()])))
+            elif m.group() == "}":
+                kinds.pop()
+            elif m.group().startswith("return") or (m.group() == "break;" and not any(kinds)):
+                found.append((code.count("\n", 0, begin) + 1, code.count("\n", 0, begin + m.start()) + 1))
+            if m.group() != ";" or body[start:m.start()].count("(") == body[start:m.start()].count(")"):
+                start = m.end()
+    return found
+
+
+@pytest.mark.parametrize("name", KERNELS)
+def test_no_warp_leaves_before_a_named_barrier(name):
+    """Warps that meet at a named barrier inside their work loop all get there, also after a wait that ran out: one that
+    leaves for the kernel's closing __syncthreads keeps the others at the named barrier for good. (Where all of them take
+    the exit together the verdict comes from named_barrier_or.)"""
+    code = _code(name)
+    shared = re.sub(r"if \(named_barrier_or\([^{]*\{[^}]*\}", lambda m: re.sub(r"[^\n]", " ", m.group()), code)
+    assert _exits_before_barrier(shared) == []

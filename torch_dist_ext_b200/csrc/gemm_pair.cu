@@ -136,7 +136,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
   const uint32_t rank = tc::cluster_ctarank();      // even: leader, odd: its peer
   const uint32_t leader = rank & ~1u, other = rank ^ 1u, both = 3u << leader;
   const int pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
-  const int nkb = a.kblocks;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
@@ -243,6 +242,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     const int q = warp & 3;
     const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16);
     const uint32_t leader_acc_empty = tc::map_to_cta(tc::smem_u32(&acc_empty[0]), leader);
+    // A warp whose wait ran out stores nothing more but walks on through its work: the barriers of a tail tile count all four
+    // warps, and the others may have had their last tile.
+    bool ok = true;
     int n = 0;
     WorkItem w;
     for (; work_item(a, pair, npairs, n, &w); ++n) {
@@ -250,11 +252,13 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
       const uint32_t buf = n & 1;
       const int x = (t % a.tiles_x) * kTileM + (int)(rank & 1u) * kRowsPerCta + q * 32 + lane;
       const int y_base = (t / a.tiles_x) * kTileN;
-      // the warp leaves the loop as a whole (tcgen05.ld is a warp-wide instruction)
-      if (nkb <= 0 || !__all_sync(0xffffffffu, tc::mbar_wait(&acc_full[buf], (n >> 1) & 1, kWaitLimit, abort_flag))) {
-        if (nkb > 0 && lane == 0 && q == 0) fail();
-        break;
+      // the warp decides as a whole (tcgen05.ld is a warp-wide instruction)
+      if (ok && !tc::mbar_wait_warp(&acc_full[buf], (n >> 1) & 1, kWaitLimit, abort_flag)) {
+        ok = false;
+        if (lane == 0) fail();
+        __syncwarp();
       }
+      if (!ok && !w.partial) continue;
       tc::fence_after_thread_sync();
       if (a.pieces > 1) {
         // a piece: every MMA of the pair has read its operands, the sums take the ring's place (one row per lane)
@@ -287,7 +291,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         float* tile_ws = a.ws + (size_t)rem * a.tail_parts * slice + half * kRowsPerCta + q * 32 + lane;
         float* mine = tile_ws + (size_t)w.part * slice;
 #pragma unroll 4
-        for (int c = 0; c < kTileN; c += 16) {
+        for (int c = ok ? 0 : kTileN; c < kTileN; c += 16) {
           float v[16];
           tc::tmem_ld_16(lane_addr + buf * kTileN + c, v);
 #pragma unroll
@@ -299,8 +303,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         __threadfence();
         tc::named_barrier_sync(1, 128);
         if (threadIdx.x == 64) {
-          const uint32_t prev = atomicAdd(&a.counters[rem * 2 + half], 1u);
-          *last_flag = (prev == (uint32_t)a.tail_parts - 1u) ? 1u : 0u;        // every piece is non-empty (host)
+          // every piece is non-empty (host); an aborted one is not counted: nobody adds the tile up, and the status says so
+          *last_flag = !*abort_flag && atomicAdd(&a.counters[rem * 2 + half], 1u) == (uint32_t)a.tail_parts - 1u ? 1u : 0u;
         }
         tc::named_barrier_sync(1, 128);
         if (*last_flag) {

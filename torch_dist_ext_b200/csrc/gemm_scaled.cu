@@ -359,6 +359,9 @@ gemm_scaled_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
     };
     uint32_t it = 0;
     bool ready = false;        // the next block's partial product has been seen to be complete
+    // A warp whose wait ran out promotes and stores nothing more but walks on through its work: the barriers of a meeting
+    // count all eight warps, and the other column half may have had its last block.
+    bool ok = true;
     Work w;
     for (int n = 0; next_work(a, worker, workers, n, &w); ++n) {
       const int tile_row = (w.tile % a.tiles_x) * (kRows * kCtas) + (int)rank * kRows + q * 32;
@@ -368,14 +371,16 @@ gemm_scaled_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
       float acc[kHalf];
 #pragma unroll
       for (int j = 0; j < kHalf; ++j) acc[j] = 0.f;
-      bool ok = true;
       const uint32_t end = it + (uint32_t)(w.kb1 - w.kb0);
-      for (; it != end; ++it) {
+      for (; ok && it != end; ++it) {
         // the warp leaves the loop as a whole (tcgen05.ld is a warp-wide instruction)
         if (it % kGroup == 0)
           ok = tc::mbar_wait_warp(&scale_full[(it / kGroup) % kGroups], (it / (kGroup * kGroups)) & 1, kWaitLimit, abort_flag);
         if (!ready) ok = ok && tc::mbar_wait_warp(&part_full[half * 2 + (it & 1)], (it >> 1) & 1, kWaitLimit, abort_flag);
-        if (!ok) break;
+        if (!ok) {
+          if (lane == 0) fail();
+          break;
+        }
         tc::fence_after_thread_sync();
         const float sc = my_scales[(it % (kGroup * kGroups)) * kScalePitch];
         if (live) {
@@ -405,14 +410,11 @@ gemm_scaled_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
           if (tc::elect_one()) tc::mbar_arrive(&scale_empty[(it / kGroup) % kGroups]);
         }
       }
-      if (!ok) {
-        if (lane == 0) fail();
-        break;
-      }
+      __syncwarp();
       if (kCtas == 1 && a.parts > 1) {
         // the meeting in the cluster, below: the sums go to shared memory once every MMA of this CTA has read its stages
         tc::named_barrier_sync(1, kPromoteWarps * 32);
-        if (live) {
+        if (ok && live) {
           float4* mine = reinterpret_cast<float4*>(smem) + row_in_cta * kSumPitch + half * (kHalf / 4);
 #pragma unroll
           for (int j = 0; j < kHalf / 4; ++j) mine[j] = make_float4(acc[4 * j], acc[4 * j + 1], acc[4 * j + 2], acc[4 * j + 3]);
@@ -422,7 +424,7 @@ gemm_scaled_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
       if (kCtas == 2 && n == a.full_rounds && a.parts > 1) {
         // a piece of a tile: leave the sums in this worker's slice (a warp's lanes write 512 consecutive bytes)
         const size_t column = ((size_t)half * (kHalf / 4) * kRows + row_in_cta) * 4;
-        if (live) {
+        if (ok && live) {
           float* mine = a.ws + ((size_t)worker * kCtas + rank) * kSliceFloats + column;
 #pragma unroll
           for (int j = 0; j < kHalf / 4; ++j)
@@ -432,8 +434,8 @@ gemm_scaled_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
         tc::named_barrier_sync(1, kPromoteWarps * 32);
         uint32_t* counter = a.counters + (size_t)(w.tile - a.full_rounds * workers) * kCtas + rank;
         if (threadIdx.x == kFirstPromoteWarp * 32) {
-          const uint32_t prev = atomicAdd(counter, 1u);
-          *last_flag = (prev == (uint32_t)a.parts - 1u) ? 1u : 0u;
+          // an aborted piece is not counted: nobody adds the tile up, and the status says so
+          *last_flag = !*abort_flag && atomicAdd(counter, 1u) == (uint32_t)a.parts - 1u ? 1u : 0u;
         }
         tc::named_barrier_sync(1, kPromoteWarps * 32);
         if (!*last_flag) break;
@@ -461,7 +463,7 @@ gemm_scaled_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
           }
         }
       }
-      if (live) {
+      if (ok && live) {
         if (a.whole_sectors && y0 + kHalf <= a.y_rows) {
           if (x < a.x_rows) {
             char* dst = static_cast<char*>(a.out) + ((int64_t)x * a.sx + y0) * 2;
