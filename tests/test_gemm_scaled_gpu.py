@@ -11,6 +11,8 @@ pytestmark = pytest.mark.gpu
     (1, 256, 128),          # one row, one K block
     (33, 384, 256),         # one and a half tiles of weights
     (64, 7168, 8192),       # decode: tiles in pieces of K
+    (17, 5376, 8192),       # four pieces whose warps add up rows 2 w, 2 w + 1 (+ 16): one row more for half the lanes
+    (49, 3840, 4096),       # the same with eight pieces, 32 rows apart
     (128, 38144, 512),      # decode: 149 tiles, one more than the multiprocessors
     (129, 256, 1024),       # the smallest pair: one row in the second CTA
     (257, 1280, 8192),      # ragged rows, fewer tiles than pairs

@@ -54,3 +54,14 @@ def test_no_warp_leaves_before_a_named_barrier(name):
     code = _code(name)
     shared = re.sub(r"if \(named_barrier_or\([^{]*\{[^}]*\}", lambda m: re.sub(r"[^\n]", " ", m.group()), code)
     assert _exits_before_barrier(shared) == []
+
+
+def test_aligned_cluster_barriers_gather_the_warp():
+    """barrier.cluster.*.aligned is undefined for a warp whose lanes arrive one by one: a lane that skipped a branch, or left a
+    loop early, in front of the barrier. The arrive gathers them, the wait follows it at once."""
+    sources = {p: re.sub(r"//[^\n]*", "", p.read_text()) for p in sorted(CSRC.glob("**/*.cu*"))}
+    raw = [(p.name, s[:m.start()]) for p, s in sources.items() for m in re.finditer(r"barrier\.cluster\.arrive[a-z.]*\.aligned", s)]
+    assert raw and all(re.search(r"__syncwarp\(\);\s*asm volatile\(\"$", before) for _, before in raw), [n for n, _ in raw]
+    for p, s in sources.items():
+        calls = len(re.findall(r"tc::cluster_arrive\(\);", s))
+        assert calls == len(re.findall(r"tc::cluster_arrive\(\);\s*tc::cluster_wait\(\);", s)) == len(re.findall(r"tc::cluster_wait\(\);", s)), p.name

@@ -60,6 +60,29 @@ def test_candidates_of_several_ranks_summed(world):
     assert torch.equal(out.cpu(), want)
 
 
+@pytest.mark.parametrize("vocab", [8192, 16032, 20001])
+def test_a_cluster_per_token_meets_ties_nan_and_minus_infinity(vocab):
+    """From 8192 logits on eight CTAs scan a token's row: CTA c has the vectors 256 c .. 256 c + 255 of every 2048."""
+    g = torch.Generator().manual_seed(vocab)
+    logits = torch.randn(40, vocab, generator=g)
+    logits[0, 7100] = logits[0, 8000] = logits[0, 40] = 9.0     # equal logits in three CTAs
+    logits[1, :] = -1.0                                         # every logit equal
+    logits[2, 5] = float("nan")                                 # a NaN never wins
+    logits[3, :] = float("nan")
+    logits[3, vocab - 1] = -3.0                                 # one number, in the last CTA that has any
+    logits[4, :] = float("nan")                                 # nothing to choose from: index 0
+    logits[5, :] = -float("inf")
+    logits[6, 1:] = -float("inf")
+    logits[7, vocab - 2] = float("inf")
+    want = torch.where(logits.isnan(), torch.full_like(logits, -float("inf")), logits).argmax(dim=-1)
+    want[0], want[1], want[4], want[5] = 40, 0, 0, 0
+    got = sampling.greedy_sample_sharded(logits.cuda(), 0, 1, 0)
+    assert torch.equal(got.cpu(), want)
+    pack = torch.full((40, 8), 123.0, device="cuda")
+    _lib.ops().argmax_pack(logits.cuda(), 1000, 1, 2, pack)
+    assert bool((pack[:, :4] == 0).all()) and bool((pack[:, 6:] == 0).all()) and torch.equal(pack[:, 5].cpu().long(), want + 1000)
+
+
 def test_index_range_is_checked():
     logits = torch.zeros(2, 64, device="cuda")
     pack = torch.empty(2, 4, device="cuda")

@@ -353,7 +353,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
       gemm_core::add_up_cluster<kTileN, 128>(a, tc::smem_u32(smem), threadIdx.x - 64, pair % a.pieces, a.pieces, rank & 1u, 2,
                                              min(kRowsPerCta, a.x_rows - x0), x0, (tile / a.tiles_x) * kTileN);
     }
-    __syncwarp();
     tc::cluster_arrive();
     tc::cluster_wait();        // no CTA leaves while another may still read its sums
   }

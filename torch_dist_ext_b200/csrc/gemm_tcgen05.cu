@@ -381,12 +381,10 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
   }
 
   if (a.cluster) {
-    __syncwarp();
     tc::cluster_arrive();
     tc::cluster_wait();
     if (warp >= 2 && !*abort_flag)
       cluster_finalize<kBN>(a, tc::smem_u32(pipe.smem), tile_x, tile_y * kBN, blockIdx.z, gridDim.z, threadIdx.x - 64);
-    __syncwarp();
     tc::cluster_arrive();
     tc::cluster_wait();        // no CTA leaves while another may still read its sums
   }

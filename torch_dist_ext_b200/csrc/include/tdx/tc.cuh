@@ -320,8 +320,12 @@ __device__ __forceinline__ float ld_cluster_f1(uint32_t cluster_addr) {
   asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(cluster_addr) : "memory");
   return v;
 }
-// Cluster-wide barrier; every thread of every CTA of the cluster executes both halves.
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+// Cluster-wide barrier; every thread of every CTA of the cluster executes both halves. The aligned forms are executed by whole
+// warps together, so the lanes are gathered first: they may come out of a branch or of loops of different lengths.
+__device__ __forceinline__ void cluster_arrive() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 
 // Arrive on an mbarrier of another CTA of the cluster (address from map_to_cta).
