@@ -65,3 +65,17 @@ def test_aligned_cluster_barriers_gather_the_warp():
     for p, s in sources.items():
         calls = len(re.findall(r"tc::cluster_arrive\(\);", s))
         assert calls == len(re.findall(r"tc::cluster_arrive\(\);\s*tc::cluster_wait\(\);", s)) == len(re.findall(r"tc::cluster_wait\(\);", s)), p.name
+
+
+@pytest.mark.parametrize("name", KERNELS)
+def test_tensor_memory_is_fenced_after_a_wait(name):
+    """tcgen05 operations are not ordered by an mbarrier alone: between a wait and the next access to tensor memory (a load, a
+    store, an MMA) in the text stands a tcgen05.fence::after_thread_sync."""
+    code, waited = _code(name), None
+    for m in re.finditer(r"mbar_wait(?:_warp)?\(&?(\w+)|fence_after_thread_sync\(\)|tc::(?:tmem_ld|tmem_st|umma)(?!_commit)\w*\s*[<(]", code):
+        if m.group().startswith("mbar_wait"):
+            waited = code.count("\n", 0, m.start()) + 1
+        elif m.group().startswith("fence"):
+            waited = None
+        else:
+            assert waited is None, f"line {code.count(chr(10), 0, m.start()) + 1}: no fence after the wait of line {waited}"

@@ -384,6 +384,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         ok = false;
         fail();
       }
+      tc::fence_after_thread_sync();    // ... which read it from tensor memory: the tile is written after that product
       tc::named_barrier_sync(2 + g, 2 * kSoftmaxThreads);      // this group's turn at the exponentials
       // probabilities against m_run, row sum, this row of the P tile (bf16, two keys per 32-bit column of tensor memory).
       // A masked score is -FLT_MAX and comes out as zero.
