@@ -79,3 +79,11 @@ def test_tensor_memory_is_fenced_after_a_wait(name):
             waited = None
         else:
             assert waited is None, f"line {code.count(chr(10), 0, m.start()) + 1}: no fence after the wait of line {waited}"
+
+
+def test_the_gate_of_a_late_operand_is_ordered_before_its_choice():
+    """One lane runs the gate and leaves in shared memory which buffer the operand is in; all lanes read that afterwards. A vote
+    alone orders no memory between lanes, __syncwarp does."""
+    code = re.sub(r"//[^\n]*", "", (CSRC / "include" / "tdx" / "gemm_core.cuh").read_text())
+    between = code[code.index("= gate_y();"):code.index("= pick_y();")]
+    assert "__syncwarp();" in between

@@ -245,6 +245,7 @@ struct Pipeline {
     __syncwarp();
     bool passed = false;
     if (tc::elect_one()) passed = gate_y();
+    __syncwarp();             // what the gate wrote to shared memory is visible to all lanes (a vote orders no memory)
     if (!__any_sync(0xffffffffu, passed)) {
       fail(status);
       return;
