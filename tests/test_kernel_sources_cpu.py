@@ -87,3 +87,15 @@ def test_the_gate_of_a_late_operand_is_ordered_before_its_choice():
     code = re.sub(r"//[^\n]*", "", (CSRC / "include" / "tdx" / "gemm_core.cuh").read_text())
     between = code[code.index("= gate_y();"):code.index("= pick_y();")]
     assert "__syncwarp();" in between
+
+
+@pytest.mark.parametrize("name,role,first_wait", [
+    ("gemm_scaled.cu", "} else if (warp <= 2 && rank == 0) {", "mbar_wait"),
+    ("gemm_tcgen05.cu", "} else if (warp == 1) {", ".template issue<"),
+])
+def test_counted_waits_begin_after_the_previous_kernel(name, role, first_wait):
+    """The MMA warps wait for operands with a limit that counts polls. Launched while the previous kernel of the stream still
+    runs (a collective that waits seconds for a late peer), they would use the limit up before the operands can come."""
+    code = _code(name)
+    begin = code.index(role)
+    assert "ptx::pdl_wait();" in code[begin:code.index(first_wait, begin)]

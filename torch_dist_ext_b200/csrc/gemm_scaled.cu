@@ -279,6 +279,7 @@ gemm_scaled_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
     } else if (warp <= 2 && rank == 0) {
       // ---- MMA issue (leader; warp 1: columns 0-127, warp 2: columns 128-255) ----
       const uint32_t half = warp - 1;
+      ptx::pdl_wait();         // a poll-counted wait must not begin while an earlier kernel may still run for seconds
       bool ok = true;
       for (int it = 0; it < blocks; ++it) {
         const uint32_t s = it % kStages, buf = it & 1;

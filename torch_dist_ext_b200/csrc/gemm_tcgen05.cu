@@ -271,6 +271,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
     }, halves ? a.epi.ffn + tile_x * 64 : -1);
     ptx::pdl_launch_dependents();
   } else if (warp == 1) {
+    ptx::pdl_wait();   // a poll-counted wait must not begin while an earlier kernel may still run for seconds
     pipe.template issue<kFp8, kScaled>(nkb, a.idesc, a.status);
   } else {
     ptx::pdl_wait();   // scales, split-K scratch and the output belong to the stream's order
