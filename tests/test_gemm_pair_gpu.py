@@ -60,3 +60,32 @@ def test_partly_filled_last_round_is_split_along_k(m, n, k):
     assert torch.equal(outs[0], outs[1]), "the sum must not depend on which piece arrives last"
     ws, counters, _ = gemm._workspace(a.device)
     assert int(counters.abs().sum()) == 0 and float(ws.abs().max()) == 0.0
+
+
+@pytest.mark.parametrize("m,n,k", [
+    (200, 28672, 8192),     # 112 tiles on 74 pairs: the last 38 in three pieces
+    (200, 19200, 4096),     # 75 tiles: one over
+    (255, 19072, 8192),     # the same, ragged columns
+    (129, 263, 4160),       # two tiles in pieces of a cluster, uneven along K
+    (255, 768, 4096),
+])
+def test_rows_from_129_on(m, n, k):
+    """Tiles of 256 rows that are half padding, the last round or every tile in pieces; and the same product on two streams at
+    a time, each with scratch of its own."""
+    g = torch.Generator(device="cuda").manual_seed(m + n + k)
+    a = [torch.randn(m, k, device="cuda", generator=g).to(torch.bfloat16) for _ in range(2)]
+    w = (torch.randn(n, k, device="cuda", generator=g) * 0.05).to(torch.bfloat16)
+    want = [x.double() @ w.double().t() for x in a]
+    streams = [torch.cuda.Stream() for _ in a]
+    torch.cuda.synchronize()
+    outs = [[], []]
+    for _ in range(4):
+        for i, s in enumerate(streams):
+            with torch.cuda.stream(s):
+                outs[i].append(gemm.linear(a[i], w))
+    torch.cuda.synchronize()
+    assert gemm.pipeline_status() == 0
+    for i in range(2):
+        assert all(torch.equal(outs[i][0], o) for o in outs[i])
+        # half a rounding step of bf16 (2^-9) of the largest value, doubled
+        assert (outs[i][0].double() - want[i]).abs().max() <= want[i].abs().max() * 2.0 ** -8

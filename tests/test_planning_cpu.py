@@ -1,5 +1,6 @@
 """Host-side launch planning of the GEMM and of decode attention (pure Python, no GPU)."""
 import pytest
+import torch
 
 from torch_dist_ext_b200.ops import attention, gemm
 
@@ -86,3 +87,35 @@ def test_pair_finalizer_threads_cover_every_row_pair_and_column_once(bn):
                         assert (row, c) not in seen
                         seen[(row, c)] = (warp, lane)
     assert len(seen) == 128 * bn
+
+
+@pytest.mark.parametrize("m,n,k", [(200, 28672, 8192), (200, 57344, 8192), (200, 19200, 4096), (2048, 4096, 14336), (300, 520, 512)])
+def test_calls_on_cta_pairs_share_no_scratch(m, n, k, monkeypatch):
+    """Two calls may run on two streams at a time: a product whose last tiles are cut along K gets slices and counters of its
+    own, of the size that its plan asks for."""
+    calls = []
+
+    class Ops:
+        def gemm_tn_pair(self, a, w, out, sx, sy, status, ws, counters):
+            calls.append((ws, counters))
+
+        def __getattr__(self, name):
+            return getattr(torch.ops.torch_dist_ext, name)
+
+    monkeypatch.setattr(gemm._lib, "ops", Ops)
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 0)
+    monkeypatch.setattr(gemm, "_workspace", lambda device: (None, torch.zeros(4096, dtype=torch.int32), None))
+    a, w = torch.empty(m, k, dtype=torch.bfloat16), torch.empty(1, k, dtype=torch.bfloat16).expand(n, k)
+    gemm.linear(a, w)
+    gemm.linear(a, w)
+    tiles = -(-m // 256) * -(-n // 256)
+    tail = tiles % (SMS // 2) if tiles > SMS // 2 else 0
+    floats, words = torch.ops.torch_dist_ext.gemm_pair_scratch(m, n, k, 2, SMS)
+    assert (floats, words) == (0, 0) or (words == 2 * tail and floats in [tail * parts * 65536 for parts in (2, 3, 4)])
+    assert (floats > 0) == (n > 4096)
+    (ws0, c0), (ws1, c1) = calls
+    if floats == 0:
+        assert ws0 is None and c0 is None
+    else:
+        assert ws0.numel() == floats and c0.numel() == words and int(c0.abs().sum()) == 0
+        assert ws0.data_ptr() != ws1.data_ptr() and c0.data_ptr() != c1.data_ptr()

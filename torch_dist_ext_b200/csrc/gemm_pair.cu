@@ -432,6 +432,43 @@ std::string launch(const CUtensorMap& mx, const CUtensorMap& my, PairArgs a, dim
 
 }  // namespace
 
+// Tail split: when the last round is partly filled, its tiles are cut along K into `parts` pieces so that the idle
+// pairs share the work; the pieces meet in fp32 scratch slices. parts minimises the time of the tail in tile-times,
+// ceil(tail * parts / pairs) / parts, plus what the pieces pay for meeting in the scratch (128 KB written per CTA,
+// a memory fence and a counter per piece, parts x 128 KB read by the one that adds up: measured about
+// 6 + 3 x parts microseconds, against 8.6 ns of tile time per unit of K).
+PairGemmPlan gemm_pair_plan(int x_rows, int y_rows, int k, int elem_size, int sms) {
+  PairGemmPlan p{};
+  const int kblocks = k / (128 / elem_size);
+  const long long ntiles = (long long)((x_rows + kTileM - 1) / kTileM) * ((y_rows + kTileN - 1) / kTileN);
+  // one pair per two SMs, fewer when there are fewer tiles; pairs that cannot be resident at once simply start later
+  p.pairs = (int)(ntiles < sms / 2 ? ntiles : sms / 2);
+  p.tail_first = (int)ntiles;
+  const int tail = p.pairs > 0 ? (int)(ntiles % p.pairs) : 0;
+  if (tail == 0 || ntiles <= p.pairs) return p;
+  const double tile_us = 8.6e-3 * (double)k;
+  int best = 1;
+  // the unsplit tail costs one tile time; a split has to win by a margin (measured against cuBLAS on the same
+  // box: 2048 x 8192 x 8192 went from 1.14 x to 1.04 x its time with two pieces, 2048 x 4096 x 14336 from 1.17 x to
+  // 1.24 x with four pieces at a predicted 0.90)
+  double best_cost = 0.89;
+  for (int parts = 2; parts <= 4 && kblocks / parts >= 4; ++parts) {
+    const double cost = (double)((tail * parts + p.pairs - 1) / p.pairs) / parts + (6.0 + 3.0 * parts) / tile_us;
+    if (cost < best_cost - 1e-9) {
+      best_cost = cost;
+      best = parts;
+    }
+  }
+  const int per = (kblocks + best - 1) / best;
+  if (best == 1 || (best - 1) * per >= kblocks) return p;      // every piece is non-empty
+  p.tail_first = (int)(ntiles - tail);
+  p.tail_parts = best;
+  p.tail_kb = per;
+  p.slice_floats = (size_t)tail * best * kTileM * kTileN;
+  p.counters = (size_t)tail * 2;
+  return p;
+}
+
 std::string gemm_tn_pair(const GemmProblem& g, cudaStream_t stream) {
   const bool fp8 = g.elem_size == 1;
   if (g.x_scale != nullptr || g.y_scale != nullptr) return "the two-CTA kernel takes unscaled operands";
@@ -456,45 +493,18 @@ std::string gemm_tn_pair(const GemmProblem& g, cudaStream_t stream) {
   if (!err.empty()) return err;
   a.tiles_x = (g.x_rows + kTileM - 1) / kTileM;
   a.tiles_y = (g.y_rows + kTileN - 1) / kTileN;
-  // one pair per two SMs, fewer when there are fewer tiles; pairs that cannot be resident at once simply start later
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const long long ntiles = (long long)a.tiles_x * a.tiles_y;
-  const int pairs = (int)(ntiles < sms / 2 ? ntiles : sms / 2);
-  const dim3 grid(2 * pairs, 1, 1);
-  // Tail split: when the last round is partly filled, its tiles are cut along K into `parts` pieces so that the idle
-  // pairs share the work; the pieces meet in fp32 scratch slices. parts minimises the time of the tail in tile-times,
-  // ceil(tail * parts / pairs) / parts, plus what the pieces pay for meeting in the scratch (128 KB written per CTA,
-  // a memory fence and a counter per piece, parts x 128 KB read by the one that adds up: measured about
-  // 6 + 3 x parts microseconds, against 8.6 ns of tile time per unit of K).
-  a.tail_first = (int)ntiles;
-  a.tail_parts = 0;
-  const int tail = (int)(ntiles % pairs);
-  if (tail > 0 && ntiles > pairs && g.ws != nullptr && g.counters != nullptr && (size_t)tail * 2 <= g.counter_count) {
-    const double tile_us = 8.6e-3 * (double)g.k;
-    int best = 1;
-    // the unsplit tail costs one tile time; a split has to win by a margin (measured against cuBLAS on the same
-    // box: 2048 x 8192 x 8192 went from 1.14 x to 1.04 x its time with two pieces, 2048 x 4096 x 14336 from 1.17 x to
-    // 1.24 x with four pieces at a predicted 0.90)
-    double best_cost = 0.89;
-    for (int parts = 2; parts <= 4 && a.kblocks / parts >= 4; ++parts) {
-      if ((size_t)tail * parts * kTileM * kTileN * sizeof(float) > g.ws_bytes) break;
-      const double cost = (double)((tail * parts + pairs - 1) / pairs) / parts + (6.0 + 3.0 * parts) / tile_us;
-      if (cost < best_cost - 1e-9) {
-        best_cost = cost;
-        best = parts;
-      }
-    }
-    if (best > 1) {
-      a.tail_kb = (a.kblocks + best - 1) / best;
-      if ((best - 1) * a.tail_kb < a.kblocks) {      // every piece non-empty
-        a.tail_first = (int)(ntiles - tail);
-        a.tail_parts = best;
-        a.ws = g.ws;
-        a.counters = g.counters;
-      }
-    }
+  const PairGemmPlan p = gemm_pair_plan(g.x_rows, g.y_rows, g.k, g.elem_size, sms);
+  const dim3 grid(2 * p.pairs, 1, 1);
+  a.tail_first = a.tiles_x * a.tiles_y;
+  if (p.tail_parts > 1 && g.ws != nullptr && g.counters != nullptr && p.slice_floats * sizeof(float) <= g.ws_bytes && p.counters <= g.counter_count) {
+    a.tail_first = p.tail_first;
+    a.tail_parts = p.tail_parts;
+    a.tail_kb = p.tail_kb;
+    a.ws = g.ws;
+    a.counters = g.counters;
   }
   return fp8 ? launch<true>(mx, my, a, grid, stream) : launch<false>(mx, my, a, grid, stream);
 }

@@ -60,7 +60,14 @@ struct GemmProblem {
 
 std::string gemm_tn(const GemmProblem& g, cudaStream_t stream);
 // Same product on 256 x 256 tiles computed by CTA pairs (tcgen05.mma.cta_group::2, gemm_pair.cu). Unscaled
-// operands, no split-K; block_n, splits and the scratch fields are ignored.
+// operands; block_n and splits are ignored. The tiles of a partly filled last round are cut along K where the scratch fields
+// hold what the plan asks for: `slice_floats` fp32 values with any contents and `counters` zeroed words (left zeroed).
+struct PairGemmPlan {
+  int pairs;                             // CTA pairs of the grid
+  int tail_first, tail_parts, tail_kb;   // first tile of the last round, its pieces (0: whole tiles), K blocks per piece
+  size_t slice_floats, counters;
+};
+PairGemmPlan gemm_pair_plan(int x_rows, int y_rows, int k, int elem_size, int sms);
 std::string gemm_tn_pair(const GemmProblem& g, cudaStream_t stream);
 // Same product by a persistent grid (one CTA per SM walks the 128 x 256 tiles, the accumulator double-buffered in
 // tensor memory so that the epilogue of a tile overlaps the main loop of the next; gemm_persist.cu). Unscaled

@@ -336,6 +336,13 @@ void gemm_tn_pair(const Tensor& x, const Tensor& y, Tensor out, int64_t sx, int6
   TORCH_CHECK(err.empty(), "gemm_tn_pair: ", err);
 }
 
+// (fp32 values, zeroed words) of scratch that gemm_tn_pair uses for a product on a device of `sms` multiprocessors
+std::vector<int64_t> gemm_pair_scratch(int64_t m, int64_t n, int64_t k, int64_t elem_size, int64_t sms) {
+  TORCH_CHECK(m >= 0 && n >= 0 && k >= 0 && (elem_size == 1 || elem_size == 2) && sms >= 2, "gemm_pair_scratch: sizes out of range");
+  const tdx::PairGemmPlan p = tdx::gemm_pair_plan((int)m, (int)n, (int)k, (int)elem_size, (int)sms);
+  return {(int64_t)p.slice_floats, (int64_t)p.counters};
+}
+
 // The same product by a persistent grid with the accumulator double-buffered in tensor memory.
 void gemm_tn_persistent(const Tensor& x, const Tensor& y, Tensor out, int64_t sx, int64_t sy, const c10::optional<Tensor>& status,
                         bool x_static) {
@@ -608,6 +615,7 @@ void register_extra_ops(torch::Library& m) {
         "Tensor(d!)? status) -> ()", &gemm_tn_silu_mul);
   m.def("gemm_tn_pair(Tensor x, Tensor y, Tensor(a!) out, int sx, int sy, Tensor(b!)? status, Tensor(c!)? ws=None, "
         "Tensor(d!)? counters=None) -> ()", &gemm_tn_pair);
+  m.def("gemm_pair_scratch(int m, int n, int k, int elem_size, int sms) -> int[]", &gemm_pair_scratch);
   m.def("gemm_tn_persistent(Tensor x, Tensor y, Tensor(a!) out, int sx, int sy, Tensor(b!)? status, bool x_static=False) -> ()",
         &gemm_tn_persistent);
   m.def("fused_add_rmsnorm(Tensor x, Tensor? residual_in, Tensor gamma, Tensor(a!)? residual_out, Tensor(b!) norm_out, "

@@ -10,6 +10,7 @@ efficiency; K is split over CTAs until the grid covers the 148 SMs.
 """
 from __future__ import annotations
 
+import functools
 import os
 from typing import Optional, Tuple
 
@@ -36,16 +37,17 @@ def _workspace(device: torch.device):
     return _ws[key]
 
 
-_pair_ws = {}
+def _pair_scratch(device: torch.device, floats: int = 73 * 4 * 256 * 256) -> torch.Tensor:
+    """Scratch of the CTA-pair kernel's tail split: fp32 partial tiles with any contents, of one call only (two calls on
+    two streams would mix their tiles in a common one). Without ``floats``: the most that a call needs."""
+    return torch.empty(floats, dtype=torch.float32, device=device)
 
 
-def _pair_scratch(device: torch.device) -> torch.Tensor:
-    """Scratch of the CTA-pair kernel's tail split: fp32 partial tiles, contents undefined between calls (unlike the
-    split-K scratch above, which every kernel leaves zeroed)."""
-    key = device.index if device.index is not None else torch.cuda.current_device()
-    if key not in _pair_ws:
-        _pair_ws[key] = torch.empty(20 << 20, dtype=torch.float32, device=device)      # 80 MiB: 73 tiles x 4 pieces
-    return _pair_ws[key]
+@functools.lru_cache(maxsize=4096)
+def _pair_tail(m: int, n: int, k: int, elem_size: int, device: torch.device) -> Tuple[int, int]:
+    """(fp32 values, zeroed words) of scratch of a product on CTA pairs; zeros where no tile is cut along K."""
+    sms = torch.cuda.get_device_properties(device).multi_processor_count if device.type == "cuda" else _SM_COUNT
+    return tuple(_lib.ops().gemm_pair_scratch(m, n, k, elem_size, sms))
 
 
 def pipeline_status(device=None) -> int:
@@ -101,8 +103,11 @@ def linear(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None,
         if out is None:
             dt = out_dtype or (torch.bfloat16 if a.element_size() == 1 else a.dtype)
             out = torch.empty(m, n, dtype=dt, device=a.device)
-        _, counters, status = _workspace(a.device)
-        _lib.ops().gemm_tn_pair(a, w, out, n, 1, status, _pair_scratch(a.device), counters)   # K-split of a partly filled last round
+        ws = counters = None
+        floats, words = _pair_tail(m, n, k, a.element_size(), a.device)
+        if floats:                                            # K-split of a partly filled last round
+            ws, counters = _pair_scratch(a.device, floats), torch.zeros(words, dtype=torch.int32, device=a.device)
+        _lib.ops().gemm_tn_pair(a, w, out, n, 1, _workspace(a.device)[2], ws, counters)
         return out
     if (use_persistent or (use_pair and persistent is None and _PERSIST_DEFAULT)) and m > 128 and n >= 256 and not swap \
             and splits in (None, 1):
