@@ -119,3 +119,30 @@ def test_calls_on_cta_pairs_share_no_scratch(m, n, k, monkeypatch):
     else:
         assert ws0.numel() == floats and c0.numel() == words and int(c0.abs().sum()) == 0
         assert ws0.data_ptr() != ws1.data_ptr() and c0.data_ptr() != c1.data_ptr()
+
+
+@pytest.mark.parametrize("m,n,default,persistent,walks", [
+    (64, 28672, True, None, True), (64, 28672, False, None, False),     # TDX_GEMM_PERSIST=0: one tile per CTA
+    (64, 28672, False, True, True), (64, 28672, True, False, False),    # an explicit choice of the call
+    (1, 18945, True, None, True), (1, 18944, True, None, False), (129, 200, True, None, False),
+])
+def test_the_persistent_kernel_can_be_turned_off(m, n, default, persistent, walks, monkeypatch):
+    taken = []
+
+    class Ops:
+        class linear_decode:
+            default = staticmethod(lambda *args: taken.append("tiles"))
+
+        def gemm_tn(self, *args):
+            taken.append("tiles")
+
+        def gemm_tn_persistent(self, *args):
+            taken.append("walk")
+
+    monkeypatch.setattr(gemm._lib, "ops", Ops)
+    monkeypatch.setattr(gemm, "_PERSIST_DEFAULT", default)
+    monkeypatch.setattr(gemm, "_workspace", lambda device: (None, None, None))
+    a, w = torch.empty(m, 64, dtype=torch.bfloat16), torch.empty(1, 64, dtype=torch.bfloat16).expand(n, 64)
+    gemm.linear(a, w, persistent=persistent)
+    gemm.linear(a, w, torch.empty(m, n, dtype=torch.bfloat16), persistent=persistent)
+    assert taken == ["walk" if walks else "tiles"] * 2
