@@ -146,3 +146,22 @@ def test_the_persistent_kernel_can_be_turned_off(m, n, default, persistent, walk
     gemm.linear(a, w, persistent=persistent)
     gemm.linear(a, w, torch.empty(m, n, dtype=torch.bfloat16), persistent=persistent)
     assert taken == ["walk" if walks else "tiles"] * 2
+
+
+@pytest.mark.parametrize("m,n,k", [(64, 7168, 1024), (2, 256, 4096)])
+def test_block_scaled_output_type_may_be_none(m, n, k, monkeypatch):
+    """``out_dtype=None`` means torch's default type, for the kernel that allocates its output natively and for the other."""
+    made = []
+
+    class Ops:
+        class gemm_scaled_call:
+            default = staticmethod(lambda a, w, out_dtype, *rest: made.append(out_dtype))
+
+        def gemm_tn(self, w, a, out, *rest):
+            made.append(out.dtype)
+
+    monkeypatch.setattr(gemm._lib, "ops", Ops)
+    monkeypatch.setattr(gemm, "_workspace", lambda device: (None, None, None))
+    a, w = torch.empty(m, k, dtype=torch.float8_e4m3fn), torch.empty(n, k, dtype=torch.float8_e4m3fn)
+    gemm.linear_fp8_blockscaled(a, torch.empty(m, k // 128), w, torch.empty(n // 128, k // 128), out_dtype=None)
+    assert made == [torch.float32]

@@ -160,6 +160,8 @@ def linear_fp8_blockscaled(a_q: torch.Tensor, a_scale: torch.Tensor, w_q: torch.
     # 32 tokens 9.2 / 10.5; 7168 x 8192 at 16 tokens 19.4 / 17.8, 1280 x 8192 at 64 tokens 13.1 / 11.6, 8192 x 1024 at 1 token
     # 6.5 / 6.4, 28672 x 8192 at 64 tokens 81 / 47.
     few = m <= 32 and n <= 20 * 256 and k > 2048
+    if out_dtype is None:
+        out_dtype = torch.get_default_dtype()      # as torch.empty takes it
     if splits is None and not few and out is None:
         return _lib.ops().gemm_scaled_call.default(a_q, w_q, out_dtype, a_scale.contiguous(), w_scale.contiguous(), status)
     if out is None:
