@@ -88,3 +88,9 @@ def test_index_range_is_checked():
     pack = torch.empty(2, 4, device="cuda")
     with pytest.raises(RuntimeError, match="2\\^24"):
         _lib.ops().argmax_pack(logits, 1 << 24, 0, 1, pack)
+
+
+@pytest.mark.parametrize("rank,world", [(1, 1), (-1, 1), (2, 2), (0, 0)])
+def test_rank_is_checked(rank, world):
+    with pytest.raises(RuntimeError, match="rank"):
+        sampling.greedy_sample_sharded(torch.zeros(2, 64, device="cuda"), rank, world, 0)

@@ -27,7 +27,7 @@ def greedy_sample_sharded(logits: torch.Tensor, rank: int, world: int, index_bas
     if not logits.is_cuda:
         return _ref.greedy_sample_sharded(logits, rank, world, index_base)
     ops = _lib.ops()
-    if world == 1:
+    if world == 1 and rank == 0:          # (any other rank is refused below)
         return ops.argmax_tokens.default(logits, index_base)
     pack = torch.empty(tokens, 4 * world, dtype=torch.float32, device=logits.device)
     ops.argmax_pack(logits, index_base, rank, world, pack)
