@@ -165,3 +165,23 @@ def test_block_scaled_output_type_may_be_none(m, n, k, monkeypatch):
     a, w = torch.empty(m, k, dtype=torch.float8_e4m3fn), torch.empty(n, k, dtype=torch.float8_e4m3fn)
     gemm.linear_fp8_blockscaled(a, torch.empty(m, k // 128), w, torch.empty(n // 128, k // 128), out_dtype=None)
     assert made == [torch.float32]
+
+
+def test_remembered_splits_follow_the_value_of_max_len(monkeypatch):
+    """Split counts are remembered by their sizes. A length held in a tensor counts by its value, not by the tensor."""
+    seen = []
+
+    class Ops:
+        class attention_decode_call:
+            default = staticmethod(lambda q, k, v, lens, part, nsplit, *rest: seen.append(nsplit))
+
+    monkeypatch.setattr(attention._lib, "ops", Ops)
+    monkeypatch.setattr(attention, "_resident_clusters", lambda device: {})
+    monkeypatch.setattr(attention, "_partial", lambda device, floats: None)
+    monkeypatch.setattr(gemm, "_workspace", lambda device: (None, None, None))
+    q, cache, length = torch.empty(1, 8, 128), torch.empty(1, 1, 1, 128).expand(1, 8192, 1, 128), torch.tensor(128)
+    for n in (128, 8192):
+        length.fill_(n)
+        attention.decode_attention(q, cache, cache, None, length)
+        attention.decode_attention(q, cache, cache, None, n)
+    assert seen[0] == seen[1] == 1 and seen[2] == seen[3] > 8

@@ -97,7 +97,7 @@ def decode_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tens
     device = q.device
     use_tc = _TC_DEFAULT if tensor_cores is None else tensor_cores
     if nsplit is None:
-        nsplit = _planned_splits(b, k_cache.shape[2], max_len, use_tc, device)
+        nsplit = _planned_splits(b, k_cache.shape[2], int(max_len), use_tc, device)
     part = _partial(device, 4096 + b * hq * nsplit * (d + 2))
     if out is None:
         return _lib.ops().attention_decode_call.default(q, k_cache, v_cache, seq_lens, part, nsplit, 1.0 / math.sqrt(d),
