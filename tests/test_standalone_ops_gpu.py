@@ -80,3 +80,25 @@ def test_rope_append_kv_writes_the_cache_rows():
     assert torch.equal(kc[idx, pos], k) and (k.float() - e_k.float()).abs().max().item() <= 3.2e-2
     assert torch.equal(vc[idx, pos], v)
     assert kc.abs().sum().item() == kc[idx, pos].abs().sum().item()      # nothing else was touched
+
+
+@pytest.mark.parametrize("rows,inter", [
+    (1, 8),            # one vector
+    (1, 1792),         # one vector per thread, a part of the last warp idle
+    (300, 8200),       # as many threads as vectors; 1025 vectors to a row
+    (2369, 1024),      # one row more than the grid has threads for: some threads take a second vector
+    (5000, 3584),      # several vectors per thread, steps across rows
+])
+def test_silu_mul_walks_rows(rows, inter):
+    gu = torch.randn(rows, 2 * inter, device="cuda", generator=torch.Generator(device="cuda").manual_seed(rows)).to(torch.bfloat16)
+    want = torch.nn.functional.silu(gu[:, :inter].double()) * gu[:, inter:].double()
+    out, _ = activation.silu_mul(gu)
+    # half a rounding step of bf16 and the error of the fp32 exponential and division, a few 2^-22 of the value
+    assert ((out.double() - want).abs() <= want.abs() * (2.0 ** -9 + 2.0 ** -18) + 1e-30).all()
+    if inter % 128 == 0:
+        q, scales = activation.silu_mul(gu, quant_block128=True)
+        amax = out.float().view(rows, inter // 128, 128).abs().amax(-1)
+        assert torch.allclose(scales, amax.clamp_min(1e-10) / 448.0, rtol=2.0 ** -22)
+        back = q.double().view(rows, inter // 128, 128) * scales.double()[..., None]
+        # half an e4m3 step: 2^-4 of the value, or half the smallest subnormal (2^-10) of the scale
+        assert ((back - out.double().view_as(back)).abs() <= out.double().view_as(back).abs() * 2.0 ** -4 * 1.01 + scales.double()[..., None] * 2.0 ** -10).all()

@@ -104,15 +104,15 @@ __global__ void __launch_bounds__(256) silu_mul_kernel(const T* __restrict__ in,
   ptx::pdl_launch_dependents();
   const int nvec = inter / kVec;
   const size_t total = (size_t)rows * nvec;
-  const size_t stride = (size_t)gridDim.x * blockDim.x;
   // Row and column of this thread's vector are carried along (one division per thread, not one per vector), and the next
-  // vectors are requested before the current ones are used. Warp-uniform trip count: the quantising variant shuffles
-  // inside the loop.
-  const size_t first = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  size_t row = first / nvec;
-  int i = int(first % nvec);
-  const size_t row_step = stride / nvec;
-  const int col_step = int(stride % nvec);
+  // vectors are requested before the current ones are used. The grid has far fewer than 2^32 threads, so the divisions are
+  // 32-bit ones; the step is divided behind the first request, and not at all where every thread has one vector (64-bit
+  // divisions of both in front of it cost a small call 0.35 of 2.05 us, B200, 1 x 1792). Warp-uniform trip count: the
+  // quantising variant shuffles inside the loop.
+  const uint32_t stride = gridDim.x * blockDim.x;
+  const uint32_t first = blockIdx.x * blockDim.x + threadIdx.x;
+  size_t row = first / (uint32_t)nvec;
+  int i = int(first % (uint32_t)nvec);
   const size_t row_bytes = (size_t)inter * sizeof(T);
   uint4 gate = make_uint4(0u, 0u, 0u, 0u), up = gate;
   auto request = [&](size_t r, int col) {
@@ -121,7 +121,9 @@ __global__ void __launch_bounds__(256) silu_mul_kernel(const T* __restrict__ in,
     up = ptx::ld_stream_v4(src + row_bytes);
   };
   if (first < total) request(row, i);
-  for (size_t base = first & ~(size_t)31; base < total; base += stride) {
+  const uint32_t row_step = stride < total ? stride / (uint32_t)nvec : 0u;
+  const int col_step = stride < total ? int(stride % (uint32_t)nvec) : 0;
+  for (size_t base = first & ~31u; base < total; base += stride) {
     const bool live = base + (threadIdx.x & 31u) < total;
     float g[kVec], u[kVec], y[kVec];
     unpack<T>(gate, g);
@@ -391,7 +393,7 @@ std::string silu_mul(const void* in, void* out, float* scales, int rows, int int
   const int vec = dtype == kF32 ? 4 : 8;
   if (inter % vec) return "intermediate size must be a multiple of 16 bytes";
   if (quant_block128 && inter % 128) return "1x128 block scaling needs intermediate size % 128 == 0";
-  if (rows == 0) return "";
+  if (rows == 0 || inter == 0) return "";
   const size_t total = (size_t)rows * (inter / vec);
   const int grid = grid_for(total, 256);
   TDX_DISPATCH_DTYPE(dtype, {
