@@ -93,8 +93,8 @@ def test_silu_mul_walks_rows(rows, inter):
     gu = torch.randn(rows, 2 * inter, device="cuda", generator=torch.Generator(device="cuda").manual_seed(rows)).to(torch.bfloat16)
     want = torch.nn.functional.silu(gu[:, :inter].double()) * gu[:, inter:].double()
     out, _ = activation.silu_mul(gu)
-    # half a rounding step of bf16 and the error of the fp32 exponential and division, a few 2^-22 of the value
-    assert ((out.double() - want).abs() <= want.abs() * (2.0 ** -9 + 2.0 ** -18) + 1e-30).all()
+    # half a rounding step of bf16 (2^-8 of the value where its fraction is 1.0) and a few 2^-22 of the fp32 operations
+    assert ((out.double() - want).abs() <= want.abs() * (2.0 ** -8 + 2.0 ** -18) + 1e-30).all()
     if inter % 128 == 0:
         q, scales = activation.silu_mul(gu, quant_block128=True)
         amax = out.float().view(rows, inter // 128, 128).abs().amax(-1)

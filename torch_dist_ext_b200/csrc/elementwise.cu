@@ -96,7 +96,8 @@ __global__ void __launch_bounds__(512) quant_fp8_kernel(const T* __restrict__ x,
 // ---- SiLU(gate) * up --------------------------------------------------------------------------
 // in: [rows, 2*inter] with the gate in the first half of each row; out: [rows, inter].
 // kQuant: out is e4m3 with 1x128 block scales (input of an fp8 block-scaled down projection).
-template <typename T, bool kQuant>
+// kWalk: there are more vectors than threads.
+template <typename T, bool kQuant, bool kWalk>
 __global__ void __launch_bounds__(256) silu_mul_kernel(const T* __restrict__ in, void* __restrict__ out,
                                                        float* __restrict__ scales, int rows, int inter) {
   constexpr int kVec = VecTraits<T>::kVec;
@@ -106,9 +107,10 @@ __global__ void __launch_bounds__(256) silu_mul_kernel(const T* __restrict__ in,
   const size_t total = (size_t)rows * nvec;
   // Row and column of this thread's vector are carried along (one division per thread, not one per vector), and the next
   // vectors are requested before the current ones are used. The grid has far fewer than 2^32 threads, so the divisions are
-  // 32-bit ones; the step is divided behind the first request, and not at all where every thread has one vector (64-bit
-  // divisions of both in front of it cost a small call 0.35 of 2.05 us, B200, 1 x 1792). Warp-uniform trip count: the
-  // quantising variant shuffles inside the loop.
+  // 32-bit ones. Where every thread has one vector nothing of the walk is compiled in: a call of a few microseconds is also
+  // bound by the instructions it fetches (B200, us, one division per vector / the walk with 64-bit divisions / without the
+  // walk: 1 x 1792 1.71 / 2.05 / 1.80, 64 x 14336 3.08 / 3.50 / 2.58). Warp-uniform trip count: the quantising variant
+  // shuffles inside the loop.
   const uint32_t stride = gridDim.x * blockDim.x;
   const uint32_t first = blockIdx.x * blockDim.x + threadIdx.x;
   size_t row = first / (uint32_t)nvec;
@@ -121,8 +123,8 @@ __global__ void __launch_bounds__(256) silu_mul_kernel(const T* __restrict__ in,
     up = ptx::ld_stream_v4(src + row_bytes);
   };
   if (first < total) request(row, i);
-  const uint32_t row_step = stride < total ? stride / (uint32_t)nvec : 0u;
-  const int col_step = stride < total ? int(stride % (uint32_t)nvec) : 0;
+  const uint32_t row_step = kWalk ? stride / (uint32_t)nvec : 0u;
+  const int col_step = kWalk ? int(stride % (uint32_t)nvec) : 0;
   for (size_t base = first & ~31u; base < total; base += stride) {
     const bool live = base + (threadIdx.x & 31u) < total;
     float g[kVec], u[kVec], y[kVec];
@@ -130,13 +132,15 @@ __global__ void __launch_bounds__(256) silu_mul_kernel(const T* __restrict__ in,
     unpack<T>(up, u);
     const size_t at_row = row;
     const int at = i;
-    row += row_step;
-    i += col_step;
-    if (i >= nvec) {
-      i -= nvec;
-      ++row;
+    if constexpr (kWalk) {
+      row += row_step;
+      i += col_step;
+      if (i >= nvec) {
+        i -= nvec;
+        ++row;
+      }
+      if (base + stride + (threadIdx.x & 31u) < total) request(row, i);
     }
-    if (base + stride + (threadIdx.x & 31u) < total) request(row, i);
 #pragma unroll
     for (int k = 0; k < kVec; ++k) y[k] = live ? g[k] / (1.f + __expf(-g[k])) * u[k] : 0.f;
     if constexpr (kQuant) {
@@ -158,6 +162,7 @@ __global__ void __launch_bounds__(256) silu_mul_kernel(const T* __restrict__ in,
     } else {
       if (live) ptx::st_stream_v4(static_cast<char*>(out) + (at_row * inter + (size_t)at * kVec) * sizeof(T), pack<T>(y));
     }
+    if constexpr (!kWalk) break;
   }
 }
 
@@ -397,10 +402,10 @@ std::string silu_mul(const void* in, void* out, float* scales, int rows, int int
   const size_t total = (size_t)rows * (inter / vec);
   const int grid = grid_for(total, 256);
   TDX_DISPATCH_DTYPE(dtype, {
-    if (quant_block128)
-      launch_chained(silu_mul_kernel<T, true>, dim3(grid), dim3(256), 0, stream, static_cast<const T*>(in), out, scales, rows, inter);
-    else
-      launch_chained(silu_mul_kernel<T, false>, dim3(grid), dim3(256), 0, stream, static_cast<const T*>(in), out, scales, rows, inter);
+    const bool walk = total > (size_t)grid * 256;
+    auto kern = quant_block128 ? (walk ? silu_mul_kernel<T, true, true> : silu_mul_kernel<T, true, false>)
+                               : (walk ? silu_mul_kernel<T, false, true> : silu_mul_kernel<T, false, false>);
+    launch_chained(kern, dim3(grid), dim3(256), 0, stream, static_cast<const T*>(in), out, scales, rows, inter);
   });
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? "" : cudaGetErrorString(e);
