@@ -53,3 +53,28 @@ def test_pieces_of_a_pair_tile_match_64_bit(m, n, k, out_dtype):
     # as above
     bound = want.abs().max() * (2.0 ** -8 if out_dtype == torch.bfloat16 else k * 2.0 ** -22)
     assert (outs[0].double() - want).abs().max() <= bound
+
+
+@pytest.mark.parametrize("m,n,k", [
+    (129, 200, 4096),    # a 256-wide tile of which 200 columns are there, one row in the second row tile
+    (300, 64, 2048),     # 64-wide
+    (512, 192, 8192),
+    (200, 130, 6400),   # output rows that are no multiple of four values: stored one by one
+])
+@pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float16, torch.float32])
+def test_splits_of_tall_products(m, n, k, out_dtype):
+    """More than 128 rows of a weight with fewer than 256: the activations are on the 128-row side and columns contiguous."""
+    g = torch.Generator(device="cuda").manual_seed(m + n + k)
+    dtype = torch.float16 if out_dtype == torch.float16 else torch.bfloat16
+    a = torch.randn(m, k, device="cuda", generator=g).to(dtype)
+    w = (torch.randn(n, k, device="cuda", generator=g) * 0.05).to(dtype)
+    want = a.double() @ w.double().t()
+    outs = [gemm.linear(a, w, out_dtype=out_dtype) for _ in range(2)]
+    torch.cuda.synchronize()
+    assert gemm.pipeline_status() == 0 and torch.equal(outs[0], outs[1])
+    bound = want.abs().max() * (k * 2.0 ** -22 if out_dtype == torch.float32 else 2.0 ** -8)      # as above
+    assert (outs[0].double() - want).abs().max() <= bound
+    # an output that starts in the middle of a wider buffer, two values off a 16-byte boundary
+    wide = torch.zeros(m * n + 2, device="cuda", dtype=out_dtype)
+    gemm.linear(a, w, wide[2:].view(m, n), out_dtype=out_dtype)
+    assert torch.equal(wide[2:].view(m, n), outs[0]) and not wide[:2].any()
