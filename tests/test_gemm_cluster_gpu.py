@@ -78,3 +78,34 @@ def test_splits_of_tall_products(m, n, k, out_dtype):
     wide = torch.zeros(m * n + 2, device="cuda", dtype=out_dtype)
     gemm.linear(a, w, wide[2:].view(m, n), out_dtype=out_dtype)
     assert torch.equal(wide[2:].view(m, n), outs[0]) and not wide[:2].any()
+
+
+@pytest.mark.parametrize("m,n,k", [
+    (16, 128, 16384),    # one tile of sixteen splits
+    (33, 512, 14336),    # four
+    (5, 640, 14400),     # five, 225 K blocks: fifteen splits of fifteen
+    (128, 250, 8192),    # two, ragged rows
+    (17, 1024, 14336),   # eight tiles: no room for sixteen
+    (160, 64, 14336),    # the activations on the 128-row side
+    (256, 200, 8192),
+])
+@pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32])
+def test_few_tiles_and_a_long_k(m, n, k, out_dtype):
+    """Clusters of up to sixteen splits, which share nothing with a call on another stream: both at a time."""
+    g = torch.Generator(device="cuda").manual_seed(m + n + k)
+    a = [torch.randn(m, k, device="cuda", generator=g).to(torch.bfloat16) for _ in range(2)]
+    w = (torch.randn(n, k, device="cuda", generator=g) * 0.05).to(torch.bfloat16)
+    want = [x.double() @ w.double().t() for x in a]
+    streams = [torch.cuda.Stream() for _ in a]
+    torch.cuda.synchronize()
+    outs = [[], []]
+    for _ in range(4):
+        for i, s in enumerate(streams):
+            with torch.cuda.stream(s):
+                outs[i].append(gemm.linear(a[i], w, out_dtype=out_dtype))
+    torch.cuda.synchronize()
+    assert gemm.pipeline_status() == 0
+    for i in range(2):
+        assert all(torch.equal(outs[i][0], o) for o in outs[i]), "the splits are added in a fixed order"
+        bound = want[i].abs().max() * (k * 2.0 ** -22 if out_dtype == torch.float32 else 2.0 ** -8)      # as above
+        assert (outs[i][0].double() - want[i]).abs().max() <= bound

@@ -163,13 +163,13 @@ __device__ __forceinline__ void pair_finalize(const GemmArgs& a, int tile_x, flo
 // Every CTA has left its 128 x kBN sums in its shared memory ([column][128 rows]) and passed the cluster barrier. CTA
 // `rank` finishes the columns rank * kBN / splits ..: its 128 epilogue threads (`t`) add up the splits' values in the
 // order of the splits and store, rotate or activate them.
-constexpr int kMaxCluster = 8;
+constexpr int kMaxCluster = 16;
 
-template <int kCols>
+template <int kMost, int kCols>
 __device__ __forceinline__ void cluster_sums(uint32_t base, int splits, int column, int row, float (&sum)[kCols]) {
-  float v[kCols][kMaxCluster];
+  float v[kCols][kMost];
 #pragma unroll
-  for (int p = 0; p < kMaxCluster; ++p) {
+  for (int p = 0; p < kMost; ++p) {
     if (p >= splits) continue;
     const uint32_t src = tc::map_to_cta(base + (uint32_t)((column * kBM + row) * 4), p);
 #pragma unroll
@@ -179,12 +179,12 @@ __device__ __forceinline__ void cluster_sums(uint32_t base, int splits, int colu
   for (int j = 0; j < kCols; ++j) {
     sum[j] = 0.f;
 #pragma unroll
-    for (int p = 0; p < kMaxCluster; ++p)
+    for (int p = 0; p < kMost; ++p)
       if (p < splits) sum[j] += v[j][p];
   }
 }
 
-template <int kBN>
+template <int kBN, int kMost>
 __device__ __forceinline__ void cluster_finalize(const GemmArgs& a, uint32_t base, int tile_x, int y_base, int rank, int splits, int t) {
   const int share = (kBN + splits - 1) / splits;
   const int c0 = rank * share, c1 = min(min(kBN, c0 + share), a.y_rows - y_base);
@@ -200,7 +200,7 @@ __device__ __forceinline__ void cluster_finalize(const GemmArgs& a, uint32_t bas
       const bool aligned = (a.sx * esz) % (4 * esz) == 0 && reinterpret_cast<uintptr_t>(a.out) % (4 * esz) == 0;
       for (int c = c0; c < c1; c += 4) {
         float s[4];
-        cluster_sums<4>(base, splits, c, t, s);
+        cluster_sums<kMost, 4>(base, splits, c, t, s);
         if (x >= a.x_rows) continue;
         if (aligned && c + 4 <= c1) {
           if (a.out_dtype == kF32) *reinterpret_cast<float4*>(static_cast<float*>(a.out) + row + c) = make_float4(s[0], s[1], s[2], s[3]);
@@ -217,7 +217,7 @@ __device__ __forceinline__ void cluster_finalize(const GemmArgs& a, uint32_t bas
     }
     for (int c = c0; c < c1; c += 2) {
       float s[2];
-      cluster_sums<2>(base, splits, c, t, s);      // an odd share's last column is followed by one that is in bounds too
+      cluster_sums<kMost, 2>(base, splits, c, t, s);      // an odd share's last column is followed by one that is in bounds too
       if (x >= a.x_rows) continue;
       gemm_core::store_out(a, (int64_t)x * a.sx + (int64_t)(y_base + c) * a.sy, s[0]);
       if (c + 1 < c1) gemm_core::store_out(a, (int64_t)x * a.sx + (int64_t)(y_base + c + 1) * a.sy, s[1]);
@@ -235,8 +235,8 @@ __device__ __forceinline__ void cluster_finalize(const GemmArgs& a, uint32_t bas
     const int y = y_base + c;
     const int pos = rope ? (int)__ldg(e.positions + y) : 0;
     float lo[1], hi[1];
-    cluster_sums<1>(base, splits, c, r, lo);
-    cluster_sums<1>(base, splits, c, r + 64, hi);
+    cluster_sums<kMost, 1>(base, splits, c, r, lo);
+    cluster_sums<kMost, 1>(base, splits, c, r + 64, hi);
     const int64_t at = x_lo * a.sx + (int64_t)y * a.sy;
     if (!rope) {   // silu(gate) * up
       gemm_core::store_out(a, at, lo[0] / (1.f + __expf(-lo[0])) * hi[0]);
@@ -259,7 +259,9 @@ __device__ __forceinline__ void cluster_finalize(const GemmArgs& a, uint32_t bas
   }
 }
 
-template <int kBN, int kStages, bool kFp8, bool kScaled>
+// kMost: the largest cluster, 8 or 16 (the finishing loops are unrolled over the splits; compiled for sixteen, a meeting of
+// at most eight took 0.1 to 0.3 us longer).
+template <int kBN, int kStages, bool kFp8, bool kScaled, int kMost>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_tn_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_y, const GemmArgs a) {
   using L = SmemLayout<kBN, kStages>;
@@ -409,7 +411,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
     tc::cluster_arrive();
     tc::cluster_wait();
     if (warp >= 2 && !*abort_flag)
-      cluster_finalize<kBN>(a, tc::smem_u32(pipe.smem), tile_x, tile_y * kBN, blockIdx.z, gridDim.z, threadIdx.x - 64);
+      cluster_finalize<kBN, kMost>(a, tc::smem_u32(pipe.smem), tile_x, tile_y * kBN, blockIdx.z, gridDim.z, threadIdx.x - 64);
     tc::cluster_arrive();
     tc::cluster_wait();        // no CTA leaves while another may still read its sums
   }
@@ -440,7 +442,8 @@ int resident_clusters(Kernel kern, int smem, int splits) {
   attr[0].val.clusterDim.z = splits;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
+  if ((splits > 8 && cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) ||
+      cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
     cudaGetLastError();
     n = 0;
   }
@@ -448,24 +451,41 @@ int resident_clusters(Kernel kern, int smem, int splits) {
   return n;
 }
 
-template <int kBN, int kStages, bool kFp8, bool kScaled>
+// kWide: clusters of more than eight are compiled too.
+template <int kBN, int kStages, bool kFp8, bool kScaled, bool kWide = false>
 std::string launch(const CUtensorMap& mx, const CUtensorMap& my, GemmArgs a, dim3 grid, cudaStream_t stream) {
   using L = SmemLayout<kBN, kStages>;
-  auto kern = gemm_tn_kernel<kBN, kStages, kFp8, kScaled>;
-  const std::string err = reserve_dynamic_smem(kern, L::kTotal);
+  auto kern = gemm_tn_kernel<kBN, kStages, kFp8, kScaled, 8>;
+  std::string err = reserve_dynamic_smem(kern, L::kTotal);
   if (!err.empty()) return err;
-  // K splits meet inside a cluster where the device holds one cluster per tile at a time: as many splits as were asked
-  // for, at most eight.
+  // K splits meet inside a cluster where the device holds one cluster per tile at a time: as many splits as were asked for,
+  // at most eight. With few tiles and a long K eight CTAs a tile leave most of the device idle, so up to sixteen are taken
+  // (more than eight is a size that the kernel opts into) where the K blocks that a CTA is spared weigh more than the larger
+  // meeting: a block takes 0.265 us, block-scaled 0.36. B200, us, 8 / 16 (with splits through global memory): 16 x 512 x 14336
+  // 9.7 / 7.5 (7.4), 128 x 512 x 14336 14.9 / 11.3 (22), 1 x 256 x 8192 6.5 / 4.8 (5.5), 16 x 128 x 4096 4.7 / 4.1 (5.6); not
+  // worth it: 16 x 768 x 4096 4.95 / 5.42, 16 x 1280 x 8192 7.95 / 8.15. One or two tiles of K beyond 14336 would still be
+  // faster in 37 to 128 splits (16 x 256 x 28672 10.1 us, through memory 7.6), whose scratch two streams would share.
   const int tiles = grid.x * grid.y;
-  for (int want = (int)grid.z < kMaxCluster ? grid.z : kMaxCluster; want >= 2; --want) {
+  auto take = [&](auto kernel, int want) {
     const int per = (a.kblocks + want - 1) / want, splits = (a.kblocks + per - 1) / per;
-    if (splits < 2) break;
-    if (tiles > resident_clusters(kern, L::kTotal, splits)) continue;
+    if (splits < 2 || tiles > resident_clusters(kernel, L::kTotal, splits)) return false;
     a.cluster = 1;
     a.kblocks_per_split = per;
     grid.z = splits;
-    break;
+    return true;
+  };
+  const int asked = grid.z, per_eight = (a.kblocks + 7) / 8;
+  if constexpr (kWide) {
+    for (int want = asked < kMaxCluster ? asked : kMaxCluster; want > 8 && !a.cluster; --want) {
+      const double spared_us = (per_eight - (a.kblocks + want - 1) / want) * (kScaled ? 0.36 : 0.265);
+      if (spared_us < (kScaled || tiles <= 4 ? 1.0 : 1.3)) break;
+      auto wide = gemm_tn_kernel<kBN, kStages, kFp8, kScaled, kMaxCluster>;
+      err = reserve_dynamic_smem(wide, L::kTotal);
+      if (!err.empty()) return err;
+      if (take(wide, want)) kern = wide;
+    }
   }
+  for (int want = asked < 8 ? asked : 8; want >= 2 && !a.cluster; --want) take(kern, want);
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
   cfg.blockDim = dim3(kThreads);
@@ -508,14 +528,14 @@ std::string launch_bn(int bn, const CUtensorMap& mx, const CUtensorMap& my, cons
     }
   }
   switch (bn) {
-    case 16: return launch<16, 10, kFp8, kScaled>(mx, my, a, grid, s);
-    case 32: return launch<32, 8, kFp8, kScaled>(mx, my, a, grid, s);
-    case 64: return launch<64, 8, kFp8, kScaled>(mx, my, a, grid, s);
+    case 16: return launch<16, 10, kFp8, kScaled, true>(mx, my, a, grid, s);
+    case 32: return launch<32, 8, kFp8, kScaled, true>(mx, my, a, grid, s);
+    case 64: return launch<64, 8, kFp8, kScaled, true>(mx, my, a, grid, s);
     case 128:
-      if constexpr (!kScaled) return launch<128, 6, kFp8, kScaled>(mx, my, a, grid, s);
+      if constexpr (!kScaled) return launch<128, 6, kFp8, kScaled, true>(mx, my, a, grid, s);
       break;
     case 256:
-      if constexpr (!kScaled) return launch<256, 4, kFp8, kScaled>(mx, my, a, grid, s);
+      if constexpr (!kScaled) return launch<256, 4, kFp8, kScaled, true>(mx, my, a, grid, s);
       break;
   }
   return "unsupported tile width";
