@@ -62,3 +62,27 @@ def test_float64_inputs_give_the_fp32_result_as_doubles():
     want = (x + r)
     want = want * torch.rsqrt(want.pow(2).mean(-1, keepdim=True) + 1e-6) * w
     assert (norm - want).abs().max().item() <= 1e-4
+
+
+@pytest.mark.parametrize("tokens,hidden", [(700, 4608), (1000, 5120), (500, 5632), (450, 8192), (600, 4096), (3100, 4096), (5000, 2560)])
+@pytest.mark.parametrize("mode", [OUT_SAME, OUT_FP8_TOKEN, OUT_FP8_BLOCK128])
+def test_fp32_rows_ahead_and_not(tokens, hidden, mode):
+    """fp32 rows of two and four vectors per thread, on either side of the lines where the next row is requested ahead, with
+    more rows than blocks."""
+    g = torch.Generator(device="cuda").manual_seed(tokens)
+    x, r = (torch.randn(tokens, hidden, device="cuda", generator=g) for _ in range(2))
+    w = 1 + 0.1 * torch.randn(hidden, device="cuda", generator=g)
+    out, res, scales = tdx.fused_allreduce_rms(x, r, w, 1e-6, out_mode=mode)
+    want = x.double() + r.double()
+    assert torch.equal(res, x + r)
+    want = want * torch.rsqrt(want.square().mean(-1, keepdim=True) + 1e-6) * w.double()
+    if mode == OUT_SAME:
+        # a sum of `hidden` squares in fp32 (a few 2^-24 each, spread over a tree), a reciprocal square root, three products
+        assert (out.double() - want).abs().max() <= want.abs().max() * 2.0 ** -20
+    else:
+        cols = hidden if mode == OUT_FP8_TOKEN else 128
+        amax = want.view(tokens, hidden // cols, cols).abs().amax(-1)
+        assert torch.allclose(scales.double(), amax / 448.0, rtol=2.0 ** -20)
+        back = out.double().view(tokens, hidden // cols, cols) * scales.double()[..., None]
+        # half an e4m3 step: 2^-4 of the value, or half the smallest subnormal (2^-10) of the scale
+        assert ((back - want.view_as(back)).abs() <= want.view_as(back).abs() * 2.0 ** -4 * 1.01 + scales.double()[..., None] * 2.0 ** -10).all()

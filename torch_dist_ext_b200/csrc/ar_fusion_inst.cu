@@ -62,7 +62,12 @@ const void* by_n(int n, int vpt, int out) {
 }
 const void* select(const LaunchPlan& plan, int out) {
   switch (plan.algo) {
-    case kAlgoLocal: return by_vpt<kAlgoLocal, 1>(plan.vpt, out);
+    case kAlgoLocal:
+      // 0: without the request ahead, which ar_fusion_launch.cpp plans for fp32 rows of two or four vectors per thread only
+      if constexpr (TDX_INST_DTYPE == 0) {
+        if (plan.n_tmpl == 0) return plan.vpt == 4 ? by_out<kAlgoLocal, 0, 4>(out) : by_out<kAlgoLocal, 0, 2>(out);
+      }
+      return by_vpt<kAlgoLocal, 1>(plan.vpt, out);
     case kAlgoOneShotLamport: return by_n<kAlgoOneShotLamport>(plan.n_tmpl, plan.vpt, out);
     case kAlgoTwoShotLamport: return by_n<kAlgoTwoShotLamport>(plan.n_tmpl, plan.vpt, out);
     case kAlgoTwoShotBarrier: return by_n<kAlgoTwoShotBarrier>(plan.n_tmpl, plan.vpt, out);

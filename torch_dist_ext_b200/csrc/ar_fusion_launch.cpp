@@ -111,6 +111,19 @@ std::string fmt(const char* f, long long a = 0, long long b = 0, long long c = 0
   return buf;
 }
 
+// Whether the single-rank kernel requests a row's vectors one row ahead. The vectors in flight take registers, which fp32 rows
+// pay for with resident blocks: 320 threads of four vectors each, one block per SM where there were three. B200, fp32, us,
+// not ahead / ahead: 8192 x 5120 to e4m3 89.5 / 126, 8192 x 4608 the same; rows of 352 threads and more have two
+// blocks or one, and gain (8192 x 6144 to 1 x 128 blocks 150 / 133) but for per-token scales (133 / 138). Rows of two vectors
+// per thread gain as well (8192 x 4096 to 1 x 128 blocks 77 / 71), except that fp32 output of a message beyond the L2 is faster
+// with the three blocks (8192 x 4096 83.6 / 90.6; 2048 x 4096 the other way, 0.98). 16-bit rows always gain (8192 x 7168 114 / 67,
+// 8192 x 10240 143 / 113).
+bool requests_ahead(const ArParams& p, const LaunchPlan& pl, uint64_t msg_bytes) {
+  if (p.dtype != kF32) return true;
+  if (pl.vpt == 4) return pl.threads > 320 && p.out_mode != kOutFp8Token;
+  return pl.vpt == 1 || p.out_mode != kOutSame || msg_bytes <= (48u << 20);
+}
+
 }  // namespace
 
 std::string plan_allreduce(const ArParams& p, int emu_ranks, LaunchPlan* plan) {
@@ -202,7 +215,7 @@ std::string plan_allreduce(const ArParams& p, int emu_ranks, LaunchPlan* plan) {
     }
   }
   pl.algo = algo;
-  pl.n_tmpl = (n == 1) ? 1 : (n == 2 || n == 4 || n == 8) ? n : 0;
+  pl.n_tmpl = (n == 1) ? int(requests_ahead(p, pl, msg_bytes)) : (n == 2 || n == 4 || n == 8) ? n : 0;
 
   // grid: one block per row (or row group), capped by what is co-resident
   // Work items that set the grid: rows, except on the flag-synchronised two-shot paths where block b

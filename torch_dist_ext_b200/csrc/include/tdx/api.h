@@ -16,7 +16,7 @@ namespace tdx {
 
 struct LaunchPlan {
   int algo;      // Algo actually used
-  int n_tmpl;    // rank-count template argument (0 = runtime loop)
+  int n_tmpl;    // rank-count template argument (0 = runtime loop); one rank: whether rows are requested ahead
   int vpt;       // 16-byte vectors per thread
   int threads;
   int grid;      // blocks per rank

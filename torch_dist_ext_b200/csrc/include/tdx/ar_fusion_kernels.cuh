@@ -245,9 +245,9 @@ __device__ __forceinline__ uint4 poll_vec(const char* addr, Waiter& w, const ArP
 
 // ---- local (single rank): residual add + RMSNorm (+ quant) --------------------------------
 
-// Bound by memory. A block walks several rows of a large message, and the vectors of its next row are requested before
-// the block-wide reduction of the current one, so that loads are in flight while the block meets at the barriers.
-template <typename T, int kVpt, int kOut>
+// Bound by memory. A block walks several rows of a large message, and (kAhead) the vectors of its next row are requested
+// before the block-wide reduction of the current one, so that loads are in flight while the block meets at the barriers.
+template <typename T, int kVpt, int kOut, bool kAhead>
 __device__ __forceinline__ void local_body(const ArParams& p) {
   constexpr int kVec = VecTraits<T>::kVec;
   __shared__ float red[4][32];
@@ -261,10 +261,11 @@ __device__ __forceinline__ void local_body(const ArParams& p) {
     }
     request_residual<T, kVpt>(p, rv, row, res);
   };
-  if ((int)blockIdx.x < p.tokens) request(blockIdx.x);
+  if (kAhead && (int)blockIdx.x < p.tokens) request(blockIdx.x);
   load_gamma<T, kVpt>(p, rv, gamma);
   int parity = 0;
   for (int row = blockIdx.x; row < p.tokens; row += gridDim.x, parity ^= 1) {
+    if (!kAhead) request(row);
     float x[kVpt][kVec];
 #pragma unroll
     for (int v = 0; v < kVpt; ++v) {
@@ -278,7 +279,7 @@ __device__ __forceinline__ void local_body(const ArParams& p) {
         for (int i = 0; i < kVec; ++i) x[v][i] = 0.f;
       }
     }
-    if (row + (int)gridDim.x < p.tokens) request(row + gridDim.x);
+    if (kAhead && row + (int)gridDim.x < p.tokens) request(row + gridDim.x);
     float rstd, sc;
     finish_row<T, kVpt, kOut>(p, rv, row, x, gamma, red, parity, rstd, sc);
   }
@@ -896,7 +897,7 @@ __device__ __forceinline__ void nvls_twoshot_body(const ArParams& p) {
 
 template <typename T, int kAlgo, int kN, int kVpt, int kOut>
 __device__ __forceinline__ void ar_dispatch_body(const ArParams& p) {
-  if constexpr (kAlgo == kAlgoLocal) local_body<T, kVpt, kOut>(p);
+  if constexpr (kAlgo == kAlgoLocal) local_body<T, kVpt, kOut, kN == 1>(p);
   else if constexpr (kAlgo == kAlgoOneShotLamport) oneshot_lamport_body<T, kN, kVpt, kOut>(p);
   else if constexpr (kAlgo == kAlgoTwoShotLamport) twoshot_lamport_body<T, kN, kVpt, kOut>(p);
   else if constexpr (kAlgo == kAlgoTwoShotBarrier) twoshot_barrier_body<T, kN, kVpt, kOut>(p);
@@ -911,13 +912,14 @@ __device__ __forceinline__ void ar_dispatch_body(const ArParams& p) {
 template <int kVpt>
 constexpr int kMaxThreadsFor = (kVpt == 1) ? 1024 : 512;
 
-// The single-rank kernel of two vectors per thread is held to 64 registers, so that an SM has two blocks: with 79 it had one,
-// and the block's loads of one row (28 KB at 7168 x bf16) were all that was in flight (8192 x 7168 to e4m3: 82 us with one, 70 with two, 6.0 TB/s).
-template <int kAlgo, int kVpt>
-constexpr int kMinBlocksFor = (kAlgo == kAlgoLocal && kVpt == 2) ? 2 : 1;
+// The single-rank kernel of two vectors per thread that requests the next row ahead (kN: 1 does, 0 does not) is held to 64
+// registers, so that an SM has two blocks: with 79 it had one, and the block's loads of one row (28 KB at 7168 x bf16) were all that was in flight (8192 x 7168 to e4m3: 82 us with one, 67 with two, 6.3 TB/s).
+// The fp16 kernels to e4m3 spill 3 and 7 registers for it (8192 x 7168: 114 us before, 65 and 67 with it, as bf16).
+template <int kAlgo, int kN, int kVpt>
+constexpr int kMinBlocksFor = (kAlgo == kAlgoLocal && kN == 1 && kVpt == 2) ? 2 : 1;
 
 template <typename T, int kAlgo, int kN, int kVpt, int kOut>
-__global__ void __launch_bounds__(kMaxThreadsFor<kVpt>, kMinBlocksFor<kAlgo, kVpt>) ar_fused_kernel(const __grid_constant__ ArParams p) {
+__global__ void __launch_bounds__(kMaxThreadsFor<kVpt>, kMinBlocksFor<kAlgo, kN, kVpt>) ar_fused_kernel(const __grid_constant__ ArParams p) {
   // Launched with programmatic stream serialisation (ar_fusion_inst.cu), the blocks of this kernel are scheduled
   // while the previous kernel of the stream still runs, and wait here until it has completed and its memory
   // is visible; the next kernel may then be scheduled in the same way. A plain launch passes straight through.
