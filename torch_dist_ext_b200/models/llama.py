@@ -49,18 +49,21 @@ _FUSED_FP8 = os.environ.get("TDX_FUSED_FP8", "0") != "0"
 _FUSED_BF16 = os.environ.get("TDX_FUSED_BF16", "0") != "0"
 # Decode steps in "ar" mode run the rotary embedding + KV append inside the qkv GEMM and (bf16 weights) silu(gate) * up
 # inside the gate_up GEMM: both are done by the CTAs of the cluster in which the GEMM's K splits meet, and each saves a launch
-# of the layer's latency chain. Measured on one B200 at the per-rank shapes of TP=8 (CUDA-graph replay of four Llama-3-8B
-# layers and the lm-head, 2048 positions, fused against separate kernels): 186 against 197 us per step at batch 1, 200 / 212
-# at 16, 217 / 228 at 17, 257 / 263 at 33, 280 / 284 at 64, so bf16 weights use them up to 64 tokens where the GEMM has at
-# most 74 tiles, as many as a B200 holds clusters of two; with more tiles one CTA finishes each alone, and 16 tokens is the
-# limit. The block-scaled e4m3 kernel that has the rotary epilogue is the faster one for a few tokens only, hence 16 there too.
-# TDX_FUSED_EPILOGUE_TOKENS sets one limit for all, TDX_FUSED_EPILOGUES=0 keeps the separate kernels everywhere.
+# of the layer's latency chain. With bf16 weights that is faster up to 64 tokens where the GEMM has at most 74 tiles, as many
+# as a B200 holds clusters of two; with more tiles one CTA finishes each alone, which is slower even at one token. Measured on
+# one B200 at the per-rank shapes of tensor-parallel decoding (CUDA-graph replay of four layers and the lm-head, 512
+# positions, us per step, separate kernels / fused, tiles of qkv and gate_up): Llama-3-8B TP=8 (6, 28) batch 1 189 / 178, 17
+# 221 / 206, 64 255 / 245; TP=4 (12, 56) 252 / 238, 282 / 268, 325 / 313; TP=2 (24, 112) 354 / 370, 392 / 407, 452 / 473; TP=1
+# (48, 224) 577 / 613, 617 / 675, 743 / 812; the 70B shape with bf16 weights TP=8 (10, 56) 336 / 323, 378 / 361, 428 / 414, TP=4
+# (20, 112) 506 / 515, 544 / 560, 598 / 622. The block-scaled e4m3 kernel that has the rotary epilogue is the faster one for a few
+# tokens only, hence 16 there. TDX_FUSED_EPILOGUE_TOKENS sets one limit for all, TDX_FUSED_EPILOGUES=0 keeps the separate
+# kernels everywhere.
 _FUSED_EPILOGUES = os.environ.get("TDX_FUSED_EPILOGUES", "1") != "0"
 _FUSED_EPILOGUE_TOKENS = os.environ.get("TDX_FUSED_EPILOGUE_TOKENS")
 
 
 def _epilogue_fits(tokens: int, tiles: int, fp8: bool) -> bool:
-    limit = int(_FUSED_EPILOGUE_TOKENS) if _FUSED_EPILOGUE_TOKENS else 64 if tiles <= 74 and not fp8 else 16
+    limit = int(_FUSED_EPILOGUE_TOKENS) if _FUSED_EPILOGUE_TOKENS else 16 if fp8 else 64 if tiles <= 74 else 0
     return _FUSED_EPILOGUES and tokens <= limit
 
 
