@@ -372,16 +372,13 @@ gemm_scaled_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
       float acc[kHalf];
 #pragma unroll
       for (int j = 0; j < kHalf; ++j) acc[j] = 0.f;
-      const uint32_t end = it + (uint32_t)(w.kb1 - w.kb0);
-      for (; ok && it != end; ++it) {
+      const uint32_t end = ok ? it + (uint32_t)(w.kb1 - w.kb0) : it;
+      for (; it != end; ++it) {
         // the warp leaves the loop as a whole (tcgen05.ld is a warp-wide instruction)
         if (it % kGroup == 0)
           ok = tc::mbar_wait_warp(&scale_full[(it / kGroup) % kGroups], (it / (kGroup * kGroups)) & 1, kWaitLimit, abort_flag);
         if (!ready) ok = ok && tc::mbar_wait_warp(&part_full[half * 2 + (it & 1)], (it >> 1) & 1, kWaitLimit, abort_flag);
-        if (!ok) {
-          if (lane == 0) fail();
-          break;
-        }
+        if (!ok) break;
         tc::fence_after_thread_sync();
         const float sc = my_scales[(it % (kGroup * kGroups)) * kScalePitch];
         if (live) {
@@ -411,6 +408,7 @@ gemm_scaled_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
           if (tc::elect_one()) tc::mbar_arrive(&scale_empty[(it / kGroup) % kGroups]);
         }
       }
+      if (!ok && lane == 0) fail();
       __syncwarp();
       if (kCtas == 1 && a.parts > 1) {
         // the meeting in the cluster, below: the sums go to shared memory once every MMA of this CTA has read its stages
