@@ -185,3 +185,17 @@ def test_remembered_splits_follow_the_value_of_max_len(monkeypatch):
         attention.decode_attention(q, cache, cache, None, length)
         attention.decode_attention(q, cache, cache, None, n)
     assert seen[0] == seen[1] == 1 and seen[2] == seen[3] > 8
+
+
+@pytest.mark.parametrize("m,n,k,few", [
+    (1, 8192, 1024, True), (16, 8320, 1024, False), (17, 5120, 8192, True), (32, 5248, 8192, False),
+    (33, 2560, 8192, True), (64, 2688, 8192, False), (65, 1280, 4096, True), (128, 1408, 4096, False),
+    (129, 1280, 1024, True), (129, 1792, 1024, False), (256, 4736, 4096, True), (257, 4736, 4096, False),
+    (192, 2688, 8192, True), (192, 2816, 8192, False), (512, 640, 14336, True), (512, 768, 14336, False),
+])
+def test_few_tiles_of_a_block_scaled_product(m, n, k, few):
+    assert gemm._few_scaled_tiles(m, n, k) == few
+    if few and m > 128:      # its K pieces are resident, or it has none: they never meet in the scratch of the device
+        tiles = -(-n // 128) * -(-m // 64)
+        _, bn, splits = gemm.plan(m, n, k, 1, scaled=True)
+        assert bn == 64 and (tiles <= SMS // 2 or splits == 1)

@@ -146,6 +146,22 @@ def linear(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None,
     return out
 
 
+def _few_scaled_tiles(m: int, n: int, k: int) -> bool:
+    """Whether a block-scaled product runs on the swapped kernel (128 weight rows x up to 64 tokens per tile, K in up to
+    sixteen pieces) and not on that of gemm_scaled.cu (256 weight rows x 128 or 256 tokens): where it has so few of its small
+    tiles that all of them, and their pieces, are resident at a time, while the large ones would leave most multiprocessors
+    idle. The line is where the two meet over 1 to 768 tokens, 128 to 8192 rows and K of 1024 to 16384 (B200, us, swapped /
+    the other: 16 x 1280 x 8192 6.5 / 10.3, 64 x 2560 x 8192 12.1 / 13.1, 64 x 3840 x 8192 15.2 / 14.1, 129 x 1280 x 8192 14.1 /
+    27.0, 192 x 2560 x 8192 24.2 / 27.6, 192 x 3840 x 8192 37.7 / 28.2, 192 x 5120 x 4096 21.7 / 23.4, 256 x 5120 x 4096 42.0 /
+    23.7, 512 x 1024 x 8192 24.3 / 27.8, 512 x 1024 x 16384 40.4 / 33.1)."""
+    tiles = -(-n // 128) * -(-m // _pick_bn(m, 64))
+    if m <= 16:
+        return tiles <= 64
+    if m <= 128:
+        return tiles <= (40 if m <= 32 else 20)
+    return tiles <= (40 if k <= 1024 else _SM_COUNT if k <= 4096 else 64 if k <= 8192 else 40)
+
+
 @traced("tdx.linear_fp8_blockscaled")
 def linear_fp8_blockscaled(a_q: torch.Tensor, a_scale: torch.Tensor, w_q: torch.Tensor, w_scale: torch.Tensor,
                            out: Optional[torch.Tensor] = None, *, out_dtype=torch.bfloat16,
@@ -154,12 +170,7 @@ def linear_fp8_blockscaled(a_q: torch.Tensor, a_scale: torch.Tensor, w_q: torch.
     m, k = a_q.shape
     n = w_q.shape[0]
     ws, counters, status = _workspace(a_q.device)
-    # The kernel of gemm_scaled.cu (activations on the 128-row side, 256 weight rows per tile), except for a few tokens of
-    # a weight with so few rows that its tiles, in up to eight pieces each, leave most multiprocessors idle: there the
-    # swapped kernel cuts finer. B200, us per call, swapped / this one: 5120 x 8192 at 16 tokens 15.1 / 16.4, 1280 x 8192 at
-    # 32 tokens 9.2 / 10.5; 7168 x 8192 at 16 tokens 19.4 / 17.8, 1280 x 8192 at 64 tokens 13.1 / 11.6, 8192 x 1024 at 1 token
-    # 6.5 / 6.4, 28672 x 8192 at 64 tokens 81 / 47.
-    few = m <= 32 and n <= 20 * 256 and k > 2048
+    few = _few_scaled_tiles(m, n, k)
     if out_dtype is None:
         out_dtype = torch.get_default_dtype()      # as torch.empty takes it
     if splits is None and not few and out is None:
