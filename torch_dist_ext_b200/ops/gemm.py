@@ -111,9 +111,10 @@ def linear(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None,
             dt = out_dtype or (torch.bfloat16 if a.element_size() == 1 else a.dtype)
             out = torch.empty(m, n, dtype=dt, device=a.device)
         ws = counters = None
-        floats, words = _pair_tail(m, n, k, a.element_size(), a.device)
-        if floats:                                            # K-split of a partly filled last round
-            ws, counters = _pair_scratch(a.device, floats), torch.zeros(words, dtype=torch.int32, device=a.device)
+        if -(-m // 256) * -(-n // 256) > _SM_COUNT // 2:      # a second round, perhaps partly filled: K-split of its tiles
+            floats, words = _pair_tail(m, n, k, a.element_size(), a.device)
+            if floats:
+                ws, counters = _pair_scratch(a.device, floats), torch.zeros(words, dtype=torch.int32, device=a.device)
         _lib.ops().gemm_tn_pair(a, w, out, n, 1, _workspace(a.device)[2], ws, counters)
         return out
     if (use_persistent or (use_pair and persistent is None and _PERSIST_DEFAULT)) and m > 128 and n >= 256 and not swap \
