@@ -8,10 +8,13 @@ models replay the role programs of
 
  * the persistent GEMM (csrc/gemm_persist.cu): operand ring that runs across tile boundaries,
    two accumulator buffers handed between the MMA thread and the epilogue warps;
- * the tensor-core decode attention kernel (csrc/attention_decode_tc.cu): K/V ring, double-buffered
-   scores, one probability tile, one P*V buffer;
+ * the tensor-core decode attention kernel (csrc/attention_decode_tc.cu): rings of K and of V chunks, double-buffered
+   scores, two probability tiles, one P*V buffer;
  * the prompt attention kernel (csrc/attention_prefill_tc.cu): separate K and V rings, two softmax groups on
-   alternate chunks, each with its score buffer, probability tile and accumulator in tensor memory;
+   alternate chunks, each with its score buffer, two probability tiles and accumulator in tensor memory;
+ * the block-scaled GEMM (csrc/gemm_scaled.cu): two column halves with an MMA warp and two partial buffers each behind one
+   operand ring, a ring of scale products handed over in groups, and a meeting that every promoting warp attends also
+   when its pipeline has been given up;
  * the CTA-pair GEMM (csrc/gemm_pair.cu): two producers crediting the leader's transaction-counting
    barriers, stages released in both CTAs by the leader's MMA thread, a persistent tile loop with two
    accumulator buffers that the epilogue warps of BOTH CTAs hand back to the leader
@@ -157,20 +160,20 @@ def test_persistent_gemm_pipeline(ntiles, nkb, stages):
 
 
 # ---- tensor-core decode attention (csrc/attention_decode_tc.cu) ----------------------------------------
-# K/V ring, double-buffered scores, TWO probability tiles and barrier pairs (p_full[c & 1], o_full[c & 1]) so that
+# K and V rings of their own (a K stage is free once its scores are complete), double-buffered scores, TWO probability tiles and barrier pairs (p_full[c & 1], o_full[c & 1]) so that
 # the softmax of chunk i runs while P*V of chunk i - 1 is still in flight; O accumulates in tensor memory and is
 # only touched by the softmax threads at the (rare) rescale, behind a wait for P*V of chunk i - 1.
 
-def attention(nchunks, stages, rng):
-    kv_full = [MBar(1) for _ in range(stages)]
-    kv_free = [MBar(1) for _ in range(stages)]
+def attention(nchunks, stages_k, stages_v, rng):
+    full = [[MBar(1) for _ in range(n)] for n in (stages_k, stages_v)]       # [K, V]
+    free = [[MBar(1) for _ in range(n)] for n in (stages_k, stages_v)]
     s_full = [MBar(1) for _ in range(2)]
     n_sm = 2                                             # stands for the 128 softmax threads
     s_free = [MBar(n_sm) for _ in range(2)]
     p_full = [MBar(n_sm) for _ in range(2)]
     o_full = [MBar(1) for _ in range(2)]
-    kv = [None] * stages
-    kv_reads_pending = [0] * stages
+    ring = [[None] * n for n in (stages_k, stages_v)]
+    reads_pending = [[0] * n for n in (stages_k, stages_v)]
     s_buf = [None, None]
     s_readers = [0, 0]
     p_tile = [{"chunk": None, "reads_pending": 0} for _ in range(2)]
@@ -178,57 +181,63 @@ def attention(nchunks, stages, rng):
     outputs = [[] for _ in range(n_sm)]
     events = {"tma": [], "mma_s": [], "mma_pv": []}      # each issuer's MMAs complete in its issue order
 
-    def copy(c):
-        s = c % stages
-        assert kv_reads_pending[s] == 0, "K/V stage overwritten while an MMA still reads it"
+    def copy(which, c):
+        s = c % len(ring[which])
+        assert reads_pending[which][s] == 0, "stage overwritten while an MMA still reads it"
 
         def land():
-            kv[s] = c
-            kv_full[s].arrive()
+            ring[which][s] = c
+            full[which][s].arrive()
         events["tma"].append(land)
 
     def issue_scores(c):
-        s = c % stages
-        assert kv[s] == c, f"scores of chunk {c} read stage holding {kv[s]}"
+        s = c % stages_k
+        assert ring[0][s] == c, f"scores of chunk {c} read stage holding {ring[0][s]}"
         assert s_readers[c & 1] == 0, "score buffer overwritten while the softmax warps read it"
-        kv_reads_pending[s] += 1
+        reads_pending[0][s] += 1
 
         def retire():
             s_buf[c & 1] = c
-            kv_reads_pending[s] -= 1
+            reads_pending[0][s] -= 1
             s_full[c & 1].arrive()
+            free[0][s].arrive()
         events["mma_s"].append(retire)
 
     def issue_pv(c):
-        s = c % stages
-        assert kv[s] == c and p_tile[c & 1]["chunk"] == c, f"P*V of chunk {c}: P tile holds {p_tile[c & 1]['chunk']}"
+        s = c % stages_v
+        assert ring[1][s] == c and p_tile[c & 1]["chunk"] == c, f"P*V of chunk {c}: P tile holds {p_tile[c & 1]['chunk']}"
         assert o_acc["rescaling"] == 0, "P*V issued while a softmax thread rescales O"
-        kv_reads_pending[s] += 1
+        reads_pending[1][s] += 1
         p_tile[c & 1]["reads_pending"] += 1
         o_acc["mma_pending"] += 1
 
         def retire():
             o_acc["chunks"].append(c)
             o_acc["mma_pending"] -= 1
-            kv_reads_pending[s] -= 1
+            reads_pending[1][s] -= 1
             p_tile[c & 1]["reads_pending"] -= 1
             o_full[c & 1].arrive()
-            kv_free[s].arrive()
+            free[1][s].arrive()
         events["mma_pv"].append(retire)
 
-    # three issuing threads: copies, score MMAs, P*V MMAs - each with its own chain of waits
+    # three issuing warps: copies, score MMAs, P*V MMAs - each with its own chain of waits
     def loader():
-        for c in range(min(nchunks, stages)):
-            copy(c)
-        for i in range(nchunks):
-            if i + stages < nchunks:
-                yield from wait(kv_free[i % stages], (i // stages) & 1)
-                copy(i + stages)
+        lag = stages_k - stages_v                        # K runs so many chunks ahead of V
+        for j in range(nchunks + lag):
+            if j < nchunks:
+                if j >= stages_k:
+                    yield from wait(free[0][j % stages_k], (j // stages_k - 1) & 1)
+                copy(0, j)
+            c = j - lag
+            if c >= 0:
+                if c >= stages_v:
+                    yield from wait(free[1][c % stages_v], (c // stages_v - 1) & 1)
+                copy(1, c)
             yield ("step",)
 
     def score_issuer():
         for c in range(nchunks):
-            yield from wait(kv_full[c % stages], (c // stages) & 1)
+            yield from wait(full[0][c % stages_k], (c // stages_k) & 1)
             if c >= 2:
                 yield from wait(s_free[c & 1], ((c >> 1) - 1) & 1)
             issue_scores(c)
@@ -237,7 +246,7 @@ def attention(nchunks, stages, rng):
     def pv_issuer():
         for c in range(nchunks):
             yield from wait(p_full[c & 1], (c >> 1) & 1)
-            yield from wait(kv_full[c % stages], (c // stages) & 1)
+            yield from wait(full[1][c % stages_v], (c // stages_v) & 1)
             issue_pv(c)
             yield ("step",)
 
@@ -270,10 +279,11 @@ def attention(nchunks, stages, rng):
     assert all(o == list(range(nchunks)) for o in outputs)
 
 
-@pytest.mark.parametrize("nchunks,stages", [(1, 3), (2, 3), (3, 3), (4, 3), (9, 3), (16, 3), (5, 2)])
+@pytest.mark.parametrize("nchunks", [1, 2, 3, 4, 5, 9, 16])
+@pytest.mark.parametrize("stages", [(3, 3), (2, 1)])          # one CTA to an SM, two
 def test_attention_pipeline(nchunks, stages):
     for seed in range(60):
-        attention(nchunks, stages, random.Random(seed))
+        attention(nchunks, *stages, random.Random(seed))
 
 
 def test_the_checker_sees_a_wrong_parity():
@@ -686,3 +696,136 @@ def test_push_epilogue_one_buffer_would_race():
         except AssertionError:
             hits += 1
     assert hits > 0
+
+
+# ---- block-scaled GEMM ---------------------------------------------------------------------------------------------
+# One CTA (the pair differs in who credits the operand barriers, which the pair GEMM's model covers): a producer, an MMA
+# issuer per column half, a warp that stages scale products in groups of four K blocks, promoting warps per half. `work` are
+# the K blocks of the tiles of this worker, the last of them a piece of a tile if `meets`. `gives_up`: (role, wait) after which
+# a role's wait runs out; it raises the flag that ends every other wait (at once, or later: a wait that has passed passes).
+# With `attends` a promoting warp that has given up still comes to the meeting.
+
+def scaled_gemm(work, meets, rng, gives_up=None, attends=True):
+    stages, group, groups, warps = 4, 4, 4, 2                # `warps` stands for the four promoting warps of a half
+    blocks = [(t, kb) for t, n in enumerate(work) for kb in range(n)]
+    full, empty = [MBar(1) for _ in range(stages)], [MBar(2) for _ in range(stages)]
+    part_full = [[MBar(1) for _ in range(2)] for _ in range(2)]
+    part_empty = [[MBar(warps) for _ in range(2)] for _ in range(2)]
+    scale_full, scale_empty = [MBar(1) for _ in range(groups)], [MBar(2 * warps) for _ in range(groups)]
+    meeting = MBar(2 * warps)
+    ring, ring_reads = [None] * stages, [0] * stages
+    part, part_readers = [[None] * 2 for _ in range(2)], [[0] * 2 for _ in range(2)]
+    scales = [None] * (group * groups)
+    sums = {}
+    events = {"tma": [], "mma0": [], "mma1": []}
+    flag = {"abort": False, "waits": {}}
+
+    def bounded(role, bar, parity):
+        """True when the phase has completed; False when the wait was given up."""
+        flag["waits"][role] = flag["waits"].get(role, -1) + 1
+        if gives_up == (role, flag["waits"][role]):
+            flag["abort"] = True
+            return False
+        while not bar.ready(parity):
+            if flag["abort"]:
+                return False
+            yield ("step",)
+        return True
+
+    def producer():
+        for it, what in enumerate(blocks):
+            s = it % stages
+            if it >= stages and not (yield from bounded("producer", empty[s], ((it // stages) - 1) & 1)):
+                return
+            assert ring_reads[s] == 0, "stage overwritten while an MMA still reads it"
+
+            def land(s=s, what=what):
+                ring[s] = what
+                full[s].arrive()
+            events["tma"].append(land)
+            yield ("step",)
+
+    def issuer(half):
+        for it, what in enumerate(blocks):
+            s, buf = it % stages, it & 1
+            if not (yield from bounded(f"mma{half}", full[s], (it // stages) & 1)):
+                return
+            if it >= 2 and not (yield from bounded(f"mma{half}", part_empty[half][buf], ((it >> 1) - 1) & 1)):
+                return
+            assert ring[s] == what and part_readers[half][buf] == 0
+            ring_reads[s] += 1
+
+            def retire(s=s, buf=buf, what=what):
+                part[half][buf] = what
+                ring_reads[s] -= 1
+                part_full[half][buf].arrive()
+                empty[s].arrive()
+            events[f"mma{half}"].append(retire)
+            yield ("step",)
+
+    def scaler():
+        for i0 in range(0, len(blocks), group):
+            g = i0 // group
+            if g >= groups and not (yield from bounded("scaler", scale_empty[g % groups], ((g // groups) - 1) & 1)):
+                return
+            for k in range(group):
+                scales[(i0 + k) % (group * groups)] = blocks[min(i0 + k, len(blocks) - 1)]
+            scale_full[g % groups].arrive()
+            yield ("step",)
+
+    def promoter(half, who):
+        it, lost = 0, False
+        for t, n in enumerate(work):
+            acc = []
+            for _ in range(n):
+                buf, role = it & 1, f"promote{half}{who}"
+                if it % group == 0 and not (yield from bounded(role, scale_full[(it // group) % groups], (it // (group * groups)) & 1)):
+                    lost = True
+                    break
+                if not (yield from bounded(role, part_full[half][buf], (it >> 1) & 1)):
+                    lost = True
+                    break
+                part_readers[half][buf] += 1
+                yield ("step",)
+                assert part[half][buf] == blocks[it] and scales[it % (group * groups)] == blocks[it]
+                acc.append(blocks[it][1])
+                part_readers[half][buf] -= 1
+                part_empty[half][buf].arrive()
+                if it % group == group - 1:
+                    scale_empty[(it // group) % groups].arrive()
+                it += 1
+            if lost:
+                break
+            if meets and t == len(work) - 1:
+                meeting.arrive()
+                yield from wait(meeting, 0)
+            sums[half, who, t] = acc
+        if lost and attends and meets:
+            meeting.arrive()
+            yield from wait(meeting, 0)
+
+    run([producer(), issuer(0), issuer(1), scaler()] + [promoter(h, w) for h in range(2) for w in range(warps)], events, rng)
+    if gives_up is None:
+        assert all(sums[h, w, t] == list(range(n)) for h in range(2) for w in range(warps) for t, n in enumerate(work))
+    return flag["abort"]
+
+
+@pytest.mark.parametrize("work", [[1], [2], [7], [16], [64], [5, 5, 3], [16, 16, 16]])
+@pytest.mark.parametrize("meets", [False, True])
+def test_scaled_gemm_pipeline(work, meets):
+    for seed in range(25):
+        scaled_gemm(work, meets, random.Random(seed))
+
+
+@pytest.mark.parametrize("role", ["producer", "mma0", "mma1", "scaler", "promote00", "promote11"])
+def test_scaled_gemm_that_gives_up_still_ends(role):
+    gave_up = 0
+    for seed in range(150):
+        rng = random.Random(seed)
+        gave_up += scaled_gemm([9, 9, 7], True, rng, gives_up=(role, rng.randrange(30)))
+    assert gave_up > 10
+    if role == "promote11":                                     # the warps of the other half may have had their last block
+        with pytest.raises(AssertionError, match="deadlock|did not finish"):
+            for seed in range(150):
+                rng = random.Random(seed)
+                scaled_gemm([9, 9, 7], True, rng, gives_up=(role, rng.randrange(30)), attends=False)
