@@ -64,3 +64,25 @@ def test_prefill_attention_tc(s, hq, hkv):
     assert gemm.pipeline_status() == 0
     want = attention.prefill_attention_reference(q, k, v)
     assert (got.float() - want.float()).abs().max().item() <= 3e-2
+
+
+@pytest.mark.parametrize("g", [1, 2, 4, 8])
+def test_decode_attention_two_ctas_to_an_sm(g):
+    """152 (sequence, KV head) pairs on 148 SMs: two CTAs to an SM, whose rings of two K and one V chunks are passed several
+    times; sequences that end at, before and behind the edge of a chunk, and scores that make the running maximum jump."""
+    b, hkv, smax = 19, 8, 1300
+    gen = torch.Generator(device="cuda").manual_seed(g)
+    q = torch.randn(b, g * hkv, 128, device="cuda", generator=gen).to(torch.bfloat16)
+    k, v = (torch.randn(b, smax, hkv, 128, device="cuda", generator=gen) for _ in range(2))
+    k = (k * torch.linspace(0.2, 2.5, smax, device="cuda").view(1, smax, 1, 1)).to(torch.bfloat16)
+    v = v.to(torch.bfloat16)
+    lens = torch.randint(1, smax + 1, (b,), device="cuda", dtype=torch.int32, generator=gen)
+    lens[:8] = torch.tensor([smax, 1, 127, 128, 129, 256, 384, 385], dtype=torch.int32)
+    got = attention.decode_attention(q, k, v, lens, smax)
+    torch.cuda.synchronize()
+    assert gemm.pipeline_status() == 0
+    scores = torch.einsum("bhgd,bnhd->bhgn", q.double().view(b, hkv, g, 128), k.double()) / 128 ** 0.5
+    scores.masked_fill_(torch.arange(smax, device="cuda").view(1, 1, 1, -1) >= lens.view(b, 1, 1, 1), float("-inf"))
+    want = torch.einsum("bhgn,bnhd->bhgd", scores.softmax(-1), v.double()).reshape(b, g * hkv, 128)
+    # probabilities and output are rounded to bf16 (2^-9 each), the sum of the former weighs values of up to max |v|
+    assert (got.double() - want).abs().max() <= 2 * v.double().abs().max() * 2.0 ** -9

@@ -1,9 +1,10 @@
-"""Decode GEMMs whose K splits meet inside a cluster: uneven splits, ragged rows and columns, every output type and the
-pair epilogues, against 64-bit PyTorch math; and the same call with its splits meeting in global memory."""
+"""GEMMs whose K splits meet inside a cluster: uneven splits, ragged rows and columns, every output type, against 64-bit
+PyTorch math; and splits of more tiles than the device holds clusters, which meet in global memory, with the rotary and silu
+epilogues (those of a cluster are in test_gemm_epilogues_gpu.py)."""
 import pytest
 import torch
 
-from torch_dist_ext_b200.ops import gemm
+from torch_dist_ext_b200.ops import gemm, rope
 
 pytestmark = pytest.mark.gpu
 
@@ -109,3 +110,65 @@ def test_few_tiles_and_a_long_k(m, n, k, out_dtype):
         assert all(torch.equal(outs[i][0], o) for o in outs[i]), "the splits are added in a fixed order"
         bound = want[i].abs().max() * (k * 2.0 ** -22 if out_dtype == torch.float32 else 2.0 ** -8)      # as above
         assert (outs[i][0].double() - want[i]).abs().max() <= bound
+
+
+def _scratch_is_zero(device):
+    ws, counters, _ = gemm._workspace(device)
+    return float(ws.abs().max()) == 0.0 and int(counters.abs().sum()) == 0
+
+
+@pytest.mark.parametrize("m,n,k,splits", [(1, 10240, 1024, 4), (33, 10101, 512, 3), (128, 9728, 640, 5)])
+def test_splits_meet_in_memory(m, n, k, splits):
+    """More than 74 tiles, cut along K all the same: fp32 additions into scratch, and the split that arrives last finishes the
+    tile and leaves the scratch zeroed for the second call."""
+    g = torch.Generator(device="cuda").manual_seed(m + n)
+    a = torch.randn(m, k, device="cuda", generator=g).to(torch.bfloat16)
+    w = (torch.randn(n, k, device="cuda", generator=g) * 0.05).to(torch.bfloat16)
+    want = a.double() @ w.double().t()
+    for out_dtype in (torch.bfloat16, torch.float32):
+        for _ in range(2):
+            out = gemm.linear(a, w, out_dtype=out_dtype, splits=splits)
+            bound = want.abs().max() * (2.0 ** -8 if out_dtype == torch.bfloat16 else k * 2.0 ** -22)      # as above
+            assert (out.double() - want).abs().max() <= bound
+            assert _scratch_is_zero(a.device) and gemm.pipeline_status() == 0
+
+
+@pytest.mark.parametrize("m", [1, 17, 100])
+def test_rotary_epilogue_in_memory(m):
+    q_heads, kv_heads, k, seq = 64, 8, 512, 40          # 80 tiles
+    g = torch.Generator(device="cuda").manual_seed(m)
+    a = torch.randn(m, k, device="cuda", generator=g).to(torch.bfloat16)
+    w = (torch.randn((q_heads + 2 * kv_heads) * 128, k, device="cuda", generator=g) * 0.05).to(torch.bfloat16)
+    positions = torch.randint(0, seq, (m,), device="cuda", generator=g)
+    cos_sin = rope.build_cos_sin_cache(seq, 128, 5e5, "cuda")
+    want = (a.double() @ w.double().t()).view(m, -1, 128)
+    cos, sin = cos_sin[positions].double()[:, None, :64], cos_sin[positions].double()[:, None, 64:]
+    x = want[:, :q_heads + kv_heads].clone()
+    want[:, :q_heads + kv_heads] = torch.cat([x[..., :64] * cos - x[..., 64:] * sin, x[..., 64:] * cos + x[..., :64] * sin], -1)
+    bound = want.abs().max() * 2.0 ** -7                # a rounding step of bf16 of the largest value
+    rows = torch.arange(m, device="cuda")
+    for _ in range(2):
+        k_cache = torch.zeros(m + 2, seq, kv_heads, 128, dtype=torch.bfloat16, device="cuda")
+        v_cache = torch.zeros_like(k_cache)
+        out = gemm.linear_rope_kv(a, w, positions, cos_sin, k_cache, v_cache, q_heads, kv_heads)
+        assert (out.view(m, -1, 128).double() - want).abs().max() <= bound
+        assert (k_cache[rows, positions].double() - want[:, q_heads:q_heads + kv_heads]).abs().max() <= bound
+        assert (v_cache[rows, positions].double() - want[:, q_heads + kv_heads:]).abs().max() <= bound
+        k_cache[rows, positions] = 0
+        v_cache[rows, positions] = 0
+        assert not k_cache.any() and not v_cache.any()
+        assert _scratch_is_zero(a.device) and gemm.pipeline_status() == 0
+
+
+@pytest.mark.parametrize("m", [1, 17, 100])
+def test_silu_epilogue_in_memory(m):
+    ffn, k = 64 * 80, 512
+    g = torch.Generator(device="cuda").manual_seed(m)
+    a = torch.randn(m, k, device="cuda", generator=g).to(torch.bfloat16)
+    w = (torch.randn(2 * ffn, k, device="cuda", generator=g) * 0.05).to(torch.bfloat16)
+    gu = a.double() @ w.double().t()
+    want = torch.nn.functional.silu(gu[:, :ffn]) * gu[:, ffn:]
+    for _ in range(2):
+        out = gemm.linear_silu_mul(a, w)
+        assert (out.double() - want).abs().max() <= want.abs().max() * 2.0 ** -7      # as above
+        assert _scratch_is_zero(a.device) and gemm.pipeline_status() == 0

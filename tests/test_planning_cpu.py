@@ -60,6 +60,17 @@ def test_tensor_core_attention_splits_follow_the_measured_costs():
     assert pick(3, 2, 100000) > 8                                # long contexts still spread over the SMs
 
 
+def test_splits_that_merge_in_a_cluster_are_cheaper():
+    held = {2: 74, 3: 45, 4: 33, 5: 26, 6: 22, 7: 15, 8: 15}    # clusters that a B200 holds at a time
+    pick = lambda b, h, n, c: attention.pick_splits(b, h, n, ctas_per_sm=1, clusters=c)
+    assert pick(16, 1, 2048, None) == 4 and pick(16, 1, 2048, held) == 6          # 16 x 6 CTAs; eight splits would not fit
+    assert pick(64, 1, 2048, None) == 1 and pick(64, 1, 2048, held) == 2
+    assert pick(1, 1, 2000, held) == 8
+    for b, h, n in [(1, 1, 128), (7, 2, 300), (3, 8, 5000), (16, 8, 2048), (40, 1, 777), (150, 1, 2048), (2, 1, 100000)]:
+        s = pick(b, h, n, held)
+        assert s >= 1 and (s == 1 or (b * h * s <= SMS and s <= -(-n // 128)))
+
+
 def test_fused_decode_epilogues_need_the_weights_on_the_wide_side_and_a_split():
     assert gemm.fused_epilogue_fits(1, 4096) and gemm.fused_epilogue_fits(128, 4096)
     assert not gemm.fused_epilogue_fits(129, 4096)                 # the tokens take the 128-row side
