@@ -235,7 +235,7 @@ def attention_split_cases(dev, steps, out):
 
 
 def decode_epilogue_cases(dev, steps, out):
-    """The decode GEMMs whose split-K finalizer does the next kernel's work, against the two-kernel form (column
+    """The decode GEMMs that do the next kernel's work where their K splits meet, against the two-kernel form (column
     `library_us` here: this library's GEMM followed by its own RoPE + KV-append / SiLU kernel). Per-rank shapes of TP=8."""
     from torch_dist_ext_b200.ops import activation, gemm, rope
 
@@ -311,7 +311,7 @@ def main():
         elementwise_cases(dev, args.steps, out)
     if g == "attention_splits":     # decode attention over the KV split count
         attention_split_cases(dev, args.steps, out)
-    if g == "decode_epilogues":     # rotary + KV append / silu inside the GEMM's finalizer against the two-kernel form
+    if g == "decode_epilogues":     # rotary + KV append / silu inside the GEMM against the two-kernel form
         decode_epilogue_cases(dev, args.steps, out)
     path = os.path.join(common.out_dir(), f"kernels_{g}.json")
     with open(path, "w") as f:

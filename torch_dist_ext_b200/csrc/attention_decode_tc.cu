@@ -13,7 +13,7 @@
 // do the online-softmax bookkeeping and write the probabilities as a bf16 [heads, keys] tile (128-byte
 // swizzle, the B operand of the second product). O^T accumulates in tensor memory over all chunks of a
 // split; a head's column of it is rescaled there only when its running maximum has to be raised.
-// Three more warps hold one single-thread role each - the TMA copies (rings of K and of V chunks), the score MMAs, the P*V MMAs -
+// Three more warps issue - the TMA copies (rings of K and of V chunks), the score MMAs, the P*V MMAs -
 // so that none of them queues behind the others' asynchronous instructions; S^T is double-buffered in TMEM and P
 // in shared memory, so that the scores of chunk i+1 and the P*V product of chunk i-1 run while the softmax
 // warps work on chunk i.
@@ -50,7 +50,7 @@ constexpr int kD = 128;
 constexpr int kKeys = 128;                        // cache positions per chunk = MMA M of the score product
 constexpr int kNq = 16;                           // MMA N: query heads of one KV head, padded
 constexpr int kSoftmaxThreads = 128;
-constexpr int kThreads = kSoftmaxThreads + 3 * 32;   // + three single-thread roles: copies (warp 4), score MMAs (5), P*V MMAs (6)
+constexpr int kThreads = kSoftmaxThreads + 3 * 32;   // + three issuing warps: copies (4), score MMAs (5), P*V MMAs (6)
 constexpr int kMaxG = 8;
 constexpr int kHalfBytes = kKeys * 128;           // one 64-column half of a K or V chunk
 constexpr int kTileBytes = 2 * kHalfBytes;        // a K chunk or a V chunk
@@ -58,7 +58,9 @@ constexpr int kSmallTileBytes = 2 * kNq * 128;    // Q or P: two 64-wide K block
 // Rings of K and V chunks. One CTA per SM with three of each where the grid has no more CTAs than SMs: the few chunks of a
 // short split are all requested at once. More CTAs than SMs run two to an SM, with two K chunks and one V chunk each (the
 // same bytes in flight): one CTA's start (barriers, tensor memory, the first chunk's latency) and end overlap the other's
-// stream. 64 ragged sequences of up to 2048 positions, 32/8 heads: 73.2 us one to an SM, 70.4 two.
+// stream. Ragged sequences, B200, us, one to an SM / two: 64 of up to 2048 positions 64/8 heads 76.1 / 71.9, 32/8 71.2 / 68.9,
+// 16/8 68.7 / 68.3, 32/32 246 / 248; 32 of 4096 64/8 73.6 / 66.8; 64 of 512 64/8 33.3 / 26.7. (With eight heads per KV head
+// the two-CTA form spills four registers.)
 struct Deep {
   static constexpr int kStagesK = 3, kStagesV = 3, kCtasPerSm = 1;
 };

@@ -3,7 +3,8 @@
 // the key/value positions 0 .. (its last query) in chunks of 64:
 //
 //   S[q 128, keys 64] = Q[q, d] * K[keys, d]^T         both operands K-major, as TMA delivers them
-//   O[q 128, d 128]  += P[q, keys] * V[keys, d]         P written by the softmax warps (K-major over keys),
+//   O[q 128, d 128]  += P[q, keys] * V[keys, d]         P written by the softmax warps to tensor memory
+//                                                       (lane = query, two keys per column), the A operand there,
 //                                                       V read MN-major (d contiguous) straight from its TMA tile
 //
 // Two softmax warpgroups of four warps, one query row per thread in each: group g takes the chunks
@@ -20,8 +21,8 @@
 // rescaled in tensor memory - when the new maximum exceeds it by more than 2^8 (a warp-uniform
 // decision); until then the probabilities are taken against the older maximum, which changes neither
 // O / l nor the accuracy of bf16 probabilities below 256 (that rescale does wait for the group's latest
-// product). Five more warps hold one single-thread role
-// each: the TMA copies (four-stage rings for K, freed as soon as the scores are computed, and for V, freed
+// product). Five more warps issue (one elected
+// lane each): the TMA copies (four-stage rings for K, freed as soon as the scores are computed, and for V, freed
 // after P*V), the score MMAs of the even and of the odd chunks, and the P*V MMAs into O_0 and into O_1.
 //
 // Every wait is bounded; a wait that runs out records a status word and raises the CTA's abort flag,
@@ -156,11 +157,11 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   const int qb = (int)gridDim.y - 1 - (int)blockIdx.y;
   const int h = blockIdx.x;
   const int hkv = h / (a.Hq / a.Hkv);
-  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int q0 = qb * kRows;
   const int nchunks = (q0 + kRows) / kKeys;  // key positions 0 .. q0 + 127 (causal)
 #ifdef TDX_ATTN_PROBE
-  const bool probe_on = blockIdx.x == 0 && blockIdx.y == 0 && ((tid & (kSoftmaxThreads - 1)) == 0 || (warp >= kLoadWarp && lane == 0));
+  const bool probe_on = blockIdx.x == 0 && blockIdx.y == 0 && ((tid & (kSoftmaxThreads - 1)) == 0 || (warp >= kLoadWarp && (tid & 31) == 0));
 #endif
 
   if (tid == 0) {

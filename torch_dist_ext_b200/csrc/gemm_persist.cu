@@ -1,5 +1,5 @@
-// Persistent tcgen05 GEMM:  D[x, y] = sum_k X[x, k] * Y[y, k], both K-major; prompts (128 < M < 256: 128 x 256 tiles), and
-// decode-sized products with more 128-row weight tiles than SMs (128 x 16 .. 128 x 128, the weights as X).
+// Persistent tcgen05 GEMM:  D[x, y] = sum_k X[x, k] * Y[y, k], both K-major; decode-sized products with more 128-row weight
+// tiles than SMs (128 x 16 .. 128 x 128, the weights as X), and prompts (128 x 256 tiles) where CTA pairs are turned off.
 //
 // One CTA per SM walks the output tiles t = blockIdx.x, blockIdx.x + gridDim.x, ... The
 // operand ring (TMA -> 128-byte-swizzled shared memory) keeps streaming across tile boundaries, and
@@ -8,8 +8,8 @@
 // one-tile-per-CTA kernel (gemm_tcgen05.cu) pays a pipeline fill, a drain and a serial epilogue per
 // tile; here they are paid once per CTA.
 //
-//   warp 0     TMA producer (one thread): K blocks of all tiles of this CTA, back to back
-//   warp 1     tensor-memory owner and MMA issue (one thread)
+//   warp 0     TMA producer (one elected lane): K blocks of all tiles of this CTA, back to back
+//   warp 1     tensor-memory owner and MMA issue (one elected lane)
 //   warps 2-5  epilogue: TMEM lane quarter = warp % 4
 //
 // Barriers: full[s] / empty[s] per ring stage (phases counted over ALL K blocks this CTA processes),
@@ -17,7 +17,7 @@
 // Every wait is bounded; a wait that runs out records a status word, raises the CTA's abort flag and
 // all roles fall through to the common exit (copies in flight land, tensor memory is freed).
 //
-// The default for prefill-sized problems (ops/gemm.py; TDX_GEMM_PERSIST=0 turns it off), bf16 / fp16 / unscaled
+// The default for such decode-sized products (ops/gemm.py; TDX_GEMM_PERSIST=0 turns it off), bf16 / fp16 / unscaled
 // e4m3 operands, no split-K. The reference (xytpai/torch_dist_ext) has no GEMM.
 #include <cuda.h>
 #include <cuda_bf16.h>

@@ -7,9 +7,11 @@
 // out[M, N] = a[M, K] * w[N, K]^T runs either as (X = a, Y = w) for large M, or as (X = w, Y = a)
 // for decode-sized M, so that the weights fill the 128-row dimension of the instruction and the
 // few tokens sit on the narrow N side; the output strides (sx, sy) place D either way round.
-// K can be split over gridDim.z; partial tiles are then reduced in an fp32 workspace with
-// red.global.add and finished by whichever CTA arrives last at the tile. That finalizer can do more than
-// store: with the weights on the 128-row side it holds 128 output features of up to kBN tokens, enough to
+// K can be split over gridDim.z. Where the device holds a cluster per tile at a time the splits of a tile are one
+// cluster (up to sixteen CTAs): each leaves its sums in shared memory and finishes its share of the columns out of
+// the others'. Otherwise partial tiles are reduced in an fp32 workspace with red.global.add and finished by
+// whichever CTA arrives last at the tile. Where the splits meet, more can be done than storing: with the weights on
+// the 128-row side there are 128 output features of a token, enough to
 // rotate a head of a fused qkv projection and append it to the KV cache (rotate-half pairs element i with
 // i + 64), or to form silu(gate) * up when the tile was loaded as 64 gate rows and the 64 up rows of the
 // same features. Either saves a kernel of the decode layer's latency chain.
@@ -72,11 +74,11 @@ struct GemmArgs {
   int cluster;             // the K splits of a tile are one cluster and meet in shared memory (ws and counters unused)
   int x_static;            // X is never written by a kernel (weights): its first tiles may be requested before the
                            // previous kernel of the stream has finished
-  PairEpilogue epi;        // what the split-K finalizer does with rows r and r + 64 of a tile (kEpiNone: plain store)
+  PairEpilogue epi;        // what is done with rows r and r + 64 of a summed tile (kEpiNone: plain store)
 };
 
 // ---- pair epilogues ---------------------------------------------------------------------------------------
-// The finalizer of a tile whose rows r and r + 64 belong together. The 128 epilogue threads split the work as 64 row
+// Splits that met in global memory: the finalizer of a tile whose rows r and r + 64 belong together. The 128 epilogue threads split the work as 64 row
 // pairs x 2 column halves; a thread walks its half in steps of kPairW columns. Everything a step needs is requested
 // before anything is used - the two sums per column from the split-K scratch, the angles of the columns' positions -
 // and the positions themselves are fetched one step ahead (those of the first step before the CTA even knows whether
@@ -565,7 +567,7 @@ std::string gemm_tn(const GemmProblem& g, cudaStream_t stream) {
   int splits = g.splits < 1 ? 1 : g.splits;
   const int epi = g.epi.kind;
   if (epi != kEpiNone) {
-    // the pair epilogues live in the split-K finalizer
+    // the pair epilogues are done where the K splits of a tile meet
     if (a.kblocks < 2) return "a pair epilogue needs K of at least two 128-byte blocks";
     if (splits < 2) splits = 2;
     if (epi == kEpiRopeKv) {

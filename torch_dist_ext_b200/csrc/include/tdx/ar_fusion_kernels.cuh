@@ -913,7 +913,8 @@ template <int kVpt>
 constexpr int kMaxThreadsFor = (kVpt == 1) ? 1024 : 512;
 
 // The single-rank kernel of two vectors per thread that requests the next row ahead (kN: 1 does, 0 does not) is held to 64
-// registers, so that an SM has two blocks: with 79 it had one, and the block's loads of one row (28 KB at 7168 x bf16) were all that was in flight (8192 x 7168 to e4m3: 82 us with one, 67 with two, 6.3 TB/s).
+// registers, so that an SM has two blocks: with 79 it had one, and the block's loads of one row (28 KB at 7168 x bf16) were all that
+// was in flight (8192 x 7168 to e4m3: 82 us with one, 67 with two, 6.2 TB/s; 72.6 per call in a loop).
 // The fp16 kernels to e4m3 spill 3 and 7 registers for it (8192 x 7168: 114 us before, 65 and 67 with it, as bf16).
 template <int kAlgo, int kN, int kVpt>
 constexpr int kMinBlocksFor = (kAlgo == kAlgoLocal && kN == 1 && kVpt == 2) ? 2 : 1;

@@ -8,9 +8,9 @@
 namespace tdx {
 
 // D[x, y] = sum_k X[x, k] * Y[y, k];  D[x, y] is written to out[x * sx + y * sy].
-// What the split-K finalizer of gemm_tn does with the summed tile instead of a plain store. Both kinds combine row r
-// of a 128-row tile with row r + 64, so they need X on the 128-row side (the weights: decode orientation), at least
-// two K splits (the finalizer is the CTA that arrives last at a tile) and a 16-bit or fp32 output.
+// What gemm_tn does with a summed tile instead of a plain store, where its K splits meet: in every CTA of a cluster, or in
+// the CTA that arrives last at the tile. Both kinds combine row r of a 128-row tile with row r + 64, so they need X on the
+// 128-row side (the weights: decode orientation), at least two K splits and a 16-bit or fp32 output.
 enum PairEpilogueKind { kEpiNone = 0, kEpiRopeKv = 1, kEpiSiluMul = 2 };
 struct PairEpilogue {
   int kind;

@@ -245,7 +245,7 @@ static void gemm_scratch(tdx::GemmProblem& g, const Tensor& ws, const Tensor& co
   g.counter_count = (size_t)counters.numel();
 }
 
-// Fused qkv projection of a decode step whose split-K finalizer rotates the query and key heads and appends keys and
+// Fused qkv projection of a decode step that rotates the query and key heads where its K splits meet, and appends keys and
 // values to the caches: out[t, :] = rope(a[t] @ w^T), k_cache[t, positions[t]] / v_cache[t, positions[t]] = the new rows.
 // w [(q_heads + 2 kv_heads) * 128, K] (bf16 / fp16, or e4m3 with 128 x 128 scales and 1 x 128 scales on a).
 void gemm_tn_rope_kv(const Tensor& w, const Tensor& a, Tensor out, int64_t block_n, int64_t splits, const Tensor& ws,
@@ -297,7 +297,7 @@ void gemm_tn_rope_kv(const Tensor& w, const Tensor& a, Tensor out, int64_t block
   TORCH_CHECK(err.empty(), "gemm_tn_rope_kv: ", err);
 }
 
-// Gate/up projection of a decode step whose split-K finalizer applies the activation:
+// Gate/up projection of a decode step that applies the activation where its K splits meet:
 // out[t, f] = silu(a[t] . w[f]) * (a[t] . w[ffn + f]) for w [2 ffn, K] (bf16 / fp16).
 void gemm_tn_silu_mul(const Tensor& w, const Tensor& a, Tensor out, int64_t block_n, int64_t splits, const Tensor& ws,
                       const Tensor& counters, const c10::optional<Tensor>& status) {

@@ -117,8 +117,7 @@ def linear(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None,
                 ws, counters = _pair_scratch(a.device, floats), torch.zeros(words, dtype=torch.int32, device=a.device)
         _lib.ops().gemm_tn_pair(a, w, out, n, 1, _workspace(a.device)[2], ws, counters)
         return out
-    if (use_persistent or (use_pair and persistent is None and _PERSIST_DEFAULT)) and m > 128 and n >= 256 and not swap \
-            and splits in (None, 1):
+    if use_persistent and m > 128 and n >= 256 and not swap and splits in (None, 1):
         if out is None:
             dt = out_dtype or (torch.bfloat16 if a.element_size() == 1 else a.dtype)
             out = torch.empty(m, n, dtype=dt, device=a.device)
@@ -191,7 +190,7 @@ def linear_fp8_blockscaled(a_q: torch.Tensor, a_scale: torch.Tensor, w_q: torch.
 def fused_epilogue_fits(tokens: int, k: int, elem_size: int = 2, scaled: bool = False) -> bool:
     """Whether ``linear_rope_kv`` / ``linear_silu_mul`` can take the problem: the weights must sit on the 128-row side of
     the tile (decode-sized token counts; always for block-scaled operands) and K must span at least two 128-byte blocks
-    (the fused epilogues live in the split-K finalizer)."""
+    (the fused epilogues are done where the K splits of a tile meet)."""
     return plan(tokens, 256, k, elem_size, scaled)[0] and k // (128 // elem_size) >= 2
 
 
@@ -225,7 +224,7 @@ def linear_rope_kv(a: torch.Tensor, w: torch.Tensor, positions: torch.Tensor, co
 def linear_silu_mul(a: torch.Tensor, w_gate_up: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """``silu(a @ w_gate^T) * (a @ w_up^T)`` for ``w_gate_up [2 ffn, K]`` (gate rows, then up rows; bf16 / fp16; ffn a
     multiple of 64) in ONE kernel: every tile of the GEMM is loaded as 64 gate rows plus the 64 up rows of the same
-    features, and the split-K finalizer applies the activation. Decode-sized token counts. PyTorch statement:
+    features, and the activation is applied where the K splits meet. Decode-sized token counts. PyTorch statement:
     ``ops.reference.linear_silu_mul_reference``."""
     m, k = a.shape
     ffn = w_gate_up.shape[0] // 2
